@@ -402,11 +402,10 @@ __global__ void __launch_bounds__(NT, 4)
     if (inst_done(c)) return;
     const LevelView<float> L = views[t.inst];
     const LevelView<float> C = cviews[t.inst];
-    const float inv_dt = (float)c->inv_dt;
     const unsigned ccols = (unsigned)C.g.nx * (unsigned)C.g.ny;
     for (unsigned w = t.begin + threadIdx.x; w < t.end; w += NT) {
         const int l = (int)(w / ccols);
-        restrict_cell<float, false>(L, C, inv_dt, w - (unsigned)l * ccols, l);
+        restrict_cell<float, false>(L, C, w - (unsigned)l * ccols, l);
     }
 }
 
@@ -421,7 +420,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     // copied before the dependent-launch wait, b and the done flag after it
     const auto wait = [] { pdl_enter(); };
     const auto go = [&] { return !inst_done(c); };
-    if (vsmall_body<float, MZ>(small[i], &c->inv_dt, smem, wait, go) == kSmallTimeout &&
+    if (vsmall_body<float, MZ>(small[i], smem, wait, go) == kSmallTimeout &&
         threadIdx.x == 0) {
         // a bounded wait ran out: record it and stop this instance
         atomicExch(&c->err, 1);

@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(32 * MZ)
         gu = L.gU[id];
         // the x = 0 sweep recomputes fcp as factor_column rounded it (one
         // operand stream less); the others load it
-        fc = ZERO ? RN<T>::mul(-(T)gu, fi) : L.fcp[id];
+        fc = ZERO ? fcp_of(gu, fi) : L.fcp[id];
     }
     if (loop_done(flags, cond)) return;  // the same for every thread of the grid
     pdl_trigger();
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(32 * MZ)
         T prev = 0;
 #pragma unroll 4
         for (int k = 0; k < nz; ++k) {
-            const T lower = k > 0 ? -(T)sgu[k - 1][tx] : T(0);
+            const T lower = k > 0 ? -face<T>(sgu[k - 1][tx]) : T(0);
             prev = (sv[k][tx] - lower * prev) * sfi[k][tx];
             sv[k][tx] = prev;
         }
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(NT)
     const bool on = q < (unsigned)cg.nx * (unsigned)cg.ny;
     const int J = on ? (int)(q / (unsigned)cg.nx) : 0, I = on ? (int)(q - (unsigned)J * cg.nx) : 0;
     const int l = (int)blockIdx.y;
-    const T sum = on ? restrict_sum<T, false>(F, (T)ctl->inv_dt, I, J, l) : T(0);
+    const T sum = on ? restrict_sum<T, false>(F, I, J, l) : T(0);
     if (loop_done(flags, cond) || !on) return;
     pdl_trigger();
     C.b[(unsigned)l * cg.plane + scol(cg, I, J)] = sum;
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(NT, 4)
     pdl_trigger();  // several waves: the dependent launches as the last one starts
     const unsigned q = blockIdx.x * NT + threadIdx.x;
     if (q >= (unsigned)C.g.nx * (unsigned)C.g.ny) return;
-    restrict_pair<T, false>(F, C, (T)ctl->inv_dt, q, 2 * (int)blockIdx.y);
+    restrict_pair<T, false>(F, C, q, 2 * (int)blockIdx.y);
 }
 
 // Restriction F -> C fused with C's first sweep (x = 0, red columns). A
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(32 * MZ)
     T sum = 0, fi = 0;
     float gu = 0.0f;
     if (on) {
-        sum = restrict_sum<T, false>(F, (T)ctl->inv_dt, I, J, l);
+        sum = restrict_sum<T, false>(F, I, J, l);
         if (red) {
             fi = C.finv[id];
             gu = C.gU[id];
@@ -277,10 +277,10 @@ __global__ void __launch_bounds__(32 * MZ)
 #pragma unroll
     for (int k = 0; k < MZ; ++k) {
         if (k < nz) {
-            const T lower = k > 0 ? -(T)sgu[k - 1][threadIdx.x] : T(0);
+            const T lower = k > 0 ? -face<T>(sgu[k - 1][threadIdx.x]) : T(0);
             prev = (sb[k][threadIdx.x] - lower * prev) * sfi[k][threadIdx.x];
             v[k] = prev;
-            fcr[k] = RN<T>::mul(-(T)sgu[k][threadIdx.x], sfi[k][threadIdx.x]);  // fcp, as factor_column rounds it
+            fcr[k] = fcp_of(sgu[k][threadIdx.x], sfi[k][threadIdx.x]);  // fcp, as factor_column rounds it
         }
     }
 #pragma unroll
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(kSmallThreadsSolver, 1)
     extern __shared__ __align__(16) unsigned char smem[];
     const auto wait = [] { pdl_enter(); };
     const auto go = [&] { return !loop_done(ctl, cond); };
-    if (mgdev::vsmall_body<T, MZ>(tl, &ctl->inv_dt, smem, wait, go, col_sweeps) == mgdev::kSmallTimeout &&
+    if (mgdev::vsmall_body<T, MZ>(tl, smem, wait, go, col_sweeps) == mgdev::kSmallTimeout &&
         threadIdx.x == 0) {
         // a bounded wait ran out: record it and stop the solve
         atomicExch(&ctl->err, 1);

@@ -4,6 +4,7 @@
 // src/mg3d.h:67-84), the fine residual and restriction
 // (src/pcg3d_cpu.cpp:87-100), and the shared-memory bottom of the V-cycle.
 #pragma once
+#include "f64_dev.cuh"
 #include "kernels.h"
 #include "tma.cuh"
 
@@ -42,10 +43,23 @@ __device__ __forceinline__ Nbr neighbours(const Geo& g, const Geo& cg, int i, in
     return n;
 }
 
+// A face conductance in the V-cycle's precision (FP64: widened by integer
+// operations, f64_dev.cuh; the hardware conversion issues at the FP64 rate).
+template <class T>
+__device__ __forceinline__ T face(float f);
+template <>
+__device__ __forceinline__ float face<float>(float f) {
+    return f;
+}
+template <>
+__device__ __forceinline__ double face<double>(float f) {
+    return f64dev::widen(f);
+}
+
 // The Thomas factor fcp of a cell from its up face and 1/pivot, rounded as
 // factor_column rounds it: -gU * finv, one rounding.
 __device__ __forceinline__ float fcp_of(float gu, float fi) { return __fmul_rn(-gu, fi); }
-__device__ __forceinline__ double fcp_of(float gu, double fi) { return __dmul_rn(-(double)gu, fi); }
+__device__ __forceinline__ double fcp_of(float gu, double fi) { return __dmul_rn(-f64dev::widen(gu), fi); }
 
 // Loads of values that other blocks of the same kernel may have written
 // (x and b inside the cluster tail kernel) go to L2 (CG = true); everything
@@ -68,22 +82,22 @@ __device__ __forceinline__ T lat_sum(const LevelView<T>& L, const LevelView<T>& 
     if (n.w) {
         T xv = ldm<CG>(L.x + base + n.sw);
         if (PRO) xv = xv + ldm<CG>(C.x + cbase + n.pw);
-        s += (T)L.gE[base + n.sw] * xv;
+        s += face<T>(L.gE[base + n.sw]) * xv;
     }
     if (n.e) {
         T xv = ldm<CG>(L.x + base + n.se);
         if (PRO) xv = xv + ldm<CG>(C.x + cbase + n.pe);
-        s += (T)L.gE[base + n.s] * xv;
+        s += face<T>(L.gE[base + n.s]) * xv;
     }
     if (n.so) {
         T xv = ldm<CG>(L.x + base + n.ss);
         if (PRO) xv = xv + ldm<CG>(C.x + cbase + n.ps);
-        s += (T)L.gN[base + n.ss] * xv;
+        s += face<T>(L.gN[base + n.ss]) * xv;
     }
     if (n.no) {
         T xv = ldm<CG>(L.x + base + n.sn);
         if (PRO) xv = xv + ldm<CG>(C.x + cbase + n.pn);
-        s += (T)L.gN[base + n.s] * xv;
+        s += face<T>(L.gN[base + n.s]) * xv;
     }
     return s;
 }
@@ -111,10 +125,10 @@ __device__ __forceinline__ T bf_rhs(const LevelView<T>& L, const LevelView<T>& C
         }
         const float ew = L.gE[base + sw], ee = L.gE[id], ns = L.gN[base + ss], nn = L.gN[id];
         T sum = 0;
-        sum += (n.w ? (T)ew : T(0)) * xw;
-        sum += (n.e ? (T)ee : T(0)) * xe;
-        sum += (n.so ? (T)ns : T(0)) * xs;
-        sum += (n.no ? (T)nn : T(0)) * xn;
+        sum += (n.w ? face<T>(ew) : T(0)) * xw;
+        sum += (n.e ? face<T>(ee) : T(0)) * xe;
+        sum += (n.so ? face<T>(ns) : T(0)) * xs;
+        sum += (n.no ? face<T>(nn) : T(0)) * xn;
         rhs = rhs + sum;
     }
     return rhs;
@@ -142,7 +156,7 @@ __device__ __forceinline__ void column_solve(const LevelView<T>& L, const T* src
 #pragma unroll
     for (int l = 0; l < MZ; ++l) {
         if (l < g.nz) {
-            const T lower = l > 0 ? -(T)gu[l - 1] : T(0);
+            const T lower = l > 0 ? -face<T>(gu[l - 1]) : T(0);
             prev = (v[l] - lower * prev) * fi[l];
             v[l] = prev;
         }
@@ -191,7 +205,7 @@ __device__ __forceinline__ void sweep_column(const LevelView<T>& L, const LevelV
 #pragma unroll
         for (int l = 0; l < MZ; ++l) {
             if (l < g.nz) {
-                const T lower = l > 0 ? -(T)gu[l - 1] : T(0);
+                const T lower = l > 0 ? -face<T>(gu[l - 1]) : T(0);
                 prev = (v[l] - lower * prev) * fi[l];
                 v[l] = prev;
             }
@@ -229,7 +243,7 @@ __device__ __forceinline__ void sweep_column(const LevelView<T>& L, const LevelV
 #pragma unroll
         for (int l = 0; l < MZ; ++l) {
             if (l < g.nz) {
-                const T lower = l > 0 ? -(T)gu[l - 1] : T(0);
+                const T lower = l > 0 ? -face<T>(gu[l - 1]) : T(0);
                 prev = (v[l] - lower * prev) * fi[l];
                 v[l] = prev;
             }
@@ -247,7 +261,7 @@ __device__ __forceinline__ void sweep_column(const LevelView<T>& L, const LevelV
             const unsigned id = (unsigned)l * g.plane + n.s;
             T rhs = ldm<CG>(L.b + id);
             if (!ZERO) rhs = rhs + lat_sum<T, PRO, CG>(L, C, n, l);
-            const T lower = l > 0 ? -(T)gu_b : T(0);
+            const T lower = l > 0 ? -face<T>(gu_b) : T(0);
             prev = (rhs - lower * prev) * L.finv[id];
             L.x[id] = prev;
             gu_b = L.gU[id];
@@ -260,80 +274,39 @@ __device__ __forceinline__ void sweep_column(const LevelView<T>& L, const LevelV
     }
 }
 
-// (b - (A + C/dt) x) at fine cell (i, j, l), in op_apply's order
-// (src/operator3d.h:108-112): diagonal (lateral faces, up, down or ambient,
-// C/dt) times x, minus the six neighbour terms.
+// b - (A + C/dt) x of a cell on operands already loaded, in op_apply's order
+// (src/operator3d.h:108-112): its diagonal dg times x minus the neighbour terms
+// (west, east, south, north, down, up). dg is the diagonal this sum would
+// form (faces west to down, then C/dt fused), stored by set_dt: seven
+// additions, six of them on the FP64 pipe's critical path in FP64, and two
+// operands (C and the bottom face) fewer per cell than forming it here.
+template <class T>
+__device__ __forceinline__ T residual_of(T b, T dg, T xc, T xw, T xe, T xs, T xn, T xd, T xu, float gew, float gee,
+                                         float gns, float gnn, float gu, float gd, bool w, bool e, bool so, bool no,
+                                         bool down, bool up) {
+    T off = 0;
+    if (w) off += face<T>(gew) * xw;
+    if (e) off += face<T>(gee) * xe;
+    if (so) off += face<T>(gns) * xs;
+    if (no) off += face<T>(gnn) * xn;
+    if (down) off += face<T>(gd) * xd;
+    if (up) off += face<T>(gu) * xu;
+    return b - (dg * xc - off);
+}
+
+// The same at fine cell (i, j, l); an absent neighbour reads the cell itself.
 template <class T, bool CG>
-__device__ __forceinline__ T residual_at(const LevelView<T>& F, T inv_dt, int i, int j, int l) {
+__device__ __forceinline__ T residual_at(const LevelView<T>& F, int i, int j, int l) {
     const Geo& fg = F.g;
     const Nbr n = neighbours<false>(fg, fg, i, j, i >> 1, (i + j) & 1);
     const unsigned base = (unsigned)l * fg.plane, id = base + n.s;
-    const bool up = l < fg.nz - 1;
-    const T xc = ldm<CG>(F.x + id);
-    T d = 0, off = 0;
-    if (n.w) {
-        const T ge = (T)F.gE[base + n.sw];
-        d += ge;
-        off += ge * ldm<CG>(F.x + base + n.sw);
-    }
-    if (n.e) {
-        const T ge = (T)F.gE[id];
-        d += ge;
-        off += ge * ldm<CG>(F.x + base + n.se);
-    }
-    if (n.so) {
-        const T gn = (T)F.gN[base + n.ss];
-        d += gn;
-        off += gn * ldm<CG>(F.x + base + n.ss);
-    }
-    if (n.no) {
-        const T gn = (T)F.gN[id];
-        d += gn;
-        off += gn * ldm<CG>(F.x + base + n.sn);
-    }
-    const float gu = F.gU[id];
-    d += (T)gu;
-    d += l > 0 ? (T)F.gU[id - fg.plane] : (T)F.gB[n.s];
-    d += (T)F.cap[id] * inv_dt;
-    if (l > 0) off += (T)F.gU[id - fg.plane] * ldm<CG>(F.x + id - fg.plane);
-    if (up) off += (T)gu * ldm<CG>(F.x + id + fg.plane);
-    return ldm<CG>(F.b + id) - (d * xc - off);
-}
-
-// residual_at's arithmetic on operands already loaded, in its order: the
-// diagonal (west, east, south, north faces, up face, down face or gB, C/dt)
-// times x minus the neighbour terms (west, east, south, north, down, up).
-template <class T>
-__device__ __forceinline__ T residual_of(T b, T xc, T xw, T xe, T xs, T xn, T xd, T xu, float gew, float gee,
-                                         float gns, float gnn, float gu, float gd, float cap, T inv_dt, bool w,
-                                         bool e, bool so, bool no, bool down, bool up) {
-    T d = 0, off = 0;
-    if (w) {
-        const T ge = (T)gew;
-        d += ge;
-        off += ge * xw;
-    }
-    if (e) {
-        const T ge = (T)gee;
-        d += ge;
-        off += ge * xe;
-    }
-    if (so) {
-        const T gn = (T)gns;
-        d += gn;
-        off += gn * xs;
-    }
-    if (no) {
-        const T gn = (T)gnn;
-        d += gn;
-        off += gn * xn;
-    }
-    d += (T)gu;
-    d += (T)gd;
-    d += (T)cap * inv_dt;
-    if (down) off += (T)gd * xd;
-    if (up) off += (T)gu * xu;
-    return b - (d * xc - off);
+    const bool down = l > 0, up = l < fg.nz - 1;
+    const unsigned sw = n.w ? base + n.sw : id, se = n.e ? base + n.se : id;
+    const unsigned ss = n.so ? base + n.ss : id, sn = n.no ? base + n.sn : id;
+    const unsigned sd = down ? id - fg.plane : id, su = up ? id + fg.plane : id;
+    return residual_of<T>(ldm<CG>(F.b + id), F.dg[id], ldm<CG>(F.x + id), ldm<CG>(F.x + sw), ldm<CG>(F.x + se),
+                          ldm<CG>(F.x + ss), ldm<CG>(F.x + sn), ldm<CG>(F.x + sd), ldm<CG>(F.x + su), F.gE[sw],
+                          F.gE[id], F.gN[ss], F.gN[id], F.gU[id], F.gU[sd], n.w, n.e, n.so, n.no, down, up);
 }
 
 // The four children of an interior coarse cell at once: their x, faces and
@@ -341,7 +314,7 @@ __device__ __forceinline__ T residual_of(T b, T xc, T xw, T xe, T xs, T xn, T xd
 // four residual_at's 60, with the index arithmetic shared), and each child's
 // residual is residual_at's, operation for operation.
 template <class T, bool CG>
-__device__ __forceinline__ T restrict_sum4(const LevelView<T>& F, T inv_dt, int I, int J, int l) {
+__device__ __forceinline__ T restrict_sum4(const LevelView<T>& F, int I, int J, int l) {
     const Geo& g = F.g;
     const int i0 = 2 * I, j0 = 2 * J;
     const bool w = i0 > 0, e = i0 + 2 < g.nx, so = j0 > 0, no = j0 + 2 < g.ny;
@@ -367,32 +340,30 @@ __device__ __forceinline__ T restrict_sum4(const LevelView<T>& F, T inv_dt, int 
     const float gNs0 = F.gN[s0], gN00 = F.gN[c00], gNs1 = F.gN[s1], gN10 = F.gN[c10];
     const float gN01 = F.gN[c01], gN11 = F.gN[c11];
     const float gu00 = F.gU[c00], gu10 = F.gU[c10], gu01 = F.gU[c01], gu11 = F.gU[c11];
-    // down face: gU of the plane below, or gB at the bottom plane
-    const unsigned cb = (unsigned)l * g.plane;
-    const float gd00 = down ? F.gU[c00 - dn] : F.gB[c00 - cb], gd10 = down ? F.gU[c10 - dn] : F.gB[c10 - cb];
-    const float gd01 = down ? F.gU[c01 - dn] : F.gB[c01 - cb], gd11 = down ? F.gU[c11 - dn] : F.gB[c11 - cb];
+    // down face: gU of the plane below (unused at the bottom plane)
+    const float gd00 = F.gU[c00 - dn], gd10 = F.gU[c10 - dn], gd01 = F.gU[c01 - dn], gd11 = F.gU[c11 - dn];
     T sum = 0;
-    sum += residual_of<T>(ldm<CG>(F.b + c00), x00, xw0, x10, xs0, x01, d00, u00, gEw0, gE00, gNs0, gN00, gu00, gd00,
-                          F.cap[c00], inv_dt, w, true, so, true, down, up);
-    sum += residual_of<T>(ldm<CG>(F.b + c10), x10, x00, xe0, xs1, x11, d10, u10, gE00, gE10, gNs1, gN10, gu10, gd10,
-                          F.cap[c10], inv_dt, true, e, so, true, down, up);
-    sum += residual_of<T>(ldm<CG>(F.b + c01), x01, xw1, x11, x00, xn0, d01, u01, gEw1, gE01, gN00, gN01, gu01, gd01,
-                          F.cap[c01], inv_dt, w, true, true, no, down, up);
-    sum += residual_of<T>(ldm<CG>(F.b + c11), x11, x01, xe1, x10, xn1, d11, u11, gE01, gE11, gN10, gN11, gu11, gd11,
-                          F.cap[c11], inv_dt, true, e, true, no, down, up);
+    sum += residual_of<T>(ldm<CG>(F.b + c00), F.dg[c00], x00, xw0, x10, xs0, x01, d00, u00, gEw0, gE00, gNs0, gN00, gu00, gd00,
+                          w, true, so, true, down, up);
+    sum += residual_of<T>(ldm<CG>(F.b + c10), F.dg[c10], x10, x00, xe0, xs1, x11, d10, u10, gE00, gE10, gNs1, gN10, gu10, gd10,
+                          true, e, so, true, down, up);
+    sum += residual_of<T>(ldm<CG>(F.b + c01), F.dg[c01], x01, xw1, x11, x00, xn0, d01, u01, gEw1, gE01, gN00, gN01, gu01, gd01,
+                          w, true, true, no, down, up);
+    sum += residual_of<T>(ldm<CG>(F.b + c11), F.dg[c11], x11, x01, xe1, x10, xn1, d11, u11, gE01, gE11, gN10, gN11, gu11, gd11,
+                          true, e, true, no, down, up);
     return sum;
 }
 
 // Restriction (src/pcg3d_cpu.cpp:87-100) of coarse cell (I, J, l): the sum
 // over the (up to 4) children, j then i, of the fine residual.
 template <class T, bool CG>
-__device__ __forceinline__ T restrict_sum(const LevelView<T>& F, T inv_dt, int I, int J, int l) {
+__device__ __forceinline__ T restrict_sum(const LevelView<T>& F, int I, int J, int l) {
     const Geo& fg = F.g;
-    if (2 * I + 1 < fg.nx && 2 * J + 1 < fg.ny) return restrict_sum4<T, CG>(F, inv_dt, I, J, l);
+    if (2 * I + 1 < fg.nx && 2 * J + 1 < fg.ny) return restrict_sum4<T, CG>(F, I, J, l);
     const int i1 = min(2 * I + 2, fg.nx), j1 = min(2 * J + 2, fg.ny);
     T sum = 0;
     for (int j = 2 * J; j < j1; ++j)
-        for (int i = 2 * I; i < i1; ++i) sum += residual_at<T, CG>(F, inv_dt, i, j, l);
+        for (int i = 2 * I; i < i1; ++i) sum += residual_at<T, CG>(F, i, j, l);
     return sum;
 }
 
@@ -400,14 +371,14 @@ __device__ __forceinline__ T restrict_sum(const LevelView<T>& F, T inv_dt, int I
 // both sums before either store, so the shared vertical operands are loaded
 // once.
 template <class T, bool CG>
-__device__ __forceinline__ void restrict_pair(const LevelView<T>& F, const LevelView<T>& C, T inv_dt,
+__device__ __forceinline__ void restrict_pair(const LevelView<T>& F, const LevelView<T>& C,
                                               unsigned q, int l) {
     const Geo& cg = C.g;
     const int J = (int)(q / (unsigned)cg.nx), I = (int)(q - (unsigned)J * cg.nx);
     const unsigned cs = scol(cg, I, J);
-    const T s0 = restrict_sum<T, CG>(F, inv_dt, I, J, l);
+    const T s0 = restrict_sum<T, CG>(F, I, J, l);
     if (l + 1 < cg.nz) {
-        const T s1 = restrict_sum<T, CG>(F, inv_dt, I, J, l + 1);
+        const T s1 = restrict_sum<T, CG>(F, I, J, l + 1);
         C.b[(unsigned)l * cg.plane + cs] = s0;
         C.b[(unsigned)(l + 1) * cg.plane + cs] = s1;
     } else {
@@ -417,11 +388,11 @@ __device__ __forceinline__ void restrict_pair(const LevelView<T>& F, const Level
 
 // The same stored as coarse b; q = J cnx + I.
 template <class T, bool CG>
-__device__ __forceinline__ void restrict_cell(const LevelView<T>& F, const LevelView<T>& C,
-                                              T inv_dt, unsigned q, int l) {
+__device__ __forceinline__ void restrict_cell(const LevelView<T>& F, const LevelView<T>& C, unsigned q,
+                                              int l) {
     const Geo& cg = C.g;
     const int J = (int)(q / (unsigned)cg.nx), I = (int)(q - (unsigned)J * cg.nx);
-    C.b[(unsigned)l * cg.plane + scol(cg, I, J)] = restrict_sum<T, CG>(F, inv_dt, I, J, l);
+    C.b[(unsigned)l * cg.plane + scol(cg, I, J)] = restrict_sum<T, CG>(F, I, J, l);
 }
 
 
@@ -445,7 +416,7 @@ __device__ __forceinline__ void gather_rhs(const LevelView<T>& L, const LevelVie
 }
 
 // Level views of the shared-memory bottom: a level's arrays lie at base in
-// the order gE, gN, gU, cap, gB, fcp, finv, x, b, each rounded up to 16 bytes
+// the order gE, gN, gU, dg, fcp, finv, x, b, each rounded up to 16 bytes
 // (small_level_bytes adds the same sizes). The views are rebuilt from the
 // block's base and a byte offset wherever they are used, never stored as
 // pointers, so every pointer visibly points into shared memory and the
@@ -464,8 +435,7 @@ __device__ __forceinline__ LevelView<T> small_view(unsigned char* base, const Ge
     S.gE = (const float*)take(ln * 4u);
     S.gN = (const float*)take(ln * 4u);
     S.gU = (const float*)take(ln * 4u);
-    S.cap = (const float*)take(ln * 4u);
-    S.gB = (const float*)take(g.plane * 4u);
+    S.dg = (T*)take(ln * (unsigned)sizeof(T));
     S.fcp = (T*)take(ln * (unsigned)sizeof(T));
     S.finv = (T*)take(ln * (unsigned)sizeof(T));
     S.x = (T*)take(ln * (unsigned)sizeof(T));
@@ -493,8 +463,8 @@ __device__ __forceinline__ LevelView<T> small_view(unsigned char* base, const Ge
 constexpr int kSmallDone = 0, kSmallTimeout = 1, kSmallClosed = 2;
 
 template <class T, int MZ, class Wait, class Go>
-__device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, const double* inv_dt_src,
-                                           unsigned char* smem, Wait wait, Go go, bool col_sweeps = false) {
+__device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, unsigned char* smem, Wait wait, Go go,
+                                           bool col_sweeps = false) {
     __shared__ Geo sg[kMaxTail];      // level geometry
     __shared__ unsigned soff[kMaxTail];  // byte offset of each level in smem
     __shared__ uint64_t bar, barb;    // operator and factors; level k0's b
@@ -507,7 +477,7 @@ __device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, const double
             soff[k] = off;
             off += (unsigned)small_level_bytes(g, sizeof(T));
             const unsigned ln = g.plane * (unsigned)g.nz;
-            total += 4u * ln * 4u + g.plane * 4u + 2u * ln * (unsigned)sizeof(T);
+            total += 3u * ln * 4u + 3u * ln * (unsigned)sizeof(T);
         }
         tma::mbar_init(&bar, 1);
         tma::mbar_init(&barb, 1);
@@ -516,9 +486,9 @@ __device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, const double
     }
     __syncthreads();
     if (threadIdx.x < 32u) {
-        // copy c of level k = c / 7: gE, gN, gU, cap, gB, fcp, finv
-        for (int c = (int)threadIdx.x; c < 7 * nl; c += 32) {
-            const int k = c / 7, a = c - 7 * k;
+        // copy c of level k = c / 6: gE, gN, gU, dg, fcp, finv
+        for (int c = (int)threadIdx.x; c < 6 * nl; c += 32) {
+            const int k = c / 6, a = c - 6 * k;
             const LevelView<T>& G = tl.L[k];
             const LevelView<T> S = small_view<T>(smem + soff[k], sg[k]);
             const unsigned ln = sg[k].plane * (unsigned)sg[k].nz;
@@ -526,9 +496,8 @@ __device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, const double
             if (a == 0) tma::bulk_load((void*)S.gE, G.gE, fb, &bar);
             else if (a == 1) tma::bulk_load((void*)S.gN, G.gN, fb, &bar);
             else if (a == 2) tma::bulk_load((void*)S.gU, G.gU, fb, &bar);
-            else if (a == 3) tma::bulk_load((void*)S.cap, G.cap, fb, &bar);
-            else if (a == 4) tma::bulk_load((void*)S.gB, G.gB, sg[k].plane * 4u, &bar);
-            else if (a == 5) tma::bulk_load(S.fcp, G.fcp, tb, &bar);
+            else if (a == 3) tma::bulk_load(S.dg, G.dg, tb, &bar);
+            else if (a == 4) tma::bulk_load(S.fcp, G.fcp, tb, &bar);
             else tma::bulk_load(S.finv, G.finv, tb, &bar);
         }
     }
@@ -557,7 +526,6 @@ __device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, const double
         }
         return kSmallClosed;
     }
-    const T inv_dt = (T)*inv_dt_src;
     const bool got = tma::mbar_wait(&bar, 0u) && tma::mbar_wait(&barb, 0u);
     if (!__syncthreads_and(got)) {
         if (threadIdx.x == 0) {  // let the copies land before leaving
@@ -599,7 +567,7 @@ __device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, const double
             const unsigned work = ccols * (unsigned)C.g.nz;
             for (unsigned w = tid; w < work; w += nth) {
                 const int l = (int)(w / ccols);
-                restrict_cell<T, false>(L, C, inv_dt, w - (unsigned)l * ccols, l);
+                restrict_cell<T, false>(L, C, w - (unsigned)l * ccols, l);
             }
         } else if (sizeof(T) == 4 && MZ > 0 && kind != 0 && col_sweeps) {
             // One thread per column gathers every plane's right-hand side

@@ -5,6 +5,7 @@
 // bit. Shared by the single solver (k_outer.cu, k_mg.cu) and the batched
 // set_dt (k_batch.cu).
 #pragma once
+#include "f64_dev.cuh"
 #include "kernels.h"
 
 namespace ct {
@@ -18,6 +19,8 @@ struct RN<float> {
     static __device__ float sub(float a, float b) { return __fsub_rn(a, b); }
     static __device__ float mul(float a, float b) { return __fmul_rn(a, b); }
     static __device__ float div(float a, float b) { return __fdiv_rn(a, b); }
+    static __device__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+    static __device__ float of(float f) { return f; }
 };
 template <>
 struct RN<double> {
@@ -25,25 +28,29 @@ struct RN<double> {
     static __device__ double sub(double a, double b) { return __dsub_rn(a, b); }
     static __device__ double mul(double a, double b) { return __dmul_rn(a, b); }
     static __device__ double div(double a, double b) { return __ddiv_rn(a, b); }
+    static __device__ double fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+    static __device__ double of(float f) { return f64dev::widen(f); }
 };
 
-// op_diag of cell (i, j, l) of a level, in T.
+// The face part of op_diag of cell (i, j, l) of a level, in T.
 template <class T>
-__device__ __forceinline__ T diag_rn(const LevelView<T>& L, int i, int j, int l, T inv_dt) {
+__device__ __forceinline__ T face_sum_rn(const LevelView<T>& L, int i, int j, int l) {
     const Geo& g = L.g;
     const unsigned base = (unsigned)l * g.plane;
     const unsigned s = scol(g, i, j), id = base + s;
     T d = 0;
-    if (i > 0) d = RN<T>::add(d, (T)L.gE[base + scol(g, i - 1, j)]);
-    if (i < g.nx - 1) d = RN<T>::add(d, (T)L.gE[id]);
-    if (j > 0) d = RN<T>::add(d, (T)L.gN[base + scol(g, i, j - 1)]);
-    if (j < g.ny - 1) d = RN<T>::add(d, (T)L.gN[id]);
-    d = RN<T>::add(d, (T)L.gU[id]);
-    d = RN<T>::add(d, l > 0 ? (T)L.gU[id - g.plane] : (T)L.gB[s]);
-    return RN<T>::add(d, RN<T>::mul((T)L.cap[id], inv_dt));
+    if (i > 0) d = RN<T>::add(d, RN<T>::of(L.gE[base + scol(g, i - 1, j)]));
+    if (i < g.nx - 1) d = RN<T>::add(d, RN<T>::of(L.gE[id]));
+    if (j > 0) d = RN<T>::add(d, RN<T>::of(L.gN[base + scol(g, i, j - 1)]));
+    if (j < g.ny - 1) d = RN<T>::add(d, RN<T>::of(L.gN[id]));
+    d = RN<T>::add(d, RN<T>::of(L.gU[id]));
+    return RN<T>::add(d, RN<T>::of(l > 0 ? L.gU[id - g.plane] : L.gB[s]));
 }
 
-// Thomas factors of natural column q = j nx + i of a level. The factors are
+// Thomas factors of natural column q = j nx + i of a level, and its cells'
+// diagonals for the restriction (dg). Both diagonals are the face sum plus
+// C/dt; the factorisation adds the rounded product (mg_factor_column's
+// arithmetic), the restriction's residual the product fused. The factors are
 // written through restrict pointers, so the operand loads of the next planes
 // may be issued before this plane's stores.
 template <class T>
@@ -53,14 +60,17 @@ __device__ __forceinline__ void factor_column(const LevelView<T>& L, T inv_dt, u
     const unsigned s = scol(g, i, j);
     T* __restrict__ finv = L.finv;
     T* __restrict__ fcp = L.fcp;
+    T* __restrict__ dg = L.dg;
     const float* __restrict__ gU = L.gU;
     T cp_prev = 0;
 #pragma unroll 4
     for (int l = 0; l < g.nz; ++l) {
         const unsigned id = (unsigned)l * g.plane + s;
-        const T d = diag_rn(L, i, j, l, inv_dt);
-        const T lower = l > 0 ? -(T)gU[id - g.plane] : T(0);
-        const T upper = l < g.nz - 1 ? -(T)gU[id] : T(0);
+        const T faces = face_sum_rn(L, i, j, l), cap = RN<T>::of(L.cap[id]);
+        const T d = RN<T>::add(faces, RN<T>::mul(cap, inv_dt));
+        dg[id] = RN<T>::fma(cap, inv_dt, faces);
+        const T lower = l > 0 ? -RN<T>::of(gU[id - g.plane]) : T(0);
+        const T upper = l < g.nz - 1 ? -RN<T>::of(gU[id]) : T(0);
         const T inv = RN<T>::div(T(1), RN<T>::sub(d, RN<T>::mul(lower, cp_prev)));
         finv[id] = inv;
         cp_prev = RN<T>::mul(upper, inv);
