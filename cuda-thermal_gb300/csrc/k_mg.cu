@@ -291,16 +291,16 @@ __global__ void __launch_bounds__(32 * MZ)
         if (k < nz) C.x[(unsigned)k * cg.plane + cs] = v[k];
 }
 
-// The bottom of the V-cycle in one block from shared memory (mgdev::vsmall_body),
-// bounded at the 256 threads it is launched with, so a thread may hold up to
+// The bottom of the V-cycle in one block from shared memory (mgdev::vsmall_body;
+// FP64, and FP32 columns of more than 32 planes), bounded at the 256 threads it is launched with, so a thread may hold up to
 // 255 registers (12 planes: 167, 16 planes: 219, no spills).
 template <class T, int MZ>
 __global__ void __launch_bounds__(kSmallThreadsSolver, 1)
-    k_vsmall(TailLevels<T> tl, Ctl* ctl, Cond cond, bool col_sweeps) {
+    k_vsmall(TailLevels<T> tl, Ctl* ctl, Cond cond) {
     extern __shared__ __align__(16) unsigned char smem[];
     const auto wait = [] { pdl_enter(); };
     const auto go = [&] { return !loop_done(ctl, cond); };
-    if (mgdev::vsmall_body<T, MZ>(tl, smem, wait, go, col_sweeps) == mgdev::kSmallTimeout &&
+    if (mgdev::vsmall_body<T, MZ>(tl, smem, wait, go) == mgdev::kSmallTimeout &&
         threadIdx.x == 0) {
         // a bounded wait ran out: record it and stop the solve
         atomicExch(&ctl->err, 1);
@@ -456,19 +456,17 @@ cudaError_t launch_vsmall(cudaStream_t st, const TailLevels<T>& tl, Ctl* ctl, Co
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              kSmallSmemMax);
         if (e != cudaSuccess) return e;
-        // FP32 sweeps one thread per column (CT_SMALL_COL_SWEEPS=0: gather
-        // and recurrence as two steps, as in FP64 and the batch)
-        const char* cs_env = std::getenv("CT_SMALL_COL_SWEEPS");
-        const bool col_sweeps = !(cs_env && cs_env[0] == '0');
-        // 256 threads (8 warps to a block barrier): 158.5 vs 158.2 solves/s
-        // with 512 at 800 x 800 (the batch's instance blocks keep 512)
-        launch_pdl(kern, 1, kSmallThreadsSolver, smem, st, tl, ctl, cond, col_sweeps);
+        // (the batch's instance blocks have 512 threads)
+        launch_pdl(kern, 1, kSmallThreadsSolver, smem, st, tl, ctl, cond);
         return cudaGetLastError();
     };
-    if (mz <= 8) return go(k_vsmall<T, 8>);
-    if (mz <= 12) return go(k_vsmall<T, 12>);
-    if (mz <= 16) return go(k_vsmall<T, 16>);
-    if (mz <= 32) return go(k_vsmall<T, 32>);
+    // (FP32 up to 32 planes runs in one cluster, k_tail.cu)
+    if constexpr (sizeof(T) == 8) {
+        if (mz <= 8) return go(k_vsmall<T, 8>);
+        if (mz <= 12) return go(k_vsmall<T, 12>);
+        if (mz <= 16) return go(k_vsmall<T, 16>);
+        if (mz <= 32) return go(k_vsmall<T, 32>);
+    }
     return go(k_vsmall<T, 0>);
 }
 

@@ -433,6 +433,20 @@ bool encode_rows_map(CUtensorMap* out, const float* base, int hx, int ny, int nz
               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Whole rows (both colours, `row` slots) of a level's array: box = a row, `rows`
+// rows and every plane.
+bool encode_tail_map(CUtensorMap* out, const float* base, const Geo& g, unsigned row, unsigned rows, unsigned nz) {
+    PFN_cuTensorMapEncodeTiled_v12000 fn = encode_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)row, (cuuint64_t)g.ny, (cuuint64_t)g.nz};
+    const cuuint64_t strides[2] = {(cuuint64_t)row * 4u, (cuuint64_t)g.plane * 4u};
+    const cuuint32_t box[3] = {row, rows, nz};
+    const cuuint32_t estr[3] = {1u, 1u, 1u};
+    return fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool make_sweep_maps(const LevelView<float>& L, int color, SweepMaps* m, int tile_t, int tile_j) {
     const Geo& g = L.g;
     const int oc = color ^ 1;

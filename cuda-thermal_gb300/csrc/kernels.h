@@ -293,6 +293,57 @@ __host__ __device__ inline size_t small_level_bytes(const Geo& g, size_t elem) {
     const size_t ln = (size_t)g.plane * (size_t)g.nz;
     return 3 * small_round16(ln * 4) + 5 * small_round16(ln * elem);
 }
+// The coarse end of the single solver's FP32 V-cycle in one cluster launch
+// (k_tail.cu): `n` levels, finest first; the first nd are split by rows over
+// the first `dist` CTAs (`rows` each), the others are CTA `bottom`'s. Offsets
+// in floats (or ints) of the CTA's shared memory.
+constexpr int kTailLevels = 16;
+constexpr int kTailSpread = 8;           // distributed levels, at most
+constexpr int kTailSmemMax = 224 * 1024;
+constexpr size_t kTailTableMax = 64 * 1024;  // bytes of descriptors and tables
+constexpr int kTailCtas = 16;            // CTAs of the cluster, at most
+// Levels of at most this many cells are one CTA's (16 x 16 columns of 10
+// planes): 800 x 800 x 10 418.8 us an iteration, 419.7 at 1000 cells; 1024 x
+// 1024 x 16 964.6 us, 967 at 1000 and 975 at 4096 (its 16 x 16 level on one CTA).
+constexpr int kTailBottomCells = 2560;
+struct TailLevel {
+    int x, b, fi, gu, ge, gn, dg;  // the level's arrays
+    int tcol, tpar, tcell;         // its tables: columns, black columns' parents, coarse cells
+    int hx, rows, nx, ny;
+    int ncol, ncell;  // slots of one colour, coarse cells of the rows
+    int gnh;          // floats of gN's halo row (0: none)
+    int pad;
+};
+constexpr int kTailDescriptors = 32;  // where the descriptors lie (a west neighbour of the first slot stays inside)
+struct TailPlan {
+    int n, nd, nz, ctas, dist, bottom;
+    int rd;                // rows of level nd whose children are one CTA's
+    int xd;                // a CTA's copy of level nd's x around those rows
+    int x, x4;             // every x: first float, float4s
+    int tab, table_bytes;  // the descriptors and tables
+    unsigned first_bytes, bottom_first_bytes, dist_bytes, bottom_bytes;  // copies: 1/pivot and gU of the first level, all
+    int smem;              // bytes
+    float* x0;             // the first level's x in global memory
+    unsigned plane;        // its plane stride
+    TailLevel L[kTailLevels];
+};
+// One level's arrays: 1/pivot, gU, gE, gN, diagonal, b. A distributed level's as
+// tensor maps, whole rows (both colours) of all planes (gN with one row more);
+// the others' as they lie.
+struct TailMaps {
+    CUtensorMap m[6];
+    const float* whole[16];  // (five, padded to the maps' alignment)
+};
+// Lays out levels views[0 .. n) for a cluster of at most `ctas` CTAs, the bottom
+// levels on a CTA of their own (apart) or with the first rows; false if they do
+// not fit smem_max bytes a CTA.
+bool plan_tail(const LevelView<float>* views, int n, int ctas, bool apart, size_t smem_max, TailPlan* out);
+void fill_tail_table(const TailPlan& p, int* table);  // p.table_bytes of it
+bool make_tail_maps(const TailPlan& p, const LevelView<float>* views, TailMaps* maps);
+bool encode_tail_map(CUtensorMap* out, const float* base, const Geo& g, unsigned row, unsigned rows, unsigned nz);
+bool tail_fits_device(const TailPlan& p);  // the device can hold such a cluster
+cudaError_t launch_tail(cudaStream_t st, const TailPlan& p, const TailMaps* maps, const int* table, Ctl* ctl,
+                        Cond cond);
 template <class T>
 size_t small_smem_bytes(const TailLevels<T>& tl);
 template <class T>

@@ -102,8 +102,8 @@ __device__ __forceinline__ T lat_sum(const LevelView<T>& L, const LevelView<T>& 
     return s;
 }
 
-// Right-hand side of plane l of a column in the branch-free form (BF below):
-// b plus the lateral sum in op_lat_sum's order (west, east, south, north),
+// Right-hand side of plane l of a column, branch-free (for levels in shared
+// memory, where load latency bounds a sweep): b plus the lateral sum in op_lat_sum's order (west, east, south, north),
 // each neighbour value with its parent's coarse correction under PRO; an
 // absent neighbour reads the column itself with weight 0.
 template <class T, bool ZERO, bool PRO, bool CG>
@@ -175,13 +175,7 @@ __device__ __forceinline__ void column_solve(const LevelView<T>& L, const T* src
 // all loads independent of one another, then the Thomas recurrence runs on
 // registers and x is written once. MZ = 0 is the general path for deep
 // columns, with forward values going through x as in the reference.
-//
-// BF (branch-free gather, for levels held in shared memory or L2, where load
-// latency rather than bandwidth bounds a sweep): planes past nz read the last
-// plane (values unused) and an absent neighbour reads the column itself with
-// weight 0 — an exact zero added where lat_sum skips the term — so every
-// load of every plane can be in flight at once.
-template <class T, int MZ, bool ZERO, bool PRO, bool CG, bool BF = false>
+template <class T, int MZ, bool ZERO, bool PRO, bool CG>
 __device__ __forceinline__ void sweep_column(const LevelView<T>& L, const LevelView<T>& C,
                                              int color, unsigned q) {
     const Geo& g = L.g;
@@ -189,34 +183,7 @@ __device__ __forceinline__ void sweep_column(const LevelView<T>& L, const LevelV
     const int i = 2 * t + ((j + color) & 1);
     if (i >= g.nx) return;
     const Nbr n = neighbours<PRO>(g, C.g, i, j, t, color);
-    if constexpr (MZ > 0 && BF) {
-        T v[MZ], fi[MZ], fc[MZ];
-        float gu[MZ];
-#pragma unroll
-        for (int l = 0; l < MZ; ++l) {
-            const unsigned lc = (unsigned)(l < g.nz ? l : g.nz - 1);
-            const unsigned id = lc * g.plane + n.s;
-            v[l] = bf_rhs<T, ZERO, PRO, CG>(L, C, n, lc);
-            fi[l] = L.finv[id];
-            fc[l] = L.fcp[id];
-            gu[l] = L.gU[id];
-        }
-        T prev = 0;
-#pragma unroll
-        for (int l = 0; l < MZ; ++l) {
-            if (l < g.nz) {
-                const T lower = l > 0 ? -face<T>(gu[l - 1]) : T(0);
-                prev = (v[l] - lower * prev) * fi[l];
-                v[l] = prev;
-            }
-        }
-#pragma unroll
-        for (int l = MZ - 2; l >= 0; --l)
-            if (l < g.nz - 1) v[l] -= fc[l] * v[l + 1];
-#pragma unroll
-        for (int l = 0; l < MZ; ++l)
-            if (l < g.nz) L.x[(unsigned)l * g.plane + n.s] = v[l];
-    } else if constexpr (MZ > 0) {
+    if constexpr (MZ > 0) {
         // Gather: every operand of every plane, all loads independent, so the
         // whole column costs about one memory latency.
         T v[MZ], fi[MZ], fc[MZ];
@@ -457,14 +424,11 @@ __device__ __forceinline__ LevelView<T> small_view(unsigned char* base, const Ge
 // issued, so the two latencies overlap) says whether to run the phases at
 // all. Returns kSmallDone, kSmallClosed (go() said no: nothing written once
 // the copies have landed) or kSmallTimeout (a bounded wait for the copies ran
-// out: nothing written). col_sweeps (FP32): each sweep one thread per column
-// over every plane; otherwise one task per column and plane gathers the
-// right-hand sides first. Same bits either way; any block size.
+// out: nothing written). Any block size.
 constexpr int kSmallDone = 0, kSmallTimeout = 1, kSmallClosed = 2;
 
 template <class T, int MZ, class Wait, class Go>
-__device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, unsigned char* smem, Wait wait, Go go,
-                                           bool col_sweeps = false) {
+__device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, unsigned char* smem, Wait wait, Go go) {
     __shared__ Geo sg[kMaxTail];      // level geometry
     __shared__ unsigned soff[kMaxTail];  // byte offset of each level in smem
     __shared__ uint64_t bar, barb;    // operator and factors; level k0's b
@@ -569,20 +533,6 @@ __device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, unsigned cha
                 const int l = (int)(w / ccols);
                 restrict_cell<T, false>(L, C, w - (unsigned)l * ccols, l);
             }
-        } else if (sizeof(T) == 4 && MZ > 0 && kind != 0 && col_sweeps) {
-            // One thread per column gathers every plane's right-hand side
-            // (branch-free, all loads in flight at once) and runs the
-            // recurrence: one block barrier a sweep instead of two (FP32
-            // only: the FP64 columns' registers would spill).
-            if constexpr (sizeof(T) == 4 && MZ > 0) {
-                for (unsigned q = tid; q < ncol; q += nth) {
-                    if (kind == 1)
-                        sweep_column<T, MZ, false, false, false, true>(L, L, color, q);
-                    else
-                        sweep_column<T, MZ, false, true, false, true>(
-                            L, small_view<T>(smem + soff[k + 1], sg[k + 1]), 1, q);
-                }
-            }
         } else if constexpr (MZ > 0) {
             // A sweep in two steps: one task per column and plane gathers
             // that plane's right-hand side into the column's own x slot (the
@@ -602,12 +552,12 @@ __device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, unsigned cha
                     column_solve<T, MZ>(L, src, (unsigned)(2 * j + color) * (unsigned)L.g.hx + (unsigned)t);
             }
         } else if (kind == 0) {  // deep columns (MZ = 0): x goes through memory
-            for (unsigned q = tid; q < ncol; q += nth) sweep_column<T, MZ, true, false, false, true>(L, L, 0, q);
+            for (unsigned q = tid; q < ncol; q += nth) sweep_column<T, MZ, true, false, false>(L, L, 0, q);
         } else if (kind == 1) {
-            for (unsigned q = tid; q < ncol; q += nth) sweep_column<T, MZ, false, false, false, true>(L, L, color, q);
+            for (unsigned q = tid; q < ncol; q += nth) sweep_column<T, MZ, false, false, false>(L, L, color, q);
         } else {
             const LevelView<T> C = small_view<T>(smem + soff[k + 1], sg[k + 1]);
-            for (unsigned q = tid; q < ncol; q += nth) sweep_column<T, MZ, false, true, false, true>(L, C, 1, q);
+            for (unsigned q = tid; q < ncol; q += nth) sweep_column<T, MZ, false, true, false>(L, C, 1, q);
         }
         __syncthreads();
     }

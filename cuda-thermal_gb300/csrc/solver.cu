@@ -135,6 +135,9 @@ ct_status Solver::create(const ct_model* m_in, ct_precond pc_, ct_precision prec
     const size_t o_nat = ar.take(ncells * 8);
     const size_t o_part = ar.take((size_t)NSLOT * 4 * maxb * 8);
     const size_t o_ctl = ar.take(sizeof(Ctl));
+    const bool want_tail = mt == MG_F32 && !skip_graphs;
+    const size_t o_tm = want_tail ? ar.take(kTailLevels * sizeof(TailMaps)) : 0;
+    const size_t o_tt = want_tail ? ar.take(kTailTableMax) : 0;
     if (pc == CT_MULTIGRID) {
         Level L;
         L.g = g0;
@@ -171,6 +174,7 @@ ct_status Solver::create(const ct_model* m_in, ct_precond pc_, ct_precision prec
             L = C;
         }
     }
+    size_t tail_max = 0;
     {
         // The smallest levels whose arrays fit one block's shared memory.
         small_k0 = lv.size();
@@ -185,6 +189,9 @@ ct_status Solver::create(const ct_model* m_in, ct_precond pc_, ct_precision prec
             if (end == e || *end != '\0' || v < 0)
                 return fail(CT_BAD_ARG, "CT_SMALL_BYTES=%s is not a byte count", e);
             small_max = std::min(small_max, v);
+            tail_max = (size_t)std::min<long>(kTailSmemMax, v);
+        } else {
+            tail_max = (size_t)std::min<long>(kTailSmemMax, optin - 4096);
         }
         size_t acc = 0;
         for (size_t k = lv.size(); k-- > 0;) {
@@ -224,6 +231,12 @@ ct_status Solver::create(const ct_model* m_in, ct_precond pc_, ct_precision prec
     nat = at<double>(o_nat);
     part = at<double>(o_part);
     ctl = at<Ctl>(o_ctl);
+    if (want_tail) {
+        tail_maps = at<TailMaps>(o_tm);
+        tail_table = at<int>(o_tt);
+        const ct_status ts = choose_tail(tail_max);
+        if (ts != CT_OK) return ts;
+    }
     CT_CK(cudaStreamSynchronize(st));
     times.alloc_ms = ms_since(t0);
 
@@ -332,6 +345,34 @@ ct_status Solver::create(const ct_model* m_in, ct_precond pc_, ct_precision prec
     return CT_OK;
 }
 
+// The coarse levels that one cluster holds in shared memory (k_tail.cu): from
+// the finest level that fits, the bottom on a CTA of its own where one is to
+// spare. The tensor maps and tables go to device memory.
+ct_status Solver::choose_tail(size_t smem_max) {
+    LevelView<float> v[kTailLevels];
+    for (size_t k0 = lv.size() > kTailLevels ? lv.size() - kTailLevels : 0; k0 < lv.size(); ++k0) {
+        const int nl = (int)(lv.size() - k0);
+        for (int q = 0; q < nl; ++q) v[q] = view<float>(k0 + (size_t)q);
+        TailPlan p, best;
+        best.n = 0;
+        for (const bool apart : {false, true})  // the one with fewer rows a CTA; of two with the same, apart
+            if (plan_tail(v, nl, kTailCtas, apart, smem_max, &p) && (best.n == 0 || p.rd <= best.rd)) best = p;
+        std::vector<TailMaps> m((size_t)nl);
+        if (best.n == 0 || (size_t)best.table_bytes > kTailTableMax || !tail_fits_device(best) ||
+            !make_tail_maps(best, v, m.data()))
+            continue;
+        std::vector<int> table((size_t)best.table_bytes / 4);
+        fill_tail_table(best, table.data());
+        CT_CK(cudaMemcpyAsync(tail_maps, m.data(), m.size() * sizeof(TailMaps), cudaMemcpyHostToDevice, st));
+        CT_CK(cudaMemcpyAsync(tail_table, table.data(), (size_t)best.table_bytes, cudaMemcpyHostToDevice, st));
+        CT_CK(cudaStreamSynchronize(st));
+        tail = best;
+        small_k0 = k0;
+        return CT_OK;
+    }
+    return CT_OK;
+}
+
 ct_status Solver::set_dt(double dt) {
     const TraceRange trace("ct_set_dt");
     if (!(dt >= 0) || !std::isfinite(dt)) return fail(CT_BAD_ARG, "ct_set_dt: dt must be >= 0");
@@ -385,7 +426,8 @@ void Solver::vcycle(size_t k, Cond cond, bool first_sweep_done) {
             b += (double)g.nx * g.ny * g.nz * (7 * sizeof(T) + 12);
         }
         enq(("mg_small_l" + std::to_string(k)).c_str(), b, [&] {
-            const cudaError_t e = launch_vsmall<T>(cs, tl, ctl, cond);
+            const cudaError_t e =
+                sizeof(T) == 4 && tail.n > 0 ? launch_tail(cs, tail, tail_maps, tail_table, ctl, cond) : launch_vsmall<T>(cs, tl, ctl, cond);
             if (e != cudaSuccess && launch_error == cudaSuccess) launch_error = e;
         });
         return;

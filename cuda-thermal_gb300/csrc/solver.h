@@ -83,6 +83,9 @@ class Solver {
     bool use_graphs = true;
     bool have_cond = false;
     size_t small_k0 = 0;   // levels from small_k0 down run in one block from shared memory
+    TailPlan tail{};       // FP32: those levels in one cluster launch (tail.n > 0)
+    TailMaps* tail_maps = nullptr;
+    int* tail_table = nullptr;
     bool fuse_sweep0 = true;  // a level's first (x = 0) sweep rides with the restriction into it
     bool sweep0_grid = true;  // x = 0 sweeps of the staged levels on the grid kernel
     // x += alpha p beside the next V-cycle (FP64 outer loop, multigrid): a
@@ -208,6 +211,7 @@ class Solver {
     ct_status async_status = CT_OK;
     ct_stats async_done{};
     ct_status record_graphs();
+    ct_status choose_tail(size_t smem_max);
 
     // Enqueues one kernel launch; in profiling mode brackets it with events.
     template <class F>
