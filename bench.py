@@ -727,11 +727,11 @@ def profile_rows(solver):
 
 
 # FP64 instructions per cell of the FP64 outer kernels (CT_MG_FP32_FLEX;
-# k_fp64.cu): 7 DFMA for (A + C/dt) p and 1 for p.Ap; r and ||r||^2 (x
-# += alpha p runs beside the next V-cycle: pcg_update_x); r.z and z.Ap; p = z
-# + beta p; ||b||^2 of a start from x = 0. Conversions are integer operations.
-FP64_OPS = {"pcg_apply": 8, "pcg_update_xr": 2, "pcg_update_x": 1, "pcg_dot": 2, "pcg_update_p": 1,
-            "pcg_residual": 1}
+# k_fp64.cu): the diagonal's product of A z and r.z, z.Ap, z.Az (the faces'
+# products are added up on the FP32 and integer pipes); p, Ap, r and ||r||^2
+# (x += alpha p runs beside the next V-cycle: pcg_update_x); ||b||^2 of a start
+# from x = 0. Conversions are integer operations.
+FP64_OPS = {"pcg_apply": 4, "pcg_update_xr": 4, "pcg_update_x": 1, "pcg_residual": 1}
 
 
 def kernel_table(rows, n=10, cells=None, dfma=None):
@@ -960,9 +960,9 @@ def main():
                            "launch_ms": top["total_ms"] / top["launches"],
                            "share": top["total_ms"] / tot_ms,
                            "solve_frac": alg_bytes_solve / (msfx / args.steps / 1e3) / 1e9 / hbm_peak}
-        out["roofline"]["note"] = ("the dominant kernel, the FP64 operator apply, is bound by the FP64 pipe "
-                                   "(8 DFMA a cell), not by HBM: fp64_pipe.frac; the smoother's HBM "
-                                   "roofline is smoother.frac")
+        out["roofline"]["note"] = ("fp64_pipe: the operator on the V-cycle's z with the dot products "
+                                   "(pcg_apply, 4 FP64 instructions a cell); smoother: the level-0 "
+                                   "line-solve sweeps")
         sw = next((r for r in rows if r["name"] == "mg_sweep_l0"), None)
         if sw:
             sw_rate = sw["bytes"] / (sw["total_ms"] / 1e3) / 1e9

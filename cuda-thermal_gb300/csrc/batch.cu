@@ -208,7 +208,7 @@ class Batch {
 
     ct_status make_red(const Plan& p, BRed* r) {
         ct_status s;
-        if ((s = dalloc(&r->part, (size_t)2 * std::max(1, p.ntasks) * sizeof(double))) != CT_OK) return s;
+        if ((s = dalloc(&r->part, (size_t)3 * std::max(1, p.ntasks) * sizeof(double))) != CT_OK) return s;
         if ((s = dalloc(&r->tickets, (size_t)ni * sizeof(unsigned))) != CT_OK) return s;
         CT_BK(cudaMemsetAsync(r->tickets, 0, (size_t)ni * sizeof(unsigned), st));
         return CT_OK;
@@ -325,6 +325,7 @@ ct_status Batch::create(int n, const ct_model* const* models, const DeviceBuild*
         I.r64 = s.r;
         I.p64 = s.p;
         I.Ap64 = s.Ap;
+        I.w64 = s.w;
         I.n = s.n;
     }
     ct_status s;
@@ -715,11 +716,8 @@ void Batch::enqueue_body(Bucket& b, cudaStream_t s, Cond cond) {
     launch_b_guard(s, b.bc, cond);
     vcycle(b, s, cond);
     if (!dw) {
-        enq(s, "b_dot", N * 20, [&] { launch_b_dot64(s, b.vec, bi, ctl, b.r_dot, b.bc, cond); });
-        enq(s, "b_update_p", N * 20, [&] { launch_b_update_p64(s, b.vec, bi, ctl); });
-        enq(s, "b_apply", N * 36, [&] { launch_b_apply64(s, b.rows, bi, ctl, b.r_apply, b.bc, cond); });
-        enq(s, "b_update_xr", N * 52,
-            [&] { launch_b_update64(s, b.vec, bi, ctl, b.r_update, b.bc, cond); });
+        enq(s, "b_apply", N * 48, [&] { launch_b_az64(s, b.rows, bi, ctl, b.r_apply, b.bc, cond); });
+        enq(s, "b_update_xr", N * 80, [&] { launch_b_step64(s, b.vec, bi, ctl, b.r_update, b.bc, cond); });
         return;
     }
     enq(s, "b_dot", N * 20, [&] { launch_b_dot(s, b.vec, bi, ctl, b.r_dot, b.bc, cond); });

@@ -52,6 +52,7 @@ struct BInst {
     double* r64;    // r, p, Ap as doubles (the FP64 outer mode)
     double* p64;
     double* Ap64;
+    double* w64;    // A z
     unsigned n;     // slots of all planes
 };
 
@@ -64,7 +65,7 @@ struct BCtl {
 
 // Per-instance reduction bookkeeping of one stage.
 struct BRed {
-    double* part;       // 2 * ntasks doubles
+    double* part;       // 3 * ntasks doubles
     unsigned* tickets;  // per instance
 };
 
@@ -83,17 +84,11 @@ void launch_b_dot(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRe
 void launch_b_update_p(cudaStream_t st, const Plan& p, const BInst* bi, const Ctl* ctl);
 
 // ---- outer PCG in FP64 (CT_MG_FP32_FLEX), one launch for the batch, k_batch64.cu
-// Items: residual and apply, rows of one colour and plane; the others, value
-// pairs.
+// Items: residual and A z, rows of one colour and plane; the step, value pairs.
 void launch_b_residual64(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc,
                          Cond cond);
-void launch_b_apply64(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc,
-                      Cond cond);
-void launch_b_update64(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc,
-                       Cond cond);
-void launch_b_dot64(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc,
-                    Cond cond);
-void launch_b_update_p64(cudaStream_t st, const Plan& p, const BInst* bi, const Ctl* ctl);
+void launch_b_az64(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond);
+void launch_b_step64(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond);
 
 // ---- multigrid, one launch per stage and depth for the batch ----------------
 // views / cviews: this depth's and the next coarser depth's LevelView per

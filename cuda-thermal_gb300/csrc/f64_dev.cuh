@@ -102,6 +102,183 @@ __device__ __forceinline__ void stream_pipelined(unsigned first, unsigned end, u
     }
 }
 
+// n 2^x as a double, to nearest even, for |n| < 2^63 and results in the normal
+// range, by integer operations (the conversion instruction holds the FP64 pipe).
+// Ties are common (sums of a few 48-bit products) and A z is a small difference
+// of large sums: rounding them away from zero moved the fields by 1e-12.
+__device__ __forceinline__ double fixed_to_double(long long n, int x) {
+    const unsigned hi = (unsigned)((unsigned long long)n >> 32);
+    unsigned long long u = n < 0 ? 0ull - (unsigned long long)n : (unsigned long long)n;
+    const int lz = __clzll((long long)(u | 1ull));
+    u <<= lz - 1;  // bit 62 set
+    // 53 bits, the leading one adding 1 to the exponent field
+    const unsigned long long m = (u + 0x1ffull + ((u >> 10) & 1ull)) >> 10;
+    const unsigned long long bits = m + ((unsigned long long)(unsigned)(1023 + 62 - lz + x) << 52);
+    return n == 0 ? 0.0 : __longlong_as_double((long long)(bits | ((unsigned long long)(hi & 0x80000000u) << 32)));
+}
+
+// ---- A z of the V-cycle's float z ------------------------------------------------
+//
+// The sum of six float x float products, correctly summed to better than a
+// double's rounding without the FP64 pipe (six DFMA a cell would hold the
+// operator at 72 us of FP64 issue at 800 x 800 x 10). Each product is split
+// exactly into h + l (one multiplication, one fused multiply-add). With 2^k above
+// every |h|, adding the constant 1.5 2^23 q rounds a value to a multiple of q and
+// leaves that multiple in the sum's mantissa bits, so integer sums of those bits
+// add the rounded parts exactly: h at q = 2^(k-19), its remainder and l at
+// 2^(k-39), what is left of both at 2^(k-59). The three integers are one 64-bit
+// integer in units of 2^(k-59): error at most 6 x 2^(k-60), i.e. 2^-56 of the
+// largest term, against 2^-53 of the partial sums for a chain of DFMA. Terms
+// outside 2^-91 .. 2^122 (and all six zero) take that chain.
+__device__ __forceinline__ double sum6(const float (&g)[6], const float (&z)[6]) {
+    float h[6], l[6], m = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        h[i] = __fmul_rn(g[i], z[i]);
+        l[i] = __fmaf_rn(g[i], z[i], -h[i]);
+        m = fmaxf(m, fabsf(h[i]));
+    }
+    const unsigned e = __float_as_uint(m) >> 23;  // 2^k has the biased exponent e + 1
+    if (e - 36u <= 213u) {
+        const unsigned half = 0x400000u;  // 1.5's mantissa
+        const unsigned b1 = ((e + 5u) << 23) | half, b2 = ((e - 15u) << 23) | half, b3 = ((e - 35u) << 23) | half;
+        const float c1 = __uint_as_float(b1), c2 = __uint_as_float(b2), c3 = __uint_as_float(b3);
+        unsigned n1 = 0u - 6u * b1, n2 = 0u - 12u * b2, n3 = 0u - 6u * b3;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            const float t1 = __fadd_rn(h[i], c1), r = __fsub_rn(h[i], __fsub_rn(t1, c1));
+            const float t2 = __fadd_rn(r, c2), r2 = __fsub_rn(r, __fsub_rn(t2, c2));
+            const float t3 = __fadd_rn(l[i], c2), l2 = __fsub_rn(l[i], __fsub_rn(t3, c2));
+            const float t4 = __fadd_rn(__fadd_rn(r2, l2), c3);
+            n1 += __float_as_uint(t1);
+            n2 += __float_as_uint(t2) + __float_as_uint(t3);
+            n3 += __float_as_uint(t4);
+        }
+        const long long n = ((long long)(int)n1 << 40) + ((long long)(int)n2 << 20) + (long long)(int)n3;
+        return fixed_to_double(n, (int)e - 185);
+    }
+    double off = 0.0;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) off = __fma_rn(widen(g[i]), widen(z[i]), off);
+    return off;
+}
+// The same for the FP64 V-cycle's z (west, east, south, north, down, up).
+__device__ __forceinline__ double sum6(const float (&g)[6], const double (&z)[6]) {
+    double off = 0.0;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) off = __fma_rn(widen(g[i]), z[i], off);
+    return off;
+}
+
+// Operands of (A + C/dt) z at one cell, loaded before any is used; an absent
+// neighbour has a zero face (and a zero value).
+template <class T>
+struct CellZ {
+    T zc, z[6];
+    float g[6];
+    double dg;
+};
+template <class T>
+__device__ __forceinline__ void load_z(const OpView& o, const double* __restrict__ diag, const T* __restrict__ z,
+                                       unsigned k, unsigned t, unsigned orow, int i, int e, bool hs, bool hn, bool hd,
+                                       bool hu, CellZ<T>& a) {
+    const Geo& g = o.g;
+    const unsigned hx = (unsigned)g.hx;
+    a.zc = z[k];
+    a.dg = diag[k];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        a.z[q] = T(0);
+        a.g[q] = 0.0f;
+    }
+    if (i > 0) {
+        const unsigned w = orow + t - 1u + (unsigned)e;
+        a.z[0] = z[w];
+        a.g[0] = o.gE[w];
+    }
+    if (i < g.nx - 1) {
+        a.z[1] = z[orow + t + (unsigned)e];
+        a.g[1] = o.gE[k];
+    }
+    if (hs) {
+        const unsigned s = orow - 2u * hx + t;
+        a.z[2] = z[s];
+        a.g[2] = o.gN[s];
+    }
+    if (hn) {
+        a.z[3] = z[orow + 2u * hx + t];
+        a.g[3] = o.gN[k];
+    }
+    if (hd) {
+        a.z[4] = z[k - g.plane];
+        a.g[4] = o.gU[k - g.plane];
+    }
+    if (hu) {
+        a.z[5] = z[k + g.plane];
+        a.g[5] = o.gU[k];
+    }
+}
+
+// Row R = l * 2 ny + 2 j + colour of (A + C/dt) z: the calling warp strides over
+// its slots, U cells a lane and step; load(slot) brings whatever else f needs,
+// with the operands, and f(slot, that, (A + C/dt) z, z) follows for each cell in
+// order. Padding slots are left alone.
+template <int U, class T, class Load, class F>
+__device__ __forceinline__ void row_z(const OpView& o, const double* __restrict__ diag, const T* __restrict__ z,
+                                      unsigned R, int lane, Load&& load, F&& f) {
+    const Geo& g = o.g;
+    const unsigned rows = 2u * (unsigned)g.ny;
+    const unsigned l = R / rows;
+    const unsigned r = R - l * rows;
+    const int j = (int)(r >> 1), c = (int)(r & 1u), e = (j + c) & 1;
+    const unsigned hx = (unsigned)g.hx;
+    const unsigned base = l * g.plane;
+    const unsigned row = base + r * hx;
+    const unsigned orow = base + (unsigned)(2 * j + (c ^ 1)) * hx;  // other colour, same j
+    const bool hs = j > 0, hn = j < g.ny - 1, hd = l > 0, hu = (int)l < g.nz - 1;
+    for (unsigned t0 = (unsigned)lane; t0 < hx; t0 += 32u * U) {
+        CellZ<T> a[U];
+        decltype(load(0u)) more[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const unsigned t = t0 + 32u * u;
+            const int i = 2 * (int)t + e;
+            if (t < hx && i < g.nx) {
+                load_z(o, diag, z, row + t, t, orow, i, e, hs, hn, hd, hu, a[u]);
+                more[u] = load(row + t);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const unsigned t = t0 + 32u * u;
+            const int i = 2 * (int)t + e;
+            if (t < hx && i < g.nx) {
+                const double zc = to_d(a[u].zc);
+                f(row + t, more[u], __fma_rn(a[u].dg, zc, -sum6(a[u].g, a[u].z)), zc);
+            }
+        }
+    }
+}
+
+// beta, p.Ap and alpha of the iteration that the V-cycle's z begins, from r.z,
+// z.Ap (Ap, pAp, rz of the iteration before) and z.Az: with p' = z + beta p,
+// A p' = A z + beta Ap, so p'.Ap' = z.Az + 2 beta z.Ap + beta^2 p.Ap. Flexible
+// beta (Polak-Ribiere): z_new.(r_new - r_old) / (z_old . r_old)
+// = -(z_new . Ap) / (p . Ap); otherwise Fletcher-Reeves (src/pcg3d_cpu.cpp:179).
+// False (a breakdown): a value is not finite, or p.Ap <= 0 (A is SPD).
+struct Scalars {
+    double beta, pAp, alpha;
+};
+__device__ __forceinline__ bool next_scalars(bool flex, bool first, double rz, double zAp, double zAz, double rz_old,
+                                             double pAp_old, Scalars& s) {
+    s.beta = first ? 0.0 : flex ? -zAp / pAp_old : rz / rz_old;
+    s.pAp = first ? zAz : __fma_rn(s.beta, __fma_rn(s.beta, pAp_old, 2.0 * zAp), zAz);
+    s.alpha = 0.0;
+    if (!isfinite(rz) || !isfinite(s.beta) || !(s.pAp > 0.0) || !isfinite(s.pAp)) return false;
+    s.alpha = rz / s.pAp;
+    return true;
+}
+
 // ---- the FP64 operator apply, one warp per row (single solver and batch) ----
 
 // Operands of one cell, loaded before any is used (absent neighbours stay

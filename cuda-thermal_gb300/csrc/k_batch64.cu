@@ -1,8 +1,7 @@
 // k_batch64.cu - the batched solver's FP64 outer PCG (CT_MG_FP32_FLEX): the
-// start residual, operator apply, x/r update, dot products and p update of
-// every instance of a bucket, one launch each, in IEEE double arithmetic as
-// the single solver's k_fp64.cu (same per-cell code, f64_dev.cuh: the fewest
-// FP64 instructions, float <-> double conversions by integer operations).
+// start residual, A z with the dot products, and the p, Ap, x, r update of every
+// instance of a bucket, one launch each, in IEEE double arithmetic as the
+// single solver's k_fp64.cu (same per-cell code, f64_dev.cuh).
 // Block tables and per-instance reductions as in k_batch.cu (batch.h).
 #include <cmath>
 
@@ -92,80 +91,110 @@ __global__ void __launch_bounds__(NT)
     }
 }
 
-// Ap = (A + C/dt) p, p.Ap, alpha; items = rows of one colour and plane.
-__global__ void __launch_bounds__(NT)
-    kb_apply64(Plan p, const BInst* __restrict__ bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
+// w = (A + C/dt) z, r.z, z.Ap, z.w, then the instance's beta, p.Ap and alpha
+// (k_az64); items = rows of one colour and plane.
+__global__ void __launch_bounds__(NT, 4)
+    kb_az64(Plan p, const BInst* __restrict__ bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
     pdl_enter();
     const Task t = p.tasks[blockIdx.x];
     Ctl* c = &ctl[t.inst];
     if (inst_done(c)) return;
-    const BInst I = bi[t.inst];
+    const BInst& I = bi[t.inst];
+    const OpView o = I.o;
+    const double *const r = I.r64, *const Ap = I.Ap64;
+    double* const w = I.w64;
+    const bool first = c->iter == 0;  // no Ap yet
     const int lane = (int)(threadIdx.x & 31u);
-    double pap = 0.0, unused = 0.0;
+    double v[3] = {0.0, 0.0, 0.0};
+    struct More {
+        double r, ap;
+    };
     for (unsigned R = t.begin + (threadIdx.x >> 5); R < t.end; R += NT / 32)
-        row64<kRowU>(I.o, I.diag, I.p64, R, lane, [&](unsigned k, bool valid, double av, double pc) {
-            I.Ap64[k] = av;
-            if (valid) pap = __fma_rn(pc, av, pap);
-        });
+        row_z<1, float>(
+            o, I.diag, I.z, R, lane, [&](unsigned k) { return More{r[k], first ? 0.0 : Ap[k]}; },
+            [&](unsigned k, const More& m, double az, double zc) {
+                w[k] = az;
+                v[0] = __fma_rn(m.r, zc, v[0]);
+                v[1] = __fma_rn(zc, m.ap, v[1]);
+                v[2] = __fma_rn(zc, az, v[2]);
+            });
     pdl_trigger();
-    block_sum2(pap, unused);
-    if (publish_inst(pap, unused, red, p.ntasks, t.inst, p.inst_count[t.inst])) {
-        double PAP, U;
-        gather_inst(red, p.ntasks, t.inst, p.inst_first[t.inst], p.inst_count[t.inst], PAP, U);
+    const unsigned count = (unsigned)p.inst_count[t.inst];
+    if (publish_sums<3>(v, red.part, p.ntasks, blockIdx.x, &red.tickets[t.inst], count)) {
+        double s3[3];
+        gather_sums<3>(red.part, p.ntasks, (unsigned)p.inst_first[t.inst], count, &red.tickets[t.inst], s3);
         if (threadIdx.x == 0) {
-            c->pAp = PAP;
-            if (!(PAP > 0.0) || !isfinite(PAP)) {
+            Scalars s;
+            const bool ok = next_scalars(true, first, s3[0], s3[1], s3[2], c->rz, c->pAp, s);
+            c->rz = s3[0];
+            c->zAp = s3[1];
+            c->beta = s.beta;
+            c->pAp = s.pAp;
+            c->alpha = s.alpha;
+            if (!ok) {
                 c->breakdown = 1;
-                c->alpha = 0.0;
                 inst_stop(c, bc, cond);
-            } else {
-                c->alpha = c->rz / PAP;
             }
         }
     }
 }
 
-// x += alpha p, r -= alpha Ap, b0 = r (float), ||r||^2, the instance's
-// convergence test; items = value pairs.
+// p = z + beta p, Ap = w + beta Ap (p = z and Ap = w on the first iteration),
+// x += alpha p, r -= alpha Ap, b0 = r (float), ||r||^2 and the instance's
+// convergence test (k_step64); items = value pairs.
 __global__ void __launch_bounds__(NT)
-    kb_update64(Plan p, const BInst* __restrict__ bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
+    kb_step64(Plan p, const BInst* __restrict__ bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
     pdl_enter();
     const Task t = p.tasks[blockIdx.x];
     Ctl* c = &ctl[t.inst];
     if (inst_done(c)) return;
-    const BInst I = bi[t.inst];
-    const double alpha = c->alpha, malpha = -alpha;
-    const double2* __restrict__ p2 = reinterpret_cast<const double2*>(I.p64);
-    const double2* __restrict__ a2 = reinterpret_cast<const double2*>(I.Ap64);
+    const BInst& I = bi[t.inst];
+    const double alpha = c->alpha, malpha = -alpha, beta = c->beta;
+    const bool first = c->iter == 0;
+    const float2* __restrict__ z2 = reinterpret_cast<const float2*>(I.z);
+    const double2* __restrict__ w2 = reinterpret_cast<const double2*>(I.w64);
+    double2* __restrict__ p2 = reinterpret_cast<double2*>(I.p64);
+    double2* __restrict__ a2 = reinterpret_cast<double2*>(I.Ap64);
     double2* __restrict__ x2 = reinterpret_cast<double2*>(I.x);
     double2* __restrict__ r2 = reinterpret_cast<double2*>(I.r64);
     float2* __restrict__ b02 = reinterpret_cast<float2*>(I.b0);
-    double rr = 0.0, unused = 0.0;
+    double v[1] = {0.0};
     struct Item {
-        double2 p, a, x, r;
+        float2 z;
+        double2 w, p, a, x, r;
     };
     stream_pipelined<1, Item>(
-        t.begin + threadIdx.x, t.end, NT, [&](unsigned k) { return Item{p2[k], a2[k], x2[k], r2[k]}; },
+        t.begin + threadIdx.x, t.end, NT,
+        [&](unsigned k) {
+            const double2 none = make_double2(0.0, 0.0);
+            return Item{z2[k], w2[k], first ? none : p2[k], first ? none : a2[k], x2[k], r2[k]};
+        },
         [&](unsigned k, Item it) {
+            it.p.x = __fma_rn(beta, it.p.x, widen(it.z.x));
+            it.p.y = __fma_rn(beta, it.p.y, widen(it.z.y));
+            it.a.x = __fma_rn(beta, it.a.x, it.w.x);
+            it.a.y = __fma_rn(beta, it.a.y, it.w.y);
             it.x.x = __fma_rn(alpha, it.p.x, it.x.x);
             it.x.y = __fma_rn(alpha, it.p.y, it.x.y);
             it.r.x = __fma_rn(malpha, it.a.x, it.r.x);
             it.r.y = __fma_rn(malpha, it.a.y, it.r.y);
+            p2[k] = it.p;
+            a2[k] = it.a;
             x2[k] = it.x;
             r2[k] = it.r;
             b02[k] = make_float2(narrow(it.r.x), narrow(it.r.y));
-            rr = __fma_rn(it.r.x, it.r.x, rr);
-            rr = __fma_rn(it.r.y, it.r.y, rr);
+            v[0] = __fma_rn(it.r.x, it.r.x, v[0]);
+            v[0] = __fma_rn(it.r.y, it.r.y, v[0]);
         });
     pdl_trigger();
-    block_sum2(rr, unused);
-    if (publish_inst(rr, unused, red, p.ntasks, t.inst, p.inst_count[t.inst])) {
-        double RR, U;
-        gather_inst(red, p.ntasks, t.inst, p.inst_first[t.inst], p.inst_count[t.inst], RR, U);
+    const unsigned count = (unsigned)p.inst_count[t.inst];
+    if (publish_sums<1>(v, red.part, p.ntasks, blockIdx.x, &red.tickets[t.inst], count)) {
+        double rr[1];
+        gather_sums<1>(red.part, p.ntasks, (unsigned)p.inst_first[t.inst], count, &red.tickets[t.inst], rr);
         if (threadIdx.x == 0) {
-            c->rr = RR;
+            c->rr = rr[0];
             c->iter += 1;
-            const double rel = sqrt(RR / c->bb);
+            const double rel = sqrt(rr[0] / c->bb);
             c->relres = rel;
             if (rel < c->tol) {
                 c->converged = 1;
@@ -180,78 +209,6 @@ __global__ void __launch_bounds__(NT)
     }
 }
 
-// rz = r.z, z.Ap, flexible beta; items = value pairs.
-__global__ void __launch_bounds__(NT)
-    kb_dot64(Plan p, const BInst* __restrict__ bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
-    pdl_enter();
-    const Task t = p.tasks[blockIdx.x];
-    Ctl* c = &ctl[t.inst];
-    if (inst_done(c)) return;
-    const BInst I = bi[t.inst];
-    const double2* __restrict__ r2 = reinterpret_cast<const double2*>(I.r64);
-    const double2* __restrict__ a2 = reinterpret_cast<const double2*>(I.Ap64);
-    const float2* __restrict__ z2 = reinterpret_cast<const float2*>(I.z);
-    double rz = 0.0, zap = 0.0;
-    struct Item {
-        double2 r, a;
-        float2 z;
-    };
-    stream_pipelined<2, Item>(
-        t.begin + threadIdx.x, t.end, NT, [&](unsigned k) { return Item{r2[k], a2[k], z2[k]}; },
-        [&](unsigned, const Item& it) {
-            const double za = widen(it.z.x), zb = widen(it.z.y);
-            rz = __fma_rn(it.r.x, za, rz);
-            rz = __fma_rn(it.r.y, zb, rz);
-            zap = __fma_rn(za, it.a.x, zap);
-            zap = __fma_rn(zb, it.a.y, zap);
-        });
-    pdl_trigger();
-    block_sum2(rz, zap);
-    if (publish_inst(rz, zap, red, p.ntasks, t.inst, p.inst_count[t.inst])) {
-        double RZ, ZAP;
-        gather_inst(red, p.ntasks, t.inst, p.inst_first[t.inst], p.inst_count[t.inst], RZ, ZAP);
-        if (threadIdx.x == 0) {
-            c->beta = c->iter > 0 ? -ZAP / c->pAp : 0.0;
-            c->rz = RZ;
-            c->zAp = ZAP;
-            if (!isfinite(RZ) || !isfinite(c->beta)) {
-                c->breakdown = 1;
-                inst_stop(c, bc, cond);
-            }
-        }
-    }
-}
-
-// p = z + beta p (p = z on the first iteration); items = value pairs.
-__global__ void __launch_bounds__(NT)
-    kb_update_p64(Plan p, const BInst* __restrict__ bi, const Ctl* ctl) {
-    pdl_enter();
-    const Task t = p.tasks[blockIdx.x];
-    const Ctl* c = &ctl[t.inst];
-    if (inst_done(c)) return;
-    const BInst I = bi[t.inst];
-    const double beta = c->beta;
-    const bool first = c->iter == 0;
-    const float2* __restrict__ z2 = reinterpret_cast<const float2*>(I.z);
-    double2* __restrict__ p2 = reinterpret_cast<double2*>(I.p64);
-    if (first) {
-        for (unsigned k = t.begin + threadIdx.x; k < t.end; k += NT) {
-            const float2 zf = z2[k];
-            p2[k] = make_double2(widen(zf.x), widen(zf.y));
-        }
-        return;
-    }
-    struct Item {
-        double2 p;
-        float2 z;
-    };
-    stream_pipelined<2, Item>(
-        t.begin + threadIdx.x, t.end, NT, [&](unsigned k) { return Item{p2[k], z2[k]}; },
-        [&](unsigned k, const Item& it) {
-            p2[k] = make_double2(__fma_rn(beta, it.p.x, widen(it.z.x)), __fma_rn(beta, it.p.y, widen(it.z.y)));
-        });
-}
-
 }  // namespace
 
 void launch_b_residual64(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc,
@@ -259,23 +216,12 @@ void launch_b_residual64(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* c
     launch_pdl(kb_residual64, p.ntasks, NT, 0, st, p, bi, ctl, red, bc, cond);
 }
 
-void launch_b_apply64(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc,
-                      Cond cond) {
-    launch_pdl(kb_apply64, p.ntasks, NT, 0, st, p, bi, ctl, red, bc, cond);
+void launch_b_az64(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
+    launch_pdl(kb_az64, p.ntasks, NT, 0, st, p, bi, ctl, red, bc, cond);
 }
 
-void launch_b_update64(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc,
-                       Cond cond) {
-    launch_pdl(kb_update64, p.ntasks, NT, 0, st, p, bi, ctl, red, bc, cond);
-}
-
-void launch_b_dot64(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc,
-                    Cond cond) {
-    launch_pdl(kb_dot64, p.ntasks, NT, 0, st, p, bi, ctl, red, bc, cond);
-}
-
-void launch_b_update_p64(cudaStream_t st, const Plan& p, const BInst* bi, const Ctl* ctl) {
-    launch_pdl(kb_update_p64, p.ntasks, NT, 0, st, p, bi, ctl);
+void launch_b_step64(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
+    launch_pdl(kb_step64, p.ntasks, NT, 0, st, p, bi, ctl, red, bc, cond);
 }
 
 }  // namespace ct

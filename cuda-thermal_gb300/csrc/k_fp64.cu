@@ -4,19 +4,20 @@
 // outer iteration is (Real = double, src/pcg3d.h:18-22; k_residual,
 // k_apply, k_update_xr, k_mg_dot, k_update_p_mg, src/pcg3d_gpu.cu:159-256).
 //
-// On GB300 these kernels are bound by the FP64 pipe, not by HBM: a DFMA
-// issues at ~1/70 of the FFMA rate (0.53 T/s on 152 SMs), so at 800 x 800 x
-// 10 every FP64 instruction per cell costs ~12 us while an 8-byte stream
-// costs ~7.5 us at the measured copy bandwidth. So each kernel does the
-// fewest FP64 instructions the algorithm needs: the float face conductances
-// and V-cycle values are widened to double, and the residual narrowed to the
-// V-cycle's float, with exact integer conversions (f64_dev.cuh) instead of
-// the FP64-rate hardware conversions, and every multiply-add is one DFMA.
-// Per cell: apply 8 (7 for Ap, 1 for p.Ap), update 3, dot 2, p update 1.
-// The memory side follows the double-word kernels (k_dw.cu): the apply runs
-// one warp per row of one colour and plane (no index division per cell),
-// the streaming kernels keep several items in flight per thread, and every
-// kernel is launched with programmatic dependent launch.
+// On GB300 FP64 arithmetic is scarce: a DFMA issues at ~1/70 of the FFMA rate
+// (0.53 T/s on 152 SMs), so at 800 x 800 x 10 every FP64 instruction per cell
+// costs ~12 us while an 8-byte stream costs ~7.5 us at the measured copy
+// bandwidth. So each kernel does the fewest FP64 instructions the algorithm
+// needs, and few kernels touch each vector: the V-cycle's float faces and values
+// are widened, and the residual narrowed to the V-cycle's float, with exact
+// integer conversions (f64_dev.cuh) instead of the FP64-rate hardware
+// conversions; the operator acts on the V-cycle's float z, whose products it
+// adds up on the FP32 and integer pipes (sum6), in the same pass as the dot
+// products (k_az64); and p, Ap and r follow in one more (k_step64). Per cell 4
+// FP64 instructions each.
+// The row kernels run one warp per row of one colour and plane (no index
+// division per cell), the streaming kernels keep several items in flight per
+// thread, and every kernel is launched with programmatic dependent launch.
 #include <algorithm>
 #include <cmath>
 
@@ -30,9 +31,67 @@ using namespace f64dev;
 
 namespace {
 
-constexpr int kRowU = 2;
+constexpr int kRowU = 2;  // cells a lane and step of the rows of A p
+constexpr int kRowZ = 1;  // and of A z
 
-// Ap = (A + C/dt) p, p.Ap and alpha = rz / p.Ap.
+// w = (A + C/dt) z, r.z, z.Ap (the Ap of the iteration before), z.w; then beta,
+// p.Ap and alpha. One warp per row of one colour and plane, two cells a lane.
+//
+// The operator acts on z, not on p: the V-cycle's z is a float, so its products
+// with the float faces are exact in two floats and their sum runs on the FP32
+// and integer pipes (sum6), where A p of the double p took seven DFMA a cell;
+// p = z + beta p and Ap = w + beta Ap follow together in k_step64. Per cell 4
+// FP64 instructions and 48 B (with the FP64 V-cycle 10 and 52), in place of the
+// 8 of A p and 2 of the dots and 56 B, and no launch, grid
+// reduction and second pass over r and Ap between them. 800 x 800 x 10:
+// 82 us a launch (105 compiled for two cells a lane
+// and the compiler's 101 registers, 94 / 82 / 87 for one cell at 2 / 5 / 6 blocks
+// per SM against 4; the next cells' loads ahead of this one's arithmetic 84 to
+// 98), against 107 + 37 for A p and the dots; the FP64 pipe is 60 % busy, memory
+// 44 %, issue 57 %, each warp going from one to the other.
+template <class T, bool FLEX>
+__global__ void __launch_bounds__(NT, 4)
+    k_az64(OpView o, const double* __restrict__ diag, const T* __restrict__ z, const double* __restrict__ r,
+           const double* __restrict__ Ap, double* __restrict__ w, Ctl* ctl, double* part, int maxb, Cond cond) {
+    pdl_enter();
+    if (loop_done(ctl, cond)) return;
+    const bool first = ctl->iter == 0;  // no Ap yet
+    const unsigned rows = 2u * (unsigned)o.g.ny * (unsigned)o.g.nz;
+    const int lane = (int)(threadIdx.x & 31u);
+    double v[3] = {0.0, 0.0, 0.0};
+    struct More {
+        double r, ap;
+    };
+    for (unsigned R = blockIdx.x * (NT / 32) + (threadIdx.x >> 5); R < rows; R += gridDim.x * (NT / 32))
+        row_z<kRowZ, T>(
+            o, diag, z, R, lane, [&](unsigned k) { return More{r[k], first ? 0.0 : Ap[k]}; },
+            [&](unsigned k, const More& m, double az, double zc) {
+                w[k] = az;
+                v[0] = __fma_rn(m.r, zc, v[0]);
+                v[1] = __fma_rn(zc, m.ap, v[1]);
+                v[2] = __fma_rn(zc, az, v[2]);
+            });
+    pdl_trigger();
+    if (publish_sums<3>(v, part, maxb, blockIdx.x, &ctl->ticket[SL_APPLY], gridDim.x)) {
+        double t[3];
+        gather_sums<3>(part, maxb, 0u, gridDim.x, &ctl->ticket[SL_APPLY], t);
+        if (threadIdx.x == 0) {
+            Scalars s;
+            const bool ok = next_scalars(FLEX, first, t[0], t[1], t[2], ctl->rz, ctl->pAp, s);
+            ctl->rz = t[0];
+            ctl->zAp = t[1];
+            ctl->beta = s.beta;
+            ctl->pAp = s.pAp;
+            ctl->alpha = s.alpha;
+            if (!ok) {
+                ctl->breakdown = 1;
+                stop_loop(ctl, cond);
+            }
+        }
+    }
+}
+
+// Ap = (A + C/dt) p, p.Ap and alpha = rz / p.Ap (the Jacobi form).
 __global__ void __launch_bounds__(NT)
     k_apply64(OpView o, const double* __restrict__ diag, const double* __restrict__ p,
               double* __restrict__ Ap, Ctl* ctl, double* part, int maxb, Cond cond) {
@@ -103,14 +162,6 @@ __device__ __forceinline__ Range block_range(unsigned n) {
     return Range{b + threadIdx.x, b + per < n ? b + per : n};
 }
 
-// Two values of the V-cycle's precision at pair index k, as doubles.
-__device__ __forceinline__ double2 load_pair(const float* z, unsigned k) {
-    const float2 v = reinterpret_cast<const float2*>(z)[k];
-    return make_double2(widen(v.x), widen(v.y));
-}
-__device__ __forceinline__ double2 load_pair(const double* z, unsigned k) {
-    return reinterpret_cast<const double2*>(z)[k];
-}
 __device__ __forceinline__ void store_pair(float* b0, unsigned k, double a, double b) {
     reinterpret_cast<float2*>(b0)[k] = make_float2(narrow(a), narrow(b));
 }
@@ -170,68 +221,82 @@ __global__ void __launch_bounds__(NT)
     }
 }
 
-// x += alpha p, r -= alpha Ap, b0 = r in the V-cycle precision, ||r||^2 and
-// the convergence test (src/pcg3d_gpu.cu:218-233). Pairs of values (double2),
-// each block a contiguous range.
-constexpr int kUpdU = 1;
-struct UpdItem {
-    double2 p, a, x, r;
-};
-struct UpdItemR {
-    double2 a, r;
-};
+// p = z + beta p, Ap = w + beta Ap (p = z and Ap = w on the first iteration),
+// r -= alpha Ap, b0 = r in the V-cycle precision, ||r||^2 and the convergence
+// test (src/pcg3d_gpu.cu:218-256). Pairs of values (double2), each block a
+// contiguous range.
 // WX = false: x is left to k_update_x64 (x += alpha p off the critical path,
-// beside the next V-cycle); alpha is kept in ctl->alpha_x for it.
-// The r-only form keeps 4 pairs in flight a thread (98 registers): 36.8 us
-// against 40.9 us with 2 and 43.0 us with 1 at 800 x 800.
-template <class T, bool WX, int UR = 4>
+// beside the next V-cycle); alpha is kept in ctl->alpha_x for it. The x update
+// that was pending at entry has run by then: none is pending when the loop has
+// ended.
+// 4 FP64 instructions and 60 B a cell. 800 x 800 x 10: 73 us (5.6 TB/s), against
+// 22 + 37 for the p update and the update of r alone.
+template <class T>
+struct Pair;
+template <>
+struct Pair<float> {
+    typedef float2 type;
+};
+template <>
+struct Pair<double> {
+    typedef double2 type;
+};
+__device__ __forceinline__ double2 to_d(float2 v) { return make_double2(widen(v.x), widen(v.y)); }
+__device__ __forceinline__ double2 to_d(double2 v) { return v; }
+
+constexpr int kStepU = 2;
+template <class T, bool WX>
 __global__ void __launch_bounds__(NT)
-    k_update64(unsigned n2, const double2* __restrict__ p, const double2* __restrict__ Ap,
-               double2* __restrict__ x, double2* __restrict__ r, T* __restrict__ b0, Ctl* ctl,
-               double* part, int maxb, Cond cond) {
+    k_step64(unsigned n2, const T* __restrict__ z, const double2* __restrict__ w, double2* __restrict__ p,
+             double2* __restrict__ Ap, double2* __restrict__ x, double2* __restrict__ r, T* __restrict__ b0, Ctl* ctl,
+             double* part, int maxb, Cond cond) {
+    typedef typename Pair<T>::type Z2;
     pdl_enter();
-    if (loop_done(ctl, cond)) return;
-    const double alpha = ctl->alpha, malpha = -alpha;
-    double rr = 0.0, unused = 0.0;
-    const Range br = block_range<2>(n2);
-    if constexpr (WX) {
-        stream_pipelined<kUpdU, UpdItem>(
-            br.begin, br.end, NT,
-            [&](unsigned k) { return UpdItem{p[k], Ap[k], x[k], r[k]}; },
-            [&](unsigned k, UpdItem it) {
-                it.x.x = __fma_rn(alpha, it.p.x, it.x.x);
-                it.x.y = __fma_rn(alpha, it.p.y, it.x.y);
-                it.r.x = __fma_rn(malpha, it.a.x, it.r.x);
-                it.r.y = __fma_rn(malpha, it.a.y, it.r.y);
-                x[k] = it.x;
-                r[k] = it.r;
-                store_pair(b0, k, it.r.x, it.r.y);
-                rr = __fma_rn(it.r.x, it.r.x, rr);
-                rr = __fma_rn(it.r.y, it.r.y, rr);
-            });
-    } else {
-        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->alpha_x = alpha;
-        stream_pipelined<UR, UpdItemR>(
-            br.begin, br.end, NT,
-            [&](unsigned k) { return UpdItemR{Ap[k], r[k]}; },
-            [&](unsigned k, UpdItemR it) {
-                it.r.x = __fma_rn(malpha, it.a.x, it.r.x);
-                it.r.y = __fma_rn(malpha, it.a.y, it.r.y);
-                r[k] = it.r;
-                store_pair(b0, k, it.r.x, it.r.y);
-                rr = __fma_rn(it.r.x, it.r.x, rr);
-                rr = __fma_rn(it.r.y, it.r.y, rr);
-            });
-    }
+    const bool done = loop_done(ctl, cond);
+    const double alpha = ctl->alpha, malpha = -alpha, beta = ctl->beta;
+    if (!WX && blockIdx.x == 0 && threadIdx.x == 0) ctl->alpha_x = done ? 0.0 : alpha;
+    if (done) return;
+    const bool first = ctl->iter == 0;
+    const Z2* const z2 = reinterpret_cast<const Z2*>(z);
+    double v[1] = {0.0};
+    const Range br = block_range<kStepU>(n2);
+    struct Item {
+        Z2 z;
+        double2 w, p, a, r;
+    };
+    stream_pipelined<kStepU, Item>(
+        br.begin, br.end, NT,
+        [&](unsigned k) {
+            const double2 none = make_double2(0.0, 0.0);
+            return Item{z2[k], w[k], first ? none : p[k], first ? none : Ap[k], r[k]};
+        },
+        [&](unsigned k, Item it) {
+            const double2 zd = to_d(it.z);
+            it.p.x = __fma_rn(beta, it.p.x, zd.x);
+            it.p.y = __fma_rn(beta, it.p.y, zd.y);
+            it.a.x = __fma_rn(beta, it.a.x, it.w.x);
+            it.a.y = __fma_rn(beta, it.a.y, it.w.y);
+            it.r.x = __fma_rn(malpha, it.a.x, it.r.x);
+            it.r.y = __fma_rn(malpha, it.a.y, it.r.y);
+            p[k] = it.p;
+            Ap[k] = it.a;
+            r[k] = it.r;
+            store_pair(b0, k, it.r.x, it.r.y);
+            if (WX) {
+                const double2 xv = x[k];
+                x[k] = make_double2(__fma_rn(alpha, it.p.x, xv.x), __fma_rn(alpha, it.p.y, xv.y));
+            }
+            v[0] = __fma_rn(it.r.x, it.r.x, v[0]);
+            v[0] = __fma_rn(it.r.y, it.r.y, v[0]);
+        });
     pdl_trigger();
-    block_sum2(rr, unused);
-    if (publish2(rr, unused, part, maxb, &ctl->ticket[SL_UPDATE])) {
-        double RR, U;
-        gather2(part, maxb, &ctl->ticket[SL_UPDATE], RR, U);
+    if (publish_sums<1>(v, part, maxb, blockIdx.x, &ctl->ticket[SL_UPDATE], gridDim.x)) {
+        double t[1];
+        gather_sums<1>(part, maxb, 0u, gridDim.x, &ctl->ticket[SL_UPDATE], t);
         if (threadIdx.x == 0) {
-            ctl->rr = RR;
+            ctl->rr = t[0];
             ctl->iter += 1;
-            const double rel = sqrt(RR / ctl->bb);
+            const double rel = sqrt(t[0] / ctl->bb);
             ctl->relres = rel;
             if (rel < ctl->tol) {
                 ctl->converged = 1;
@@ -246,10 +311,10 @@ __global__ void __launch_bounds__(NT)
     }
 }
 
-// x += alpha p with the alpha k_update64<T, false> left in ctl->alpha_x (0:
+// x += alpha p with the alpha k_step64<T, false> left in ctl->alpha_x (0:
 // nothing pending), the same rounding as the fused update. It runs beside the
 // V-cycle of the next iteration (or after the loop for the last one) and
-// before the p update of that iteration, which clears alpha_x.
+// before that iteration's k_step64, which writes the next p and alpha_x.
 struct XItem {
     double2 p, x;
 };
@@ -262,123 +327,6 @@ __global__ void __launch_bounds__(NT)
         [&](unsigned k, const XItem& it) {
             x[k] = make_double2(__fma_rn(alpha, it.p.x, it.x.x), __fma_rn(alpha, it.p.y, it.x.y));
         });
-}
-
-// rz = r.z (and z.Ap for the flexible beta); beta (src/pcg3d_gpu.cu:239-247,
-// 121-126). Pairs strided over the whole grid.
-constexpr int kDotU = 2;
-struct DotItem {
-    double2 r, z, a;
-};
-template <class T>
-struct DotItemN {
-    double2 r;
-    float2 z;
-    double2 a;
-};
-template <class T, bool FLEX, int DU = kDotU>
-__global__ void __launch_bounds__(NT)
-    k_dot64(unsigned n2, const double2* __restrict__ r, const T* __restrict__ z,
-            const double2* __restrict__ Ap, Ctl* ctl, double* part, int maxb, Cond cond) {
-    pdl_enter();
-    if (loop_done(ctl, cond)) return;
-    double rz = 0.0, zap = 0.0;
-    if constexpr (sizeof(T) == 4) {
-        // z kept as loaded (a float pair) until it is used: 2 registers an item
-        // fewer than widening it at the load (42.7 -> 38.7 us at 800 x 800)
-        const float2* z2 = reinterpret_cast<const float2*>(z);
-        stream_pipelined<DU, DotItemN<T>>(
-            blockIdx.x * NT + threadIdx.x, n2, gridDim.x * NT,
-            [&](unsigned k) {
-                return DotItemN<T>{r[k], z2[k], FLEX ? Ap[k] : make_double2(0.0, 0.0)};
-            },
-            [&](unsigned, const DotItemN<T>& it) {
-                const double zx = widen(it.z.x), zy = widen(it.z.y);
-                rz = __fma_rn(it.r.x, zx, rz);
-                rz = __fma_rn(it.r.y, zy, rz);
-                if (FLEX) {
-                    zap = __fma_rn(zx, it.a.x, zap);
-                    zap = __fma_rn(zy, it.a.y, zap);
-                }
-            });
-    } else {
-        stream_pipelined<kDotU, DotItem>(
-            blockIdx.x * NT + threadIdx.x, n2, gridDim.x * NT,
-            [&](unsigned k) {
-                return DotItem{r[k], load_pair(z, k), FLEX ? Ap[k] : make_double2(0.0, 0.0)};
-            },
-            [&](unsigned, const DotItem& it) {
-                rz = __fma_rn(it.r.x, it.z.x, rz);
-                rz = __fma_rn(it.r.y, it.z.y, rz);
-                if (FLEX) {
-                    zap = __fma_rn(it.z.x, it.a.x, zap);
-                    zap = __fma_rn(it.z.y, it.a.y, zap);
-                }
-            });
-    }
-    pdl_trigger();
-    block_sum2(rz, zap);
-    if (publish2(rz, zap, part, maxb, &ctl->ticket[SL_DOT])) {
-        double RZ, ZAP;
-        gather2(part, maxb, &ctl->ticket[SL_DOT], RZ, ZAP);
-        if (threadIdx.x == 0) {
-            if (ctl->iter > 0) {
-                // Fletcher-Reeves (src/pcg3d_cpu.cpp:179) or flexible
-                // Polak-Ribiere: z_new.(r_new - r_old) / (z_old . r_old)
-                // = -(z_new . Ap) / (p . Ap).
-                ctl->beta = FLEX ? -ZAP / ctl->pAp : RZ / ctl->rz;
-            } else {
-                ctl->beta = 0.0;
-            }
-            ctl->rz = RZ;
-            ctl->zAp = ZAP;
-            if (!isfinite(RZ) || !isfinite(ctl->beta)) {
-                ctl->breakdown = 1;
-                stop_loop(ctl, cond);
-            }
-        }
-    }
-}
-
-// p = z + beta p (p = z on the first iteration; src/pcg3d_gpu.cu:249-256).
-constexpr int kPU = 2;
-struct PItem {
-    double2 z, p;
-};
-template <class T>
-__global__ void __launch_bounds__(NT)
-    k_update_p64(unsigned n2, const T* __restrict__ z, double2* __restrict__ p, Ctl* ctl,
-                 Cond cond) {
-    pdl_enter();
-    // the pending x update (k_update_x64) has run by now: none pending after
-    // this point, also when the loop has ended
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->alpha_x = 0.0;
-    if (loop_done(ctl, cond)) return;
-    const double beta = ctl->beta;
-    const Range br = block_range<2 * kPU>(n2);
-    if (ctl->iter == 0) {
-        for (unsigned k = br.begin; k < br.end; k += NT) p[k] = load_pair(z, k);
-        return;
-    }
-    if constexpr (sizeof(T) == 4) {
-        // z kept as loaded (a float pair) until it is used, as in k_dot64
-        struct Item {
-            float2 z;
-            double2 p;
-        };
-        const float2* z2 = reinterpret_cast<const float2*>(z);
-        stream_pipelined<kPU, Item>(
-            br.begin, br.end, NT, [&](unsigned k) { return Item{z2[k], p[k]}; },
-            [&](unsigned k, const Item& it) {
-                p[k] = make_double2(__fma_rn(beta, it.p.x, widen(it.z.x)), __fma_rn(beta, it.p.y, widen(it.z.y)));
-            });
-    } else {
-        stream_pipelined<kPU, PItem>(
-            br.begin, br.end, NT, [&](unsigned k) { return PItem{load_pair(z, k), p[k]}; },
-            [&](unsigned k, const PItem& it) {
-                p[k] = make_double2(__fma_rn(beta, it.p.x, it.z.x), __fma_rn(beta, it.p.y, it.z.y));
-            });
-    }
 }
 
 // ---- self-test of the integer conversions -----------------------------------
@@ -450,6 +398,25 @@ void launch_apply64(cudaStream_t st, const OpView& o, const double* diag, const 
     launch_pdl(k_apply64, std::min(red.maxb, wb), NT, 0, st, o, diag, p, Ap, ctl, red.part, red.maxb, cond);
 }
 
+void launch_az64(cudaStream_t st, MgType mt, bool flexible, const OpView& o, const double* diag, const void* z,
+                 const double* r, const double* Ap, double* w, Ctl* ctl, const Red& red, Cond cond) {
+    const int rows = 2 * o.g.ny * o.g.nz, want = std::max(1, (rows + NT / 32 - 1) / (NT / 32));
+    auto go = [&](auto kern, int wb, auto* zt) {
+        launch_pdl(kern, std::min(std::min(red.maxb, wb), want), NT, 0, st, o, diag, zt, r, Ap, w, ctl, red.part,
+                   red.maxb, cond);
+    };
+    if (mt == MG_F64) {
+        static const int wb = wave_blocks(k_az64<double, false>, 1 << 30);
+        go(k_az64<double, false>, wb, (const double*)z);
+    } else if (flexible) {
+        static const int wb = wave_blocks(k_az64<float, true>, 1 << 30);
+        go(k_az64<float, true>, wb, (const float*)z);
+    } else {
+        static const int wb = wave_blocks(k_az64<float, false>, 1 << 30);
+        go(k_az64<float, false>, wb, (const float*)z);
+    }
+}
+
 void launch_residual64(cudaStream_t st, MgType mt, const OpView& o, unsigned n, const double* diag,
                        const double* b, const double* x, double* r, void* b0, Ctl* ctl, const Red& red,
                        Cond cond) {
@@ -464,28 +431,25 @@ void launch_residual64(cudaStream_t st, MgType mt, const OpView& o, unsigned n, 
     }
 }
 
-void launch_update64(cudaStream_t st, MgType mt, unsigned n, const double* p, const double* Ap, double* x,
-                     double* r, void* b0, Ctl* ctl, const Red& red, Cond cond, bool write_x) {
+void launch_step64(cudaStream_t st, MgType mt, unsigned n, const void* z, const double* w, double* p, double* Ap,
+                   double* x, double* r, void* b0, Ctl* ctl, const Red& red, Cond cond, bool write_x) {
     const unsigned n2 = n / 2;
-    const auto* p2 = reinterpret_cast<const double2*>(p);
-    const auto* a2 = reinterpret_cast<const double2*>(Ap);
-    auto* x2 = reinterpret_cast<double2*>(x);
-    auto* r2 = reinterpret_cast<double2*>(r);
+    auto d2 = [](auto* q) { return reinterpret_cast<double2*>(q); };
     // (wave_blocks once per kernel: the four have their own occupancies)
-    auto go = [&](auto kern, int wb, auto* b) {
-        launch_pdl(kern, std::min(red.blocks, wb), NT, 0, st, n2, p2, a2, x2, r2, b, ctl, red.part, red.maxb,
-                   cond);
+    auto go = [&](auto kern, int wb, auto* zt, auto* b) {
+        launch_pdl(kern, std::min(red.blocks, wb), NT, 0, st, n2, zt, reinterpret_cast<const double2*>(w), d2(p), d2(Ap),
+                   d2(x), d2(r), b, ctl, red.part, red.maxb, cond);
     };
     if (mt == MG_F64) {
-        static const int wb1 = wave_blocks(k_update64<double, true>, 1 << 30);
-        static const int wb0 = wave_blocks(k_update64<double, false>, 1 << 30);
-        if (write_x) go(k_update64<double, true>, wb1, (double*)b0);
-        else go(k_update64<double, false>, wb0, (double*)b0);
+        static const int wb1 = wave_blocks(k_step64<double, true>, 1 << 30);
+        static const int wb0 = wave_blocks(k_step64<double, false>, 1 << 30);
+        if (write_x) go(k_step64<double, true>, wb1, (const double*)z, (double*)b0);
+        else go(k_step64<double, false>, wb0, (const double*)z, (double*)b0);
     } else {
-        static const int wb1 = wave_blocks(k_update64<float, true>, 1 << 30);
-        static const int wb0 = wave_blocks(k_update64<float, false>, 1 << 30);
-        if (write_x) go(k_update64<float, true>, wb1, (float*)b0);
-        else go(k_update64<float, false>, wb0, (float*)b0);
+        static const int wb1 = wave_blocks(k_step64<float, true>, 1 << 30);
+        static const int wb0 = wave_blocks(k_step64<float, false>, 1 << 30);
+        if (write_x) go(k_step64<float, true>, wb1, (const float*)z, (float*)b0);
+        else go(k_step64<float, false>, wb0, (const float*)z, (float*)b0);
     }
 }
 
@@ -496,49 +460,6 @@ void launch_update_x(cudaStream_t st, unsigned n, const double* p, double* x, co
     if (blocks > 0) want = std::min(want, (unsigned)blocks);
     k_update_x64<<<(int)std::min(want, (unsigned)wb), NT, 0, st>>>(n2, reinterpret_cast<const double2*>(p),
                                                                     reinterpret_cast<double2*>(x), ctl);
-}
-
-void launch_dot64(cudaStream_t st, MgType mt, bool flexible, unsigned n, const double* r, const void* z,
-                  const double* Ap, Ctl* ctl, const Red& red, Cond cond) {
-    const unsigned n2 = n / 2;
-    const auto* r2 = reinterpret_cast<const double2*>(r);
-    const auto* a2 = reinterpret_cast<const double2*>(Ap);
-    const int nb = std::min(red.maxb, std::max(1, red.maxb / 2));
-    if (mt == MG_F64) {
-        if (flexible)
-            launch_pdl(k_dot64<double, true>, nb, NT, 0, st, n2, r2, (const double*)z, a2, ctl, red.part,
-                       red.maxb, cond);
-        else
-            launch_pdl(k_dot64<double, false>, nb, NT, 0, st, n2, r2, (const double*)z, a2, ctl, red.part,
-                       red.maxb, cond);
-    } else {
-        // the flexible FP32-V-cycle dot keeps four pairs in flight a thread
-        // on one wave of blocks (100 registers): 36.7 us against 38.7 us
-        // with two on 608 blocks and 37.0 us with three, at 800 x 800
-        static const int wb4 = wave_blocks(k_dot64<float, true, 4>, 1 << 30);
-        if (flexible)
-            launch_pdl(k_dot64<float, true, 4>, std::min(nb, wb4), NT, 0, st, n2, r2, (const float*)z, a2, ctl,
-                       red.part, red.maxb, cond);
-        else
-            launch_pdl(k_dot64<float, false>, nb, NT, 0, st, n2, r2, (const float*)z, a2, ctl, red.part,
-                       red.maxb, cond);
-    }
-}
-
-void launch_update_p64(cudaStream_t st, MgType mt, unsigned n, const void* z, double* p, Ctl* ctl,
-                       Cond cond) {
-    const unsigned n2 = n / 2;
-    auto* p2 = reinterpret_cast<double2*>(p);
-    const unsigned want = std::max(1u, (n2 + NT * 2 * kPU - 1) / (NT * 2 * kPU));
-    if (mt == MG_F64) {
-        static const int wb = wave_blocks(k_update_p64<double>, 1 << 30);
-        launch_pdl(k_update_p64<double>, (int)std::min(want, (unsigned)wb), NT, 0, st, n2, (const double*)z, p2,
-                   ctl, cond);
-    } else {
-        static const int wb = wave_blocks(k_update_p64<float>, 1 << 30);
-        launch_pdl(k_update_p64<float>, (int)std::min(want, (unsigned)wb), NT, 0, st, n2, (const float*)z, p2,
-                   ctl, cond);
-    }
 }
 
 cudaError_t measure_dfma_rate(double* per_s) {

@@ -452,33 +452,18 @@ void launch_apply(cudaStream_t st, const OpView& o, const double* diag, const do
     launch_apply64(st, o, diag, p, Ap, ctl, red, cond);
 }
 
-void launch_update(cudaStream_t st, MgType mt, unsigned n, const double* p, const double* Ap,
-                   double* x, double* r, void* b0, Ctl* ctl, const Red& red, Cond cond, bool write_x) {
-    if (mt != MG_NONE) {
-        launch_update64(st, mt, n, p, Ap, x, r, b0, ctl, red, cond, write_x);
-        return;
-    }
+void launch_update(cudaStream_t st, unsigned n, const double* p, const double* Ap, double* x, double* r, Ctl* ctl,
+                   const Red& red, Cond cond) {
     static const int wb = wave_blocks(k_update, 1 << 30);
     k_update<<<std::min(red.blocks, wb), NT, 0, st>>>(n / 2, p, Ap, x, r, ctl, red.part, red.maxb, cond);
 }
 
-void launch_dot(cudaStream_t st, MgType mt, bool flexible, unsigned n, const double* r,
-                const void* z, const double* invd, const double* Ap, Ctl* ctl, const Red& red,
-                Cond cond) {
-    if (mt != MG_NONE) {
-        launch_dot64(st, mt, flexible, n, r, z, Ap, ctl, red, cond);
-        return;
-    }
+void launch_dot(cudaStream_t st, unsigned n, const double* r, const double* invd, Ctl* ctl, const Red& red, Cond cond) {
     static const int wb = wave_blocks(k_dot, 1 << 30);
     k_dot<<<std::min(red.blocks, wb), NT, 0, st>>>(n / 2, r, invd, ctl, red.part, red.maxb, cond);
 }
 
-void launch_update_p(cudaStream_t st, MgType mt, unsigned n, const void* z, const double* r,
-                     const double* invd, double* p, Ctl* ctl, Cond cond) {
-    if (mt != MG_NONE) {
-        launch_update_p64(st, mt, n, z, p, ctl, cond);
-        return;
-    }
+void launch_update_p(cudaStream_t st, unsigned n, const double* r, const double* invd, double* p, Ctl* ctl, Cond cond) {
     static const int wb = wave_blocks(k_update_p, 1 << 30);
     k_update_p<<<std::min(grid_for(n / 2), (unsigned)wb), NT, 0, st>>>(n / 2, r, invd, p, ctl, cond);
 }

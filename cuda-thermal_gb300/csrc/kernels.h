@@ -90,42 +90,34 @@ inline void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sme
 void launch_residual(cudaStream_t st, MgType mt, const OpView& o, const double* diag,
                      const double* b, const double* x, double* r, void* b0, Ctl* ctl,
                      const Red& red, Cond cond);
-// Ap = (A + C/dt) p; p.Ap; alpha = rz / p.Ap.
+// The Jacobi form's iteration: Ap = (A + C/dt) p, p.Ap, alpha = rz / p.Ap;
+// x += alpha p, r -= alpha Ap, rr, convergence test; rz = r.(r * invd), beta;
+// p = r * invd + beta p (p = r * invd on the first iteration).
 void launch_apply(cudaStream_t st, const OpView& o, const double* diag, const double* p,
                   double* Ap, Ctl* ctl, const Red& red, Cond cond);
-// x += alpha p, r -= alpha Ap, b0 = r; rr; convergence test (write_x =
-// false, FP64 outer loop only: x left to launch_update_x).
-void launch_update(cudaStream_t st, MgType mt, unsigned n, const double* p, const double* Ap,
-                   double* x, double* r, void* b0, Ctl* ctl, const Red& red, Cond cond, bool write_x = true);
-// rz = r.z (and z.Ap for the flexible beta); beta. z = V-cycle result
-// (mt = MG_F32 / MG_F64) or r * invd (mt = MG_NONE, Jacobi).
-void launch_dot(cudaStream_t st, MgType mt, bool flexible, unsigned n, const double* r,
-                const void* z, const double* invd, const double* Ap, Ctl* ctl, const Red& red,
-                Cond cond);
-// p = z + beta p (p = z on the first iteration).
-void launch_update_p(cudaStream_t st, MgType mt, unsigned n, const void* z, const double* r,
-                     const double* invd, double* p, Ctl* ctl, Cond cond);
+void launch_update(cudaStream_t st, unsigned n, const double* p, const double* Ap, double* x, double* r, Ctl* ctl,
+                   const Red& red, Cond cond);
+void launch_dot(cudaStream_t st, unsigned n, const double* r, const double* invd, Ctl* ctl, const Red& red, Cond cond);
+void launch_update_p(cudaStream_t st, unsigned n, const double* r, const double* invd, double* p, Ctl* ctl, Cond cond);
 
 // ---- FP64 outer PCG of the multigrid modes, k_fp64.cu --------------------------
-// The same operations for mt = MG_F32 / MG_F64 with the fewest FP64
-// instructions (integer float <-> double conversions); the launchers above
-// hand the multigrid modes to these.
+// The iteration for mt = MG_F32 / MG_F64, with the fewest FP64 instructions.
 void launch_residual64(cudaStream_t st, MgType mt, const OpView& o, unsigned n, const double* diag,
                        const double* b, const double* x, double* r, void* b0, Ctl* ctl, const Red& red,
                        Cond cond);
 void launch_apply64(cudaStream_t st, const OpView& o, const double* diag, const double* p,
-                    double* Ap, Ctl* ctl, const Red& red, Cond cond);
-// write_x = false: r only; alpha left in ctl->alpha_x for launch_update_x.
-void launch_update64(cudaStream_t st, MgType mt, unsigned n, const double* p, const double* Ap, double* x,
-                     double* r, void* b0, Ctl* ctl, const Red& red, Cond cond, bool write_x = true);
+                    double* Ap, Ctl* ctl, const Red& red, Cond cond);  // the Jacobi form's
+// w = (A + C/dt) z, r.z, z.Ap, z.w; beta, p.Ap, alpha (k_az64).
+void launch_az64(cudaStream_t st, MgType mt, bool flexible, const OpView& o, const double* diag, const void* z,
+                 const double* r, const double* Ap, double* w, Ctl* ctl, const Red& red, Cond cond);
+// p = z + beta p, Ap = w + beta Ap, r -= alpha Ap, b0 = r; rr; convergence test.
+// write_x = false: x left to launch_update_x, alpha in ctl->alpha_x for it.
+void launch_step64(cudaStream_t st, MgType mt, unsigned n, const void* z, const double* w, double* p, double* Ap,
+                   double* x, double* r, void* b0, Ctl* ctl, const Red& red, Cond cond, bool write_x = true);
 // x += ctl->alpha_x p where an update is pending (a plain launch: it runs
 // beside other work and is ordered by events, not by programmatic launch), on
 // at most `blocks` blocks (0: as many as the vector wants, up to one wave).
 void launch_update_x(cudaStream_t st, unsigned n, const double* p, double* x, const Ctl* ctl, int blocks);
-void launch_dot64(cudaStream_t st, MgType mt, bool flexible, unsigned n, const double* r, const void* z,
-                  const double* Ap, Ctl* ctl, const Red& red, Cond cond);
-void launch_update_p64(cudaStream_t st, MgType mt, unsigned n, const void* z, double* p, Ctl* ctl,
-                       Cond cond);
 // The GPU's DFMA issue rate (instructions per second, independent chains on
 // every SM; synchronises the device): the FP64-pipe roofline's denominator.
 cudaError_t measure_dfma_rate(double* per_s);

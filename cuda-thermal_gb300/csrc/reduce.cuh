@@ -76,6 +76,71 @@ __device__ __forceinline__ void gather2(const double* part, int maxb, unsigned* 
     }
 }
 
+// The same for N sums at once with fewer FP64 instructions: the threads' values
+// go through shared memory, and warp v adds value v of all threads (eight a
+// lane, then the shuffles), 12 warp-wide additions a value instead of the 45 of
+// eight shuffle trees: an FP64 instruction holds the pipe for 18 cycles a warp,
+// so the trees of three values kept a block's tail about a microsecond. Warp v's
+// lane 0 gets value v; call by every thread of a block of NT threads.
+template <int N>
+__device__ __forceinline__ double block_sums(const double (&v)[N]) {
+    constexpr int NW = NT / 32;
+    static_assert(N <= NW, "a warp a value");
+    __shared__ double s[N][NT];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < N; ++q) s[q][threadIdx.x] = v[q];
+    __syncthreads();
+    double a = 0.0;
+    if (w < N) {
+        a = s[w][lane];
+#pragma unroll
+        for (int k = 1; k < NW; ++k) a += s[w][lane + 32 * k];
+        a = warp_sum(a);
+    }
+    return a;
+}
+// Publishes the block's N sums as slots `slot`, `stride` + slot, ... of part and
+// takes a ticket; true in every thread of the last of `count` blocks.
+template <int N>
+__device__ __forceinline__ bool publish_sums(const double (&v)[N], double* part, int stride, unsigned slot,
+                                             unsigned* ticket, unsigned count) {
+    __shared__ int last;
+    const double a = block_sums<N>(v);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (w < N && lane == 0) {
+        part[(size_t)w * stride + slot] = a;
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == count - 1u ? 1 : 0;
+    __syncthreads();
+    return last != 0;
+}
+// In the last block: the totals of slots first .. first + count - 1, in thread 0.
+// Resets the ticket.
+template <int N>
+__device__ __forceinline__ void gather_sums(const double* part, int stride, unsigned first, unsigned count,
+                                            unsigned* ticket, double (&total)[N]) {
+    __shared__ double t[N];
+    __threadfence();
+    double v[N];
+#pragma unroll
+    for (int q = 0; q < N; ++q) v[q] = 0.0;
+    for (unsigned k = threadIdx.x; k < count; k += NT)
+#pragma unroll
+        for (int q = 0; q < N; ++q) v[q] += __ldcg(part + (size_t)q * stride + first + k);
+    const double a = block_sums<N>(v);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (w < N && lane == 0) t[w] = a;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < N; ++q) total[q] = t[q];
+        *ticket = 0u;
+    }
+}
+
 // Stops the solve: marks it done and, inside a graph loop, ends the loop
 // after the current body. Called by one thread.
 __device__ __forceinline__ void stop_loop(Ctl* c, const Cond& cond) {

@@ -9,7 +9,7 @@
 // and launches ONE CUDA graph: the start residual, then a conditional WHILE
 // node whose body is one PCG iteration rotated so that it ends with the
 // convergence test,
-//     V-cycle(r) -> z;  beta;  p = z + beta p;  Ap, alpha;  x, r update, test
+//     V-cycle(r) -> z;  A z, beta, alpha;  p, Ap, r (and x) update, test
 // The kernel that finishes the test clears the loop condition, and once the
 // solve is done every later kernel of the body returns at entry. alpha, beta
 // and the dot products never leave the device; the host reads the control
@@ -128,6 +128,7 @@ ct_status Solver::create(const ct_model* m_in, ct_precond pc_, ct_precision prec
     const size_t o_gE = ar.take(n * 4), o_gN = ar.take(n * 4), o_gU = ar.take(n * 4);
     const size_t o_cap = ar.take(n * 4), o_gB = ar.take((size_t)g0.plane * 4);
     size_t o_vec[9];
+    const size_t o_w = mt != MG_NONE && !dw ? ar.take((size_t)n * 8) : 0;
     for (size_t& o : o_vec) o = ar.take((size_t)n * 8);
     const size_t o_invd = pc == CT_JACOBI ? ar.take((size_t)n * 8) : 0;
     const size_t o_dgw = dw ? ar.take((size_t)n * 8) : 0;
@@ -225,6 +226,7 @@ ct_status Solver::create(const ct_model* m_in, ct_precond pc_, ct_precision prec
     diag = at<double>(o_vec[6]);
     xold = at<double>(o_vec[7]);
     dface = at<double>(o_vec[8]);
+    w = o_w ? at<double>(o_w) : nullptr;
     invd = pc == CT_JACOBI ? at<double>(o_invd) : nullptr;
     dgw = dw ? at<float2>(o_dgw) : nullptr;
     xwc = dw ? at<float2>(o_xwc) : nullptr;
@@ -520,16 +522,21 @@ void Solver::enqueue_body(Cond cond) {
         z = base + lv[0].o_x;
     }
     if (lag_now && !forked) fork_x();
-    const double zb = mt == MG_NONE ? 16.0 : (double)tsize;
-    enq("pcg_dot", N * (8 + zb + (flex ? 8 : 0)),
-        [&] { launch_dot(cs, mt, flex, n, r, z, invd, Ap, ctl, red_vec(SL_DOT), cond); });
-    // the p update overwrites the p that the x update reads: join first
+    if (mt == MG_NONE) {
+        enq("pcg_dot", N * (8 + 16), [&] { launch_dot(cs, n, r, invd, ctl, red_vec(SL_DOT), cond); });
+        enq("pcg_update_p", N * (16 + 16), [&] { launch_update_p(cs, n, r, invd, p, ctl, cond); });
+        enq("pcg_apply", N * 36, [&] { launch_apply(cs, op(), diag, p, Ap, ctl, red_cols(SL_APPLY), cond); });
+        enq("pcg_update_xr", N * 48, [&] { launch_update(cs, n, p, Ap, x, r, ctl, red_vec(SL_UPDATE), cond); });
+        return;
+    }
+    const double zb = (double)tsize;
+    enq("pcg_apply", N * (zb + 12 + 8 + 16 + 8),
+        [&] { launch_az64(cs, mt, flex, op(), diag, z, r, Ap, w, ctl, red_cols(SL_APPLY), cond); });
+    // the step overwrites the p that the x update reads: join first
     if (lag_now && !prof) cudaStreamWaitEvent(cs, ev_join, 0);
-    enq("pcg_update_p", N * (zb + 16), [&] { launch_update_p(cs, mt, n, z, r, invd, p, ctl, cond); });
-    enq("pcg_apply", N * 36, [&] { launch_apply(cs, op(), diag, p, Ap, ctl, red_cols(SL_APPLY), cond); });
-    void* b0 = mt == MG_NONE ? nullptr : (void*)(base + lv[0].o_b);
-    enq("pcg_update_xr", N * ((lag_now ? 24 : 48) + (mt == MG_NONE ? 0 : tsize)),
-        [&] { launch_update(cs, mt, n, p, Ap, x, r, b0, ctl, red_vec(SL_UPDATE), cond, !lag_now); });
+    enq("pcg_update_xr", N * (zb + 8 + 3 * 16 + zb + (lag_now ? 0 : 16)), [&] {
+        launch_step64(cs, mt, n, z, w, p, Ap, x, r, base + lv[0].o_b, ctl, red_vec(SL_UPDATE), cond, !lag_now);
+    });
     lag_now = false;
 }
 
