@@ -408,19 +408,20 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
             const int nr = rows_of(k);
             int xc = N.x, xcp = (N.rows + 2) * 2 * N.hx;
             if (k == nd - 1) {
-                // the bottom's finest x goes to each CTA, the rows of its parents
+                // the bottom's finest x goes to each CTA, the rows of its parents:
+                // a warp a plane, two lanes a CTA
                 if (bottom) {
-                    const int RC = 2 * N.hx, xdpl = (P.rd + 2) * RC;
-#pragma unroll 1
-                    for (int l = warp; l < nz; l += warps)
-#pragma unroll 1
-                        for (int d = 0; d < P.dist; ++d) {
-                            const int j = d * P.rd - 1, r0 = max(j, 0), r1 = min(j + P.rd + 1, N.ny - 1);
-                            const unsigned to = remote(base, (unsigned)d) + 4u * (unsigned)(P.xd + l * xdpl + (r0 - j) * RC);
-                            const unsigned tb = remote(tma::smem_addr(baru), (unsigned)d);
+                    const int RC = 2 * N.hx, xdpl = (P.rd + 2) * RC, d = lane & 15;
+                    const int j = d * P.rd - 1, r0 = max(j, 0), n4 = (min(j + P.rd + 1, N.ny - 1) - r0 + 1) * RC / 4;
+                    if (d < P.dist) {
+                        const unsigned to = remote(base, (unsigned)d) + 4u * (unsigned)(P.xd + (r0 - j) * RC);
+                        const unsigned tb = remote(tma::smem_addr(baru), (unsigned)d);
+                        for (int l = warp; l < nz; l += warps) {
                             const float4* const from = reinterpret_cast<const float4*>(sm + N.x + l * xcp + (r0 + 1) * RC);
-                            for (int s = lane; s < (r1 - r0 + 1) * RC / 4; s += 32) send4(to + 16u * (unsigned)s, from[s], tb);
+#pragma unroll 4
+                            for (int s = lane >> 4; s < n4; s += 2) send4(to + 4u * (unsigned)(l * xdpl) + 16u * (unsigned)s, from[s], tb);
                         }
+                    }
                 }
                 if (!dist) break;
                 ok = ok && receive(baru);

@@ -251,17 +251,19 @@ ct_status Solver::create(const ct_model* m_in, ct_precond pc_, ct_precision prec
     // three operand streams faster than the tile ring (800 x 800 x 10 FLEX
     // solve 6.52 -> 6.46 ms). CT_SWEEP0_GRID=0 stages them too.
     if (const char* e = std::getenv("CT_SWEEP0_GRID")) sweep0_grid = e[0] != '0';
-    // x += alpha p leaves the update (which then moves 24 B a cell fewer on
-    // the iteration's critical path) for a launch of a few blocks beside the
-    // next V-cycle, forked after the restriction out of level 1: it streams x
-    // and p while the coarse levels, latency-bound, leave the memory system
-    // idle (800 x 800 FLEX solve 155.3 -> 157.8 solves/s at 64 blocks; 16 /
-    // 32 / 128 / 192 blocks: 145.7 / 155.4 / 157.6 / 156.8; forked after
-    // level 0's restriction: 156.3; the whole grid at once: 154.3).
+    // x += alpha p leaves the update (which then moves 16 B a cell fewer on the
+    // iteration's critical path) for a launch of its own beside the next
+    // V-cycle, forked after the last restriction: the bottom levels then hold
+    // at most kTailCtas SMs and leave the memory system idle, and their cluster
+    // is resident before the x update's blocks are (forked earlier, those
+    // held back or shared the cluster's SMs: 800 x 800 x 10 us an iteration
+    // 383.0 at 100 blocks, 386.5 at 64 and 383.1 at 136; after level 1's
+    // restriction 392-397 at 64, after level 2's 385 at 64 and 405 at 100; x in
+    // the update 402. 1024 x 1024 x 16: 889, 887, 889; 892; 886, 882; 924).
     // CT_XLAG = k forks after level k's restriction instead, -1 keeps x in
     // the update; CT_XLAG_BLOCKS sets the blocks.
     if (const char* e = std::getenv("CT_XLAG")) xlag = std::atoi(e);
-    xlag_blocks = std::max(1, sms * 64 / 152);
+    xlag_blocks = std::max(1, sms * 100 / 152);
     if (const char* e = std::getenv("CT_XLAG_BLOCKS")) xlag_blocks = std::max(1, std::atoi(e));
     // Tensor maps of the levels whose sweeps are staged by bulk tensor copies
     // (FP32 levels with at least one full tile row, above the shared-memory

@@ -92,8 +92,8 @@ class Solver {
     // x += alpha p beside the next V-cycle (FP64 outer loop, multigrid): a
     // launch of xlag_blocks blocks on st_side, forked after the restriction
     // out of level fork_level() (xlag < 0: x stays in the update)
-    int xlag = 1;
-    int xlag_blocks = 64;
+    int xlag = kMaxTail;
+    int xlag_blocks = 100;
     cudaStream_t st_side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     bool lag_now = false, forked = false;  // while a body is enqueued
