@@ -173,18 +173,42 @@ __global__ void __launch_bounds__(32 * MZ)
     __syncthreads();
     const int nz = g.nz;
     if (on && l == 0) {
-        // the recurrence of sweep_column, on shared memory
-        T prev = 0;
+        // the recurrence of sweep_column, on shared memory; FP32 up to 16 planes
+        // on registers, all MZ planes without a test (the ones past nz hold
+        // nothing and reach nothing): one warp runs it while the block waits, so
+        // its instruction count is the kernel's time. 237 x 181 x 10: an
+        // iteration of 105.2 us against 109.4 with the loop over shared memory;
+        // 501 x 333 x 10: 167.1 against 169.8
+        if constexpr (sizeof(T) == 4 && MZ <= 16) {
+            T v[MZ], c[MZ], prev = 0, lower = 0;
+#pragma unroll
+            for (int k = 0; k < MZ; ++k) {
+                prev = (sv[k][tx] - lower * prev) * sfi[k][tx];
+                v[k] = prev;
+                c[k] = sfc[k][tx];
+                lower = -sgu[k][tx];
+            }
+#pragma unroll
+            for (int k = MZ - 2; k >= 0; --k) {
+                const T n = v[k] - c[k] * v[k + 1];
+                v[k] = k < nz - 1 ? n : v[k];
+            }
+#pragma unroll
+            for (int k = 0; k < MZ; ++k)
+                if (k < nz) sv[k][tx] = v[k];
+        } else {
+            T prev = 0;
 #pragma unroll 4
-        for (int k = 0; k < nz; ++k) {
-            const T lower = k > 0 ? -face<T>(sgu[k - 1][tx]) : T(0);
-            prev = (sv[k][tx] - lower * prev) * sfi[k][tx];
-            sv[k][tx] = prev;
-        }
+            for (int k = 0; k < nz; ++k) {
+                const T lower = k > 0 ? -face<T>(sgu[k - 1][tx]) : T(0);
+                prev = (sv[k][tx] - lower * prev) * sfi[k][tx];
+                sv[k][tx] = prev;
+            }
 #pragma unroll 4
-        for (int k = nz - 2; k >= 0; --k) {
-            prev = sv[k][tx] - sfc[k][tx] * prev;
-            sv[k][tx] = prev;
+            for (int k = nz - 2; k >= 0; --k) {
+                prev = sv[k][tx] - sfc[k][tx] * prev;
+                sv[k][tx] = prev;
+            }
         }
     }
     __syncthreads();
@@ -361,6 +385,8 @@ void launch_sweep(cudaStream_t st, const LevelView<T>& L, int color, bool zero_x
     } while (0)
         if (nz <= 8)
             CT_SPLIT(8);
+        else if (nz <= 12)
+            CT_SPLIT(12);
         else if (nz <= 16)
             CT_SPLIT(16);
         else
