@@ -121,7 +121,7 @@ class Batch {
         cudaGraphExec_t gx = nullptr;
         BCtl* bc = nullptr;
         Plan vec{}, cols{}, rows{};  // value pairs, fine columns, fine rows
-        BRed r_res{}, r_apply{}, r_update{}, r_dot{};
+        BRed r_res{}, r_apply{}, r_update{};
         std::vector<Plan> sweep, restr;
         std::vector<unsigned> sweep_tile, restr_tile;
         // per depth: 0 grid sweeps, 1 sweeps staged by bulk tensor copies,
@@ -318,6 +318,7 @@ ct_status Batch::create(int n, const ct_model* const* models, const DeviceBuild*
         I.r = s.rw();
         I.p = s.pw();
         I.Ap = s.Apw();
+        I.w = s.ww();
         I.dgw = s.dgw;
         I.b0 = s.at<float>(s.lv[0].o_b);
         I.z = s.at<float>(s.lv[0].o_x);
@@ -454,7 +455,6 @@ ct_status Batch::build_bucket(Bucket& b) {
     if ((s = make_red(dw ? b.cols : b.rows, &b.r_res)) != CT_OK) return s;
     if ((s = make_red(b.rows, &b.r_apply)) != CT_OK) return s;
     if ((s = make_red(b.vec, &b.r_update)) != CT_OK) return s;
-    if ((s = make_red(b.vec, &b.r_dot)) != CT_OK) return s;
     if ((s = upload(&b.small_insts, b.inst)) != CT_OK) return s;
     b.sweep.assign((size_t)b.depth, Plan{});
     b.sweep_grid.assign((size_t)b.depth, Plan{});
@@ -720,11 +720,8 @@ void Batch::enqueue_body(Bucket& b, cudaStream_t s, Cond cond) {
         enq(s, "b_update_xr", N * 80, [&] { launch_b_step64(s, b.vec, bi, ctl, b.r_update, b.bc, cond); });
         return;
     }
-    enq(s, "b_dot", N * 20, [&] { launch_b_dot(s, b.vec, bi, ctl, b.r_dot, b.bc, cond); });
-    enq(s, "b_update_p", N * 20, [&] { launch_b_update_p(s, b.vec, bi, ctl); });
-    enq(s, "b_apply", N * 36, [&] { launch_b_apply(s, b.rows, bi, ctl, b.r_apply, b.bc, cond); });
-    enq(s, "b_update_xr", N * 52,
-        [&] { launch_b_update(s, b.vec, bi, ctl, b.r_update, b.bc, cond); });
+    enq(s, "b_apply", N * 48, [&] { launch_b_az_dw(s, b.rows, bi, ctl, b.r_apply, b.bc, cond); });
+    enq(s, "b_update_xr", N * 80, [&] { launch_b_step_dw(s, b.vec, bi, ctl, b.r_update, b.bc, cond); });
     // residual replacement of the instances whose first phase just ended
     // (blocks of the other instances return at entry)
     enq(s, "b_fold_pe", 0, [&] { launch_b_fold(s, b.vec, bi, ctl, 1); });

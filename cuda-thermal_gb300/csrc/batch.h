@@ -31,9 +31,9 @@ struct Plan {
 };
 
 // One instance's fine-level arrays (split layout). The double-word mode
-// (CT_MG_FP32_FLEX_DW) reads r, p, Ap as float pairs and keeps x as an FP64
+// (CT_MG_FP32_FLEX_DW) reads r, p, Ap, w as float pairs and keeps x as an FP64
 // base plus xw; the FP64 mode (CT_MG_FP32_FLEX) reads the same storage as
-// doubles (r64, p64, Ap64) and x is the whole iterate (xw, dgw null).
+// doubles (r64, p64, Ap64, w64) and x is the whole iterate (xw, dgw null).
 struct BInst {
     OpView o;
     const double* P;
@@ -45,14 +45,15 @@ struct BInst {
     float2* r;
     float2* p;
     float2* Ap;
+    float2* w;      // A z
     const float2* dgw;
     float* b0;      // V-cycle input (level 0 b)
     const float* z; // V-cycle result (level 0 x)
     double* xold;   // x at the last set_rhs_transient (step bookkeeping)
-    double* r64;    // r, p, Ap as doubles (the FP64 outer mode)
+    double* r64;    // r, p, Ap, A z as doubles (the FP64 outer mode)
     double* p64;
     double* Ap64;
-    double* w64;    // A z
+    double* w64;
     unsigned n;     // slots of all planes
 };
 
@@ -75,13 +76,8 @@ void launch_b_guard(cudaStream_t st, BCtl* bc, Cond cond);
 void launch_b_fold(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, int only_phase_end);
 void launch_b_residual(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red,
                        int start, BCtl* bc, Cond cond);
-void launch_b_apply(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red,
-                    BCtl* bc, Cond cond);
-void launch_b_update(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red,
-                     BCtl* bc, Cond cond);
-void launch_b_dot(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc,
-                  Cond cond);
-void launch_b_update_p(cudaStream_t st, const Plan& p, const BInst* bi, const Ctl* ctl);
+void launch_b_az_dw(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond);
+void launch_b_step_dw(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond);
 
 // ---- outer PCG in FP64 (CT_MG_FP32_FLEX), one launch for the batch, k_batch64.cu
 // Items: residual and A z, rows of one colour and plane; the step, value pairs.

@@ -64,6 +64,7 @@ struct Ctl {
     double aux0, aux1, aux2;  // results of the auxiliary reductions
     double stop;              // relres at which the current loop ends (double-word mode: phase 1)
     float2 alpha_w, beta_w;   // alpha, beta as float pairs (double-word mode)
+    float2 alpha_xw;          // as alpha_x, in the double-word mode
     int iter;                 // completed iterations
     int body;                 // loop bodies entered (bounds the graph loop)
     // done and phase_end sit side by side on an 8-byte boundary: every kernel

@@ -23,18 +23,6 @@ using namespace mgdev;
 
 namespace {
 
-// The same for double-word accumulators (float pairs in the same slots),
-// summed on the FP32 pipe.
-__device__ __forceinline__ bool publish_inst_acc(const DwAcc& a, const DwAcc& b, const BRed& red, int ntasks,
-                                                 int inst, int count) {
-    return publish_acc2(a, b, red.part, ntasks, blockIdx.x, &red.tickets[inst], (unsigned)count);
-}
-
-__device__ __forceinline__ void gather_inst_acc(const BRed& red, int ntasks, int inst, int first, int count,
-                                                double& A, double& B) {
-    gather_acc2(red.part, ntasks, (unsigned)first, (unsigned)count, &red.tickets[inst], A, B);
-}
-
 // Start of every loop body: ends the loop once no instance is active, and
 // bounds the number of bodies.
 __global__ void kb_guard(BCtl* bc, Cond cond) {
@@ -160,70 +148,99 @@ __global__ void __launch_bounds__(NT)
     }
 }
 
-// Ap = d p - sum G p_nbr over rows [begin, end) of the instance (one warp
-// per row of one colour of one plane, apply_row with one cell per lane, every
-// operand of it gathered at once), p.Ap, alpha. Measured on the 256-instance
-// floorplan batch: 40.7 ms per solve against 50.0 ms with the operands loaded
-// term by term and 59.0 ms with two cells per lane; compiled for 4 blocks per
-// SM (64 registers: 600 us per launch against 722 us with the compiler's 78).
+// w = (A + C/dt) z, r.z, z.Ap, z.w, then the instance's beta, p.Ap and alpha
+// (k_az_dw); items = rows of one colour and plane.
 __global__ void __launch_bounds__(NT, 4)
-    kb_apply(Plan p, const BInst* __restrict__ bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
+    kb_az_dw(Plan p, const BInst* __restrict__ bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
     pdl_enter();
     const Task t = p.tasks[blockIdx.x];
     Ctl* c = &ctl[t.inst];
     if (inst_done(c)) return;
-    const OpView o = bi[t.inst].o;
-    const float2* __restrict__ pv = bi[t.inst].p;
-    const float2* __restrict__ dgw = bi[t.inst].dgw;
-    float2* __restrict__ Ap = bi[t.inst].Ap;
+    const BInst& I = bi[t.inst];
+    const OpView o = I.o;
+    const float2 *const r = I.r, *const Ap = I.Ap;
+    float2* const w = I.w;
+    const bool first = c->iter == 0;  // no Ap yet
     const int lane = (int)(threadIdx.x & 31u);
-    DwAcc pacc = {0.0f, 0.0f};
+    DwAcc v[3] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
     for (unsigned R = t.begin + (threadIdx.x >> 5); R < t.end; R += NT / 32)
-        apply_row<1>(o, dgw, pv, Ap, R, lane, pacc);
+        row_z<1>(
+            o, I.dgw, I.z, R, lane,
+            [&](unsigned k) { return DotItem{r[k], first ? make_float2(0.0f, 0.0f) : Ap[k]}; },
+            [&](unsigned k, const DotItem& m, const CellZ<float, float2>& a) {
+                const float2 az = az_dw(a);
+                w[k] = az;
+                dots_dw(v, m, a.zc, az);
+            });
     pdl_trigger();
-    DwAcc unused = {0.0f, 0.0f};
-    block_sum_acc2(pacc, unused);
-    if (publish_inst_acc(pacc, unused, red, p.ntasks, t.inst, p.inst_count[t.inst])) {
-        double PAP, unused2;
-        gather_inst_acc(red, p.ntasks, t.inst, p.inst_first[t.inst], p.inst_count[t.inst], PAP, unused2);
+    const unsigned count = (unsigned)p.inst_count[t.inst];
+    if (publish_acc<3>(v, red.part, p.ntasks, blockIdx.x, &red.tickets[t.inst], count)) {
+        double s3[3];
+        gather_acc<3>(red.part, p.ntasks, (unsigned)p.inst_first[t.inst], count, &red.tickets[t.inst], s3);
         if (threadIdx.x == 0) {
-            c->pAp = PAP;
-            if (!(PAP > 0.0) || !isfinite(PAP)) {
+            Scalars s;
+            const bool ok = next_scalars(true, first, s3[0], s3[1], s3[2], c->rz, c->pAp, s);
+            c->rz = s3[0];
+            c->zAp = s3[1];
+            c->beta = s.beta;
+            c->pAp = s.pAp;
+            c->alpha = s.alpha;
+            c->beta_w = dw_of(s.beta);
+            c->alpha_w = dw_of(s.alpha);
+            if (!ok) {
                 c->breakdown = 1;
-                c->alpha = 0.0;
                 inst_stop(c, bc, cond);
-            } else {
-                c->alpha = c->rz / PAP;
-                c->alpha_w = dw_of(c->alpha);
             }
         }
     }
 }
 
-// x += alpha p, r -= alpha Ap, b0 = r, ||r||^2, the instance's convergence
-// test. Items are value pairs.
+// p = z + beta p, Ap = w + beta Ap, x += alpha p, r -= alpha Ap, b0 = r, ||r||^2,
+// the instance's convergence test (k_step_dw). Items are value pairs.
 __global__ void __launch_bounds__(NT)
-    kb_update(Plan p, const BInst* __restrict__ bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
+    kb_step_dw(Plan p, const BInst* __restrict__ bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
     pdl_enter();
     const Task t = p.tasks[blockIdx.x];
     Ctl* c = &ctl[t.inst];
     if (inst_done(c)) return;
-    DwAcc acc = {0.0f, 0.0f};
-    update_range(t.begin + threadIdx.x, t.end, NT, c->alpha_w,
-                 reinterpret_cast<const float4*>(bi[t.inst].p),
-                 reinterpret_cast<const float4*>(bi[t.inst].Ap),
-                 reinterpret_cast<float4*>(bi[t.inst].xw), reinterpret_cast<float4*>(bi[t.inst].r),
-                 reinterpret_cast<float2*>(bi[t.inst].b0), acc);
+    const BInst& I = bi[t.inst];
+    const float2 alpha = c->alpha_w, beta = c->beta_w;
+    const bool first = c->iter == 0;
+    const float2* __restrict__ z2 = reinterpret_cast<const float2*>(I.z);
+    const float4* __restrict__ w2 = reinterpret_cast<const float4*>(I.w);
+    float4* __restrict__ p2 = reinterpret_cast<float4*>(I.p);
+    float4* __restrict__ a2 = reinterpret_cast<float4*>(I.Ap);
+    float4* __restrict__ x2 = reinterpret_cast<float4*>(I.xw);
+    float4* __restrict__ r2 = reinterpret_cast<float4*>(I.r);
+    float2* __restrict__ b02 = reinterpret_cast<float2*>(I.b0);
+    DwAcc v[1] = {{0.0f, 0.0f}};
+    struct Item {
+        StepItem s;
+        float4 x;
+    };
+    stream_pipelined<1, Item>(
+        t.begin + threadIdx.x, t.end, NT,
+        [&](unsigned k) {
+            const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            return Item{StepItem{z2[k], w2[k], first ? none : p2[k], first ? none : a2[k], r2[k]}, x2[k]};
+        },
+        [&](unsigned k, Item it) {
+            step_item(it.s, alpha, beta, v[0]);
+            p2[k] = it.s.p;
+            a2[k] = it.s.a;
+            x2[k] = x_item(it.x, it.s.p, alpha);
+            r2[k] = it.s.r;
+            b02[k] = make_float2(it.s.r.x, it.s.r.z);
+        });
     pdl_trigger();
-    DwAcc unused = {0.0f, 0.0f};
-    block_sum_acc2(acc, unused);
-    if (publish_inst_acc(acc, unused, red, p.ntasks, t.inst, p.inst_count[t.inst])) {
-        double RR, U;
-        gather_inst_acc(red, p.ntasks, t.inst, p.inst_first[t.inst], p.inst_count[t.inst], RR, U);
+    const unsigned count = (unsigned)p.inst_count[t.inst];
+    if (publish_acc<1>(v, red.part, p.ntasks, blockIdx.x, &red.tickets[t.inst], count)) {
+        double rr[1];
+        gather_acc<1>(red.part, p.ntasks, (unsigned)p.inst_first[t.inst], count, &red.tickets[t.inst], rr);
         if (threadIdx.x == 0) {
-            c->rr = RR;
+            c->rr = rr[0];
             c->iter += 1;
-            const double rel = sqrt(RR / c->bb);
+            const double rel = sqrt(rr[0] / c->bb);
             c->relres = rel;
             if (rel < c->tol) {
                 c->converged = 1;
@@ -238,45 +255,6 @@ __global__ void __launch_bounds__(NT)
             }
         }
     }
-}
-
-// rz = r.z, z.Ap, flexible beta.
-__global__ void __launch_bounds__(NT)
-    kb_dot(Plan p, const BInst* __restrict__ bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
-    pdl_enter();
-    const Task t = p.tasks[blockIdx.x];
-    Ctl* c = &ctl[t.inst];
-    if (inst_done(c)) return;
-    DwAcc rz = {0.0f, 0.0f}, zap = {0.0f, 0.0f};
-    dot_range(t.begin + threadIdx.x, t.end, NT, reinterpret_cast<const float4*>(bi[t.inst].r),
-              reinterpret_cast<const float2*>(bi[t.inst].z),
-              reinterpret_cast<const float4*>(bi[t.inst].Ap), rz, zap);
-    pdl_trigger();
-    block_sum_acc2(rz, zap);
-    if (publish_inst_acc(rz, zap, red, p.ntasks, t.inst, p.inst_count[t.inst])) {
-        double RZ, ZAP;
-        gather_inst_acc(red, p.ntasks, t.inst, p.inst_first[t.inst], p.inst_count[t.inst], RZ, ZAP);
-        if (threadIdx.x == 0) {
-            c->beta = c->iter > 0 ? -ZAP / c->pAp : 0.0;
-            c->beta_w = dw_of(c->beta);
-            c->rz = RZ;
-            c->zAp = ZAP;
-            if (!isfinite(RZ) || !isfinite(c->beta)) {
-                c->breakdown = 1;
-                inst_stop(c, bc, cond);
-            }
-        }
-    }
-}
-
-__global__ void __launch_bounds__(NT)
-    kb_update_p(Plan p, const BInst* __restrict__ bi, const Ctl* ctl) {
-    pdl_enter();
-    const Task t = p.tasks[blockIdx.x];
-    const Ctl* c = &ctl[t.inst];
-    if (inst_done(c)) return;
-    update_p_range(t.begin + threadIdx.x, t.end, NT, c->beta_w, c->iter == 0,
-                   reinterpret_cast<const float2*>(bi[t.inst].z), reinterpret_cast<float4*>(bi[t.inst].p));
 }
 
 // Pairs of values: b = P + C/dt x (x = FP64 base, folded), x_old = x.
@@ -442,23 +420,12 @@ void launch_b_residual(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl
     launch_pdl(kb_residual, p.ntasks, NT, 0, st, p, bi, ctl, red, start, bc, cond);
 }
 
-void launch_b_apply(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red,
-                    BCtl* bc, Cond cond) {
-    launch_pdl(kb_apply, p.ntasks, NT, 0, st, p, bi, ctl, red, bc, cond);
+void launch_b_az_dw(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
+    launch_pdl(kb_az_dw, p.ntasks, NT, 0, st, p, bi, ctl, red, bc, cond);
 }
 
-void launch_b_update(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red,
-                     BCtl* bc, Cond cond) {
-    launch_pdl(kb_update, p.ntasks, NT, 0, st, p, bi, ctl, red, bc, cond);
-}
-
-void launch_b_dot(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc,
-                  Cond cond) {
-    launch_pdl(kb_dot, p.ntasks, NT, 0, st, p, bi, ctl, red, bc, cond);
-}
-
-void launch_b_update_p(cudaStream_t st, const Plan& p, const BInst* bi, const Ctl* ctl) {
-    launch_pdl(kb_update_p, p.ntasks, NT, 0, st, p, bi, ctl);
+void launch_b_step_dw(cudaStream_t st, const Plan& p, const BInst* bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
+    launch_pdl(kb_step_dw, p.ntasks, NT, 0, st, p, bi, ctl, red, bc, cond);
 }
 
 void launch_b_step_record(cudaStream_t st, const Plan& p, const BInst* bi, BRed red, double* mx,

@@ -110,9 +110,10 @@ __global__ void __launch_bounds__(NT, 4)
         double r, ap;
     };
     for (unsigned R = t.begin + (threadIdx.x >> 5); R < t.end; R += NT / 32)
-        row_z<1, float>(
+        row_z<1>(
             o, I.diag, I.z, R, lane, [&](unsigned k) { return More{r[k], first ? 0.0 : Ap[k]}; },
-            [&](unsigned k, const More& m, double az, double zc) {
+            [&](unsigned k, const More& m, const CellZ<float, double>& a) {
+                const double az = az64(a), zc = to_d(a.zc);
                 w[k] = az;
                 v[0] = __fma_rn(m.r, zc, v[0]);
                 v[1] = __fma_rn(zc, m.ap, v[1]);

@@ -38,17 +38,6 @@ using namespace dwdev;
 
 namespace {
 
-// Block b of the grid streams the contiguous items [begin, end) with stride
-// NT (as a batched task does) rather than striding over the whole vector.
-struct BlockRange {
-    unsigned begin, end;
-};
-__device__ __forceinline__ BlockRange block_range(unsigned n) {
-    const unsigned per = ((n + gridDim.x - 1) / gridDim.x + NT * kU - 1) / (NT * kU) * (NT * kU);
-    const unsigned b = blockIdx.x * per;
-    return BlockRange{b + threadIdx.x, b + per < n ? b + per : n};
-}
-
 // ---- FP64 residual from a double-word x: start and replacement -------------
 
 // r = b - (A + C/dt) x in FP64 with x = hi + lo, the stored FP64 diagonal;
@@ -61,6 +50,8 @@ __global__ void __launch_bounds__(NT)
                  const double* __restrict__ x, float2* __restrict__ r, float* __restrict__ b0,
                  int start, Ctl* ctl, double* part, int maxb, Cond cond) {
     pdl_enter();
+    // the pending x update went into the base before this residual
+    if (!start && blockIdx.x == 0 && threadIdx.x == 0) ctl->alpha_xw = make_float2(0.0f, 0.0f);
     if (!start && *(volatile const int*)&ctl->done) {  // converged or stopped in phase 1
         if (cond.use && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond.h, 0u);
         return;
@@ -151,62 +142,97 @@ __global__ void __launch_bounds__(NT)
 
 // ---- the iteration ------------------------------------------------------------
 
-// Ap = d p - sum G p_nbr (op_apply, src/operator3d.h:108-112), p.Ap and
-// alpha: one warp per row of one colour of one plane (no integer division per
-// cell), two cells per lane, products summed with DwAcc.
-__global__ void __launch_bounds__(NT)
-    k_apply_dw_rows(OpView o, const float2* __restrict__ dgw, const float2* __restrict__ p,
-                    float2* __restrict__ Ap, Ctl* ctl, double* part, int maxb, Cond cond) {
+constexpr int kRowZ = 1;   // cells a lane and step of k_az_dw
+constexpr int kStepU = 2;  // pairs a thread and step of k_step_dw
+
+// w = (A + C/dt) z, r.z, z.Ap and z.w in one pass (one warp per row of one colour
+// of one plane), then beta, p.Ap and alpha (next_scalars): the step below makes
+// A p from w, so neither a dot pass nor an apply on p follows.
+// 640 x 640 x 10: 48.8 us (4.0 TB/s), and the step 43.8 us (6.0 TB/s), where the
+// dots, the p update, the apply on p and the update of x and r took 22.5 + 14.1 +
+// 47.1 + 36.1 us; the x update (16.1 us alone) hides beside the V-cycle's bottom.
+// A solve: 3.81 ms against 4.04.
+__global__ void __launch_bounds__(NT, 4)
+    k_az_dw(OpView o, const float2* __restrict__ dgw, const float* __restrict__ z, const float2* __restrict__ r,
+            const float2* __restrict__ Ap, float2* __restrict__ w, Ctl* ctl, double* part, int maxb, Cond cond) {
     pdl_enter();
     if (loop_done(ctl, cond)) return;
     const Geo& g = o.g;
+    const bool first = ctl->iter == 0;  // no Ap yet
     const unsigned rows = 2u * (unsigned)g.ny * (unsigned)g.nz;
     const int lane = (int)(threadIdx.x & 31u);
-    DwAcc acc = {0.0f, 0.0f};
+    DwAcc v[3] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
     for (unsigned R = blockIdx.x * (NT / 32) + (threadIdx.x >> 5); R < rows; R += gridDim.x * (NT / 32))
-        apply_row<2>(o, dgw, p, Ap, R, lane, acc);
-    DwAcc unused = {0.0f, 0.0f};
+        row_z<kRowZ>(
+            o, dgw, z, R, lane,
+            [&](unsigned k) { return DotItem{r[k], first ? make_float2(0.0f, 0.0f) : Ap[k]}; },
+            [&](unsigned k, const DotItem& m, const CellZ<float, float2>& a) {
+                const float2 az = az_dw(a);
+                w[k] = az;
+                dots_dw(v, m, a.zc, az);
+            });
     pdl_trigger();
-    block_sum_acc2(acc, unused);
-    if (publish_acc2(acc, unused, part, maxb, blockIdx.x, &ctl->ticket[SL_APPLY], gridDim.x)) {
-        double PAP, U;
-        gather_acc2(part, maxb, 0u, gridDim.x, &ctl->ticket[SL_APPLY], PAP, U);
+    if (publish_acc<3>(v, part, maxb, blockIdx.x, &ctl->ticket[SL_APPLY], gridDim.x)) {
+        double t[3];
+        gather_acc<3>(part, maxb, 0u, gridDim.x, &ctl->ticket[SL_APPLY], t);
         if (threadIdx.x == 0) {
-            ctl->pAp = PAP;
-            if (!(PAP > 0.0) || !isfinite(PAP)) {
+            Scalars s;
+            const bool ok = next_scalars(true, first, t[0], t[1], t[2], ctl->rz, ctl->pAp, s);
+            ctl->rz = t[0];
+            ctl->zAp = t[1];
+            ctl->beta = s.beta;
+            ctl->pAp = s.pAp;
+            ctl->alpha = s.alpha;
+            ctl->beta_w = dw_of(s.beta);
+            ctl->alpha_w = dw_of(s.alpha);
+            if (!ok) {
                 ctl->breakdown = 1;
-                ctl->alpha = 0.0;
                 stop_loop(ctl, cond);
-            } else {
-                ctl->alpha = ctl->rz / PAP;
-                ctl->alpha_w = dw_of(ctl->alpha);
             }
         }
     }
 }
 
-
-// x += alpha p, r -= alpha Ap, b0 = r (hi word), ||r||^2, convergence test.
-// Two values per thread and step (float4 = two double words).
+// p = z + beta p, Ap = w + beta Ap, r -= alpha Ap, b0 = r (hi word), ||r||^2,
+// convergence test. Two values a thread and step (float4 = two double words),
+// each block a contiguous range. WX = false: x is left to k_update_x_dw beside
+// the next V-cycle, alpha in ctl->alpha_xw for it (k_step64 likewise).
+template <bool WX>
 __global__ void __launch_bounds__(NT)
-    k_update_dw(unsigned n2, const float4* __restrict__ p, const float4* __restrict__ Ap,
-                float4* __restrict__ x, float4* __restrict__ r, float2* __restrict__ b0, Ctl* ctl,
-                double* part, int maxb, Cond cond) {
+    k_step_dw(unsigned n2, const float2* __restrict__ z, const float4* __restrict__ w, float4* __restrict__ p,
+              float4* __restrict__ Ap, float4* __restrict__ x, float4* __restrict__ r, float2* __restrict__ b0,
+              Ctl* ctl, double* part, int maxb, Cond cond) {
     pdl_enter();
-    if (loop_done(ctl, cond)) return;
-    DwAcc acc = {0.0f, 0.0f};
-    const BlockRange br = block_range(n2);
-    update_range(br.begin, br.end, NT, ctl->alpha_w, p, Ap, x, r, b0, acc);
-    DwAcc unused = {0.0f, 0.0f};
+    const bool done = loop_done(ctl, cond);
+    const float2 alpha = ctl->alpha_w, beta = ctl->beta_w;
+    if (!WX && blockIdx.x == 0 && threadIdx.x == 0) ctl->alpha_xw = done ? make_float2(0.0f, 0.0f) : alpha;
+    if (done) return;
+    const bool first = ctl->iter == 0;
+    DwAcc v[1] = {{0.0f, 0.0f}};
+    const unsigned per = ((n2 + gridDim.x - 1) / gridDim.x + NT * kStepU - 1) / (NT * kStepU) * (NT * kStepU);
+    const unsigned begin = blockIdx.x * per, end = begin + per < n2 ? begin + per : n2;
+    stream_pipelined<kStepU, StepItem>(
+        begin + threadIdx.x, end, NT,
+        [&](unsigned k) {
+            const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            return StepItem{z[k], w[k], first ? none : p[k], first ? none : Ap[k], r[k]};
+        },
+        [&](unsigned k, StepItem it) {
+            step_item(it, alpha, beta, v[0]);
+            p[k] = it.p;
+            Ap[k] = it.a;
+            r[k] = it.r;
+            b0[k] = make_float2(it.r.x, it.r.z);
+            if (WX) x[k] = x_item(x[k], it.p, alpha);
+        });
     pdl_trigger();
-    block_sum_acc2(acc, unused);
-    if (publish_acc2(acc, unused, part, maxb, blockIdx.x, &ctl->ticket[SL_UPDATE], gridDim.x)) {
-        double RR, U;
-        gather_acc2(part, maxb, 0u, gridDim.x, &ctl->ticket[SL_UPDATE], RR, U);
+    if (publish_acc<1>(v, part, maxb, blockIdx.x, &ctl->ticket[SL_UPDATE], gridDim.x)) {
+        double t[1];
+        gather_acc<1>(part, maxb, 0u, gridDim.x, &ctl->ticket[SL_UPDATE], t);
         if (threadIdx.x == 0) {
-            ctl->rr = RR;
+            ctl->rr = t[0];
             ctl->iter += 1;
-            const double rel = sqrt(RR / ctl->bb);
+            const double rel = sqrt(t[0] / ctl->bb);
             ctl->relres = rel;
             if (rel < ctl->tol) {
                 ctl->converged = 1;
@@ -225,43 +251,19 @@ __global__ void __launch_bounds__(NT)
     }
 }
 
-// rz = r.z and z.Ap (flexible beta); beta. Items strided over the whole grid
-// on 4 blocks per SM, compiled for 4 blocks per SM: 31.7 us at 800 x 800 x 10
-// against 32.9 us with the compiler's own register choice and 34.5 us with
-// one contiguous range per block on 6 blocks per SM.
-__global__ void __launch_bounds__(NT, 4)
-    k_dot_dw(unsigned n2, const float4* __restrict__ r, const float2* __restrict__ z,
-             const float4* __restrict__ Ap, Ctl* ctl, double* part, int maxb, Cond cond) {
-    pdl_enter();
-    if (loop_done(ctl, cond)) return;
-    DwAcc rz = {0.0f, 0.0f}, zap = {0.0f, 0.0f};
-    dot_range(blockIdx.x * NT + threadIdx.x, n2, gridDim.x * NT, r, z, Ap, rz, zap);
-    pdl_trigger();
-    block_sum_acc2(rz, zap);
-    if (publish_acc2(rz, zap, part, maxb, blockIdx.x, &ctl->ticket[SL_DOT], gridDim.x)) {
-        double RZ, ZAP;
-        gather_acc2(part, maxb, 0u, gridDim.x, &ctl->ticket[SL_DOT], RZ, ZAP);
-        if (threadIdx.x == 0) {
-            ctl->beta = ctl->iter > 0 ? -ZAP / ctl->pAp : 0.0;
-            ctl->beta_w = dw_of(ctl->beta);
-            ctl->rz = RZ;
-            ctl->zAp = ZAP;
-            if (!isfinite(RZ) || !isfinite(ctl->beta)) {
-                ctl->breakdown = 1;
-                stop_loop(ctl, cond);
-            }
-        }
-    }
-}
-
-// p = z + beta p (p = z on the first iteration).
+// x += alpha p with the alpha k_step_dw<false> left in ctl->alpha_xw (zero:
+// nothing pending), the same rounding as the fused update; ordered as
+// k_update_x64 is.
+struct XItemDw {
+    float4 p, x;
+};
 __global__ void __launch_bounds__(NT)
-    k_update_p_dw(unsigned n2, const float2* __restrict__ z, float4* __restrict__ p, const Ctl* ctl,
-                  Cond cond) {
-    pdl_enter();
-    if (loop_done(ctl, cond)) return;
-    const BlockRange br = block_range(n2);
-    update_p_range(br.begin, br.end, NT, ctl->beta_w, ctl->iter == 0, z, p);
+    k_update_x_dw(unsigned n2, const float4* __restrict__ p, float4* __restrict__ x, const Ctl* ctl) {
+    const float2 alpha = ctl->alpha_xw;
+    if (alpha.x == 0.0f) return;
+    stream_pipelined<4, XItemDw>(
+        blockIdx.x * NT + threadIdx.x, n2, gridDim.x * NT, [&](unsigned k) { return XItemDw{p[k], x[k]}; },
+        [&](unsigned k, const XItemDw& it) { x[k] = x_item(it.x, it.p, alpha); });
 }
 
 // xb += xw (in FP64), xw = 0: the double-word correction goes into the base.
@@ -347,31 +349,29 @@ void launch_residual_x(cudaStream_t st, const OpView& o, const double* diag, con
                                             red.maxb, cond);
 }
 
-void launch_apply_dw(cudaStream_t st, const OpView& o, const float2* dgw, const float2* p,
-                     float2* Ap, Ctl* ctl, const Red& red, Cond cond) {
-    static const int wb = wave_blocks(k_apply_dw_rows, 1 << 30);
-    launch_pdl(k_apply_dw_rows, std::min(red.maxb, wb), NT, 0, st, o, dgw, p, Ap, ctl, red.part, red.maxb, cond);
+void launch_az_dw(cudaStream_t st, const OpView& o, const float2* dgw, const float* z, const float2* r,
+                  const float2* Ap, float2* w, Ctl* ctl, const Red& red, Cond cond) {
+    static const int wb = wave_blocks(k_az_dw, 1 << 30);
+    launch_pdl(k_az_dw, std::min(red.maxb, wb), NT, 0, st, o, dgw, z, r, Ap, w, ctl, red.part, red.maxb, cond);
 }
 
-void launch_update_dw(cudaStream_t st, unsigned n, const float2* p, const float2* Ap, float2* x,
-                      float2* r, float* b0, Ctl* ctl, const Red& red, Cond cond) {
-    static const int wb = wave_blocks(k_update_dw, 1 << 30);
-    launch_pdl(k_update_dw, std::min(red.blocks, wb), NT, 0, st, n / 2, (const float4*)p, (const float4*)Ap, (float4*)x,
-                                           (float4*)r, (float2*)b0, ctl, red.part, red.maxb, cond);
+void launch_step_dw(cudaStream_t st, unsigned n, const float* z, const float2* w, float2* p, float2* Ap, float2* x,
+                    float2* r, float* b0, Ctl* ctl, const Red& red, Cond cond, bool write_x) {
+    auto go = [&](auto kern, int wb) {
+        launch_pdl(kern, std::min(red.blocks, wb), NT, 0, st, n / 2, (const float2*)z, (const float4*)w, (float4*)p,
+                   (float4*)Ap, (float4*)x, (float4*)r, (float2*)b0, ctl, red.part, red.maxb, cond);
+    };
+    static const int wx = wave_blocks(k_step_dw<true>, 1 << 30), wr = wave_blocks(k_step_dw<false>, 1 << 30);
+    if (write_x)
+        go(k_step_dw<true>, wx);
+    else
+        go(k_step_dw<false>, wr);
 }
 
-void launch_dot_dw(cudaStream_t st, unsigned n, const float2* r, const float* z, const float2* Ap,
-                   Ctl* ctl, const Red& red, Cond cond) {
-    static const int wb = wave_blocks(k_dot_dw, 1 << 30);
-    launch_pdl(k_dot_dw, std::min(std::max(1, red.maxb / 2), wb), NT, 0, st, n / 2, (const float4*)r,
-               (const float2*)z, (const float4*)Ap, ctl, red.part, red.maxb, cond);
-}
-
-void launch_update_p_dw(cudaStream_t st, unsigned n, const float* z, float2* p, Ctl* ctl,
-                        Cond cond) {
-    static const int wb = wave_blocks(k_update_p_dw, 1 << 30);
-    launch_pdl(k_update_p_dw, std::min((int)blocks_of(n / 2), wb), NT, 0, st, n / 2, (const float2*)z, (float4*)p, ctl,
-               cond);
+void launch_update_x_dw(cudaStream_t st, unsigned n, const float2* p, float2* x, const Ctl* ctl, int blocks) {
+    static const int wb = wave_blocks(k_update_x_dw, 1 << 30);
+    const int want = std::min((int)blocks_of(n / 2), wb);
+    k_update_x_dw<<<blocks > 0 ? std::min(blocks, want) : want, NT, 0, st>>>(n / 2, (const float4*)p, (float4*)x, ctl);
 }
 
 void launch_to_dw(cudaStream_t st, unsigned n, const double* in, float2* out) {

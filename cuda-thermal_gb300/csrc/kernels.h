@@ -175,14 +175,12 @@ void launch_residual_x(cudaStream_t st, const OpView& o, const double* diag, con
 // xb += xw in FP64, xw = 0 (skipped once the solve is done when check_done).
 void launch_fold(cudaStream_t st, unsigned n, double* xb, float2* xw, const Ctl* ctl,
                  bool check_done);
-void launch_apply_dw(cudaStream_t st, const OpView& o, const float2* dgw, const float2* p,
-                     float2* Ap, Ctl* ctl, const Red& red, Cond cond);
-void launch_update_dw(cudaStream_t st, unsigned n, const float2* p, const float2* Ap, float2* x,
-                      float2* r, float* b0, Ctl* ctl, const Red& red, Cond cond);
-void launch_dot_dw(cudaStream_t st, unsigned n, const float2* r, const float* z, const float2* Ap,
-                   Ctl* ctl, const Red& red, Cond cond);
-void launch_update_p_dw(cudaStream_t st, unsigned n, const float* z, float2* p, Ctl* ctl,
-                        Cond cond);
+// The iteration, as launch_az64, launch_step64 and launch_update_x do it.
+void launch_az_dw(cudaStream_t st, const OpView& o, const float2* dgw, const float* z, const float2* r,
+                  const float2* Ap, float2* w, Ctl* ctl, const Red& red, Cond cond);
+void launch_step_dw(cudaStream_t st, unsigned n, const float* z, const float2* w, float2* p, float2* Ap, float2* x,
+                    float2* r, float* b0, Ctl* ctl, const Red& red, Cond cond, bool write_x);
+void launch_update_x_dw(cudaStream_t st, unsigned n, const float2* p, float2* x, const Ctl* ctl, int blocks);
 void launch_to_dw(cudaStream_t st, unsigned n, const double* in, float2* out);
 void launch_dw_to_natural(cudaStream_t st, const Geo& g, const float2* split, double* nat);
 void launch_natural_to_dw(cudaStream_t st, const Geo& g, const double* nat, float2* split);

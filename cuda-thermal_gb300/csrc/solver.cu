@@ -128,7 +128,7 @@ ct_status Solver::create(const ct_model* m_in, ct_precond pc_, ct_precision prec
     const size_t o_gE = ar.take(n * 4), o_gN = ar.take(n * 4), o_gU = ar.take(n * 4);
     const size_t o_cap = ar.take(n * 4), o_gB = ar.take((size_t)g0.plane * 4);
     size_t o_vec[9];
-    const size_t o_w = mt != MG_NONE && !dw ? ar.take((size_t)n * 8) : 0;
+    const size_t o_w = mt != MG_NONE ? ar.take((size_t)n * 8) : 0;
     for (size_t& o : o_vec) o = ar.take((size_t)n * 8);
     const size_t o_invd = pc == CT_JACOBI ? ar.take((size_t)n * 8) : 0;
     const size_t o_dgw = dw ? ar.take((size_t)n * 8) : 0;
@@ -489,6 +489,7 @@ void Solver::enqueue_init(Cond cond) {
 
 void Solver::enqueue_replace(Cond cond) {
     float* b0 = at<float>(lv[0].o_b);
+    if (x_lag()) enq("pcg_update_x", (double)ncells * 24, [&] { update_x(cs, 0); });  // phase 1's last
     enq("pcg_fold_x", (double)ncells * 32, [&] { launch_fold(cs, n, x, xwc, ctl, true); });
     enq("pcg_residual_fp64", (double)ncells * (36 + 8 + 8 + 4), [&] {
         launch_residual_x(cs, op(), diag, b, x, rw(), b0, false, ctl, red_cols(SL_INIT), cond);
@@ -498,20 +499,6 @@ void Solver::enqueue_replace(Cond cond) {
 void Solver::enqueue_body(Cond cond) {
     const double N = (double)ncells;
     const void* z = nullptr;
-    if (dw) {
-        vcycle<float>(0, cond);
-        const float* zf = at<float>(lv[0].o_x);
-        float* b0 = at<float>(lv[0].o_b);
-        enq("pcg_dot", N * (8 + 4 + 8),
-            [&] { launch_dot_dw(cs, n, rw(), zf, Apw(), ctl, red_vec(SL_DOT), cond); });
-        enq("pcg_update_p", N * (4 + 16), [&] { launch_update_p_dw(cs, n, zf, pw(), ctl, cond); });
-        enq("pcg_apply", N * 36,
-            [&] { launch_apply_dw(cs, op(), dgw, pw(), Apw(), ctl, red_cols(SL_APPLY), cond); });
-        enq("pcg_update_xr", N * (48 + 4), [&] {
-            launch_update_dw(cs, n, pw(), Apw(), xw(), rw(), b0, ctl, red_vec(SL_UPDATE), cond);
-        });
-        return;
-    }
     // x += alpha p of the previous iteration beside this V-cycle (x_lag())
     lag_now = x_lag();
     forked = false;
@@ -532,6 +519,18 @@ void Solver::enqueue_body(Cond cond) {
         return;
     }
     const double zb = (double)tsize;
+    if (dw) {
+        const float* zf = (const float*)z;
+        enq("pcg_apply", N * (zb + 12 + 8 + 16 + 8),
+            [&] { launch_az_dw(cs, op(), dgw, zf, rw(), Apw(), ww(), ctl, red_cols(SL_APPLY), cond); });
+        if (lag_now && !prof) cudaStreamWaitEvent(cs, ev_join, 0);
+        enq("pcg_update_xr", N * (zb + 8 + 3 * 16 + zb + (lag_now ? 0 : 16)), [&] {
+            launch_step_dw(cs, n, zf, ww(), pw(), Apw(), xw(), rw(), at<float>(lv[0].o_b), ctl, red_vec(SL_UPDATE),
+                           cond, !lag_now);
+        });
+        lag_now = false;
+        return;
+    }
     enq("pcg_apply", N * (zb + 12 + 8 + 16 + 8),
         [&] { launch_az64(cs, mt, flex, op(), diag, z, r, Ap, w, ctl, red_cols(SL_APPLY), cond); });
     // the step overwrites the p that the x update reads: join first
@@ -542,15 +541,23 @@ void Solver::enqueue_body(Cond cond) {
     lag_now = false;
 }
 
+// The pending x update, on `blocks` blocks (0: as many as it wants).
+void Solver::update_x(cudaStream_t s, int blocks) {
+    if (dw)
+        launch_update_x_dw(s, n, pw(), xw(), ctl, blocks);
+    else
+        launch_update_x(s, n, p, x, ctl, blocks);
+}
+
 void Solver::fork_x() {
     forked = true;
     if (prof) {  // timed in line, on as many blocks as it wants
-        enq("pcg_update_x", (double)ncells * 24, [&] { launch_update_x(cs, n, p, x, ctl, 0); });
+        enq("pcg_update_x", (double)ncells * 24, [&] { update_x(cs, 0); });
         return;
     }
     cudaEventRecord(ev_fork, cs);
     cudaStreamWaitEvent(st_side, ev_fork, 0);
-    launch_update_x(st_side, n, p, x, ctl, xlag_blocks);
+    update_x(st_side, xlag_blocks);
     cudaEventRecord(ev_join, st_side);
 }
 
@@ -602,10 +609,11 @@ ct_status Solver::record_graphs() {
             cs = st;
             enqueue_init(Cond{h1, 1});
             ok = add_while(h1);
-            if (ok && x_lag()) launch_update_x(st, n, p, x, ctl, 0);  // the last iteration's x update
+            if (ok && x_lag() && !dw) update_x(st, 0);  // the last iteration's x update
             if (ok && dw) {
                 enqueue_replace(Cond{h2, 1});
                 ok = add_while(h2);
+                if (ok && x_lag()) update_x(st, 0);
             }
             cudaGraph_t outg = nullptr;
             const bool ended = cudaStreamEndCapture(st, &outg) == cudaSuccess;
@@ -697,7 +705,7 @@ ct_status Solver::solve(double tol, int maxit, ct_stats* out) {
             launched += k;
             if (graphs) k = std::min(k * 2, 8);
         }
-        if (x_lag()) launch_update_x(st, n, p, x, ctl, 0);  // the last iteration's x update
+        if (x_lag()) update_x(st, 0);  // the last iteration's x update
     }
     CT_CK(cudaGetLastError());
     return finish_solve(out);

@@ -97,12 +97,13 @@ class Solver {
     cudaStream_t st_side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     bool lag_now = false, forked = false;  // while a body is enqueued
-    bool x_lag() const { return xlag >= 0 && !dw && mt != MG_NONE && st_side; }
+    bool x_lag() const { return xlag >= 0 && mt != MG_NONE && st_side; }
     // the last level with a restriction out of it, at most xlag (a V-cycle
     // all in the shared-memory bottom: lv.size(), the start of the body)
     int fork_level() const {
         return small_k0 == 0 ? (int)lv.size() : std::min(xlag, (int)small_k0 - 1);
     }
+    void update_x(cudaStream_t s, int blocks);
     void fork_x();
     // queued host copies (ct_set_power_async, ct_get_x_async): two staging
     // buffers each way, a copy stream each way, events that keep a buffer
@@ -238,6 +239,7 @@ class Solver {
     float2* rw() const { return reinterpret_cast<float2*>(r); }
     float2* pw() const { return reinterpret_cast<float2*>(p); }
     float2* Apw() const { return reinterpret_cast<float2*>(Ap); }
+    float2* ww() const { return reinterpret_cast<float2*>(w); }
     // x as split-layout FP64: in the double-word mode the correction is first
     // folded into the FP64 base (which leaves x unchanged).
     const double* x_as_double(double*) const {
