@@ -59,7 +59,6 @@ namespace {
 
 // Items per block of the stages whose tile is not tuned.
 constexpr unsigned kVecChunk = 4096;   // value pairs (fold, update, dot, p, rhs)
-constexpr unsigned kColChunk = 512;    // fine columns (FP64 residual)
 // fine rows of one colour and plane per block of the operator apply: the
 // FP64 apply is FP64-pipe-bound, and per-block reduction overhead weighs less
 // on longer tables (256 instances, two cells per lane: 16 / 32 / 64 / 128 rows
@@ -120,7 +119,7 @@ class Batch {
         cudaStream_t st = nullptr, st_body = nullptr;
         cudaGraphExec_t gx = nullptr;
         BCtl* bc = nullptr;
-        Plan vec{}, cols{}, rows{};  // value pairs, fine columns, fine rows
+        Plan vec{}, rows{};  // value pairs, fine rows
         BRed r_res{}, r_apply{}, r_update{};
         std::vector<Plan> sweep, restr;
         std::vector<unsigned> sweep_tile, restr_tile;
@@ -436,11 +435,10 @@ ct_status Batch::build_bucket(Bucket& b) {
     ct_status s;
     if ((s = dalloc(&b.bc, sizeof(BCtl))) != CT_OK) return s;
     CT_BK(cudaMemsetAsync(b.bc, 0, sizeof(BCtl), st));
-    std::vector<unsigned> pairs, cols, rows;
+    std::vector<unsigned> pairs, rows;
     for (int i : b.inst) {
         const Solver& v = inst(i);
         pairs.push_back(v.n / 2);
-        cols.push_back(v.g0.plane);
         rows.push_back(2u * (unsigned)v.g0.ny * (unsigned)v.g0.nz);
         b.mz = std::max(b.mz, v.g0.nz);
         TailLevels<float> tl;
@@ -449,10 +447,8 @@ ct_status Batch::build_bucket(Bucket& b) {
         b.smem = std::max(b.smem, small_smem_bytes(tl));
     }
     if ((s = upload_plan(make_plan(ni, b.inst, pairs, kVecChunk), &b.vec)) != CT_OK) return s;
-    if ((s = upload_plan(make_plan(ni, b.inst, cols, kColChunk), &b.cols)) != CT_OK) return s;
     if ((s = upload_plan(make_plan(ni, b.inst, rows, dw ? kRowChunkDw : kRowChunk64), &b.rows)) != CT_OK) return s;
-    // the start residual walks columns (double words) or rows (FP64)
-    if ((s = make_red(dw ? b.cols : b.rows, &b.r_res)) != CT_OK) return s;
+    if ((s = make_red(b.rows, &b.r_res)) != CT_OK) return s;
     if ((s = make_red(b.rows, &b.r_apply)) != CT_OK) return s;
     if ((s = make_red(b.vec, &b.r_update)) != CT_OK) return s;
     if ((s = upload(&b.small_insts, b.inst)) != CT_OK) return s;
@@ -708,7 +704,7 @@ void Batch::enqueue_init(Bucket& b, cudaStream_t s, Cond cond) {
     }
     enq(s, "b_fold", N * 32, [&] { launch_b_fold(s, b.vec, bi, ctl, 0); });
     enq(s, "b_residual", N * 56,
-        [&] { launch_b_residual(s, b.cols, bi, ctl, b.r_res, 1, b.bc, cond); });
+        [&] { launch_b_residual(s, b.rows, bi, ctl, b.r_res, 1, b.bc, cond); });
 }
 
 void Batch::enqueue_body(Bucket& b, cudaStream_t s, Cond cond) {
@@ -726,7 +722,7 @@ void Batch::enqueue_body(Bucket& b, cudaStream_t s, Cond cond) {
     // (blocks of the other instances return at entry)
     enq(s, "b_fold_pe", 0, [&] { launch_b_fold(s, b.vec, bi, ctl, 1); });
     enq(s, "b_residual_pe", 0,
-        [&] { launch_b_residual(s, b.cols, bi, ctl, b.r_res, 0, b.bc, cond); });
+        [&] { launch_b_residual(s, b.rows, bi, ctl, b.r_res, 0, b.bc, cond); });
 }
 
 ct_status Batch::record(Bucket& b) {

@@ -51,6 +51,12 @@ __device__ __forceinline__ float narrow(double d) {
     return (float)d;
 }
 
+// A double as a float pair: dw_of (dw_dev.cuh) without its three conversions.
+__device__ __forceinline__ float2 split(double d) {
+    const float h = narrow(d);
+    return make_float2(h, narrow(d - widen(h)));
+}
+
 // The V-cycle's values as doubles: T = float (widened) or double (as is).
 __device__ __forceinline__ double to_d(float v) { return widen(v); }
 __device__ __forceinline__ double to_d(double v) { return v; }

@@ -12,6 +12,7 @@
 #include "batch.h"
 #include "batch_dev.cuh"
 #include "dw_dev.cuh"
+#include "f64_dev.cuh"
 #include "mg_dev.cuh"
 #include "reduce.cuh"
 #include "setup_dev.cuh"
@@ -19,6 +20,7 @@
 namespace ct {
 
 using namespace dwdev;
+using namespace f64dev;
 using namespace mgdev;
 
 namespace {
@@ -56,65 +58,50 @@ __global__ void __launch_bounds__(NT)
 }
 
 // r = b - A x in FP64 from the FP64 base x: the start of a solve, or (start
-// = 0) the residual replacement of instances whose first phase ended.
-__global__ void __launch_bounds__(NT)
+// = 0) the residual replacement of instances whose first phase ended. Items =
+// rows of one colour and plane (k_residual_x; a start from x = 0 splits b).
+__global__ void __launch_bounds__(NT, 4)
     kb_residual(Plan p, const BInst* __restrict__ bi, Ctl* ctl, BRed red, int start, BCtl* bc,
                 Cond cond) {
     pdl_enter();
     const Task t = p.tasks[blockIdx.x];
     Ctl* c = &ctl[t.inst];
     if (inst_done(c) || (!start && !c->phase_end)) return;
-    const BInst I = bi[t.inst];
-    const Geo& g = I.o.g;
+    const BInst& I = bi[t.inst];
+    const OpView o = I.o;
+    const double *const diag = I.diag, *const x = I.x, *const b = I.b;
+    float2* const r = I.r;
+    float* const b0 = I.b0;
     const bool zero = start && c->x_zero;
+    const int lane = (int)(threadIdx.x & 31u);
     double rr = 0.0, bb = 0.0;
-    for (unsigned s = t.begin + threadIdx.x; s < t.end; s += NT) {
-        const Col cl = col_of_slot(g, s);
-        if (!cl.valid) {
-            for (int l = 0; l < g.nz; ++l) {
-                I.r[(unsigned)l * g.plane + s] = make_float2(0.0f, 0.0f);
-                I.b0[(unsigned)l * g.plane + s] = 0.0f;
-            }
-            continue;
-        }
+    for (unsigned R = t.begin + (threadIdx.x >> 5); R < t.end; R += NT / 32) {
         if (zero) {
-            for (int l = 0; l < g.nz; ++l) {
-                const unsigned id = (unsigned)l * g.plane + cl.s;
-                const double bv = I.b[id];
-                const float2 rw = dw_of(bv);
-                I.r[id] = rw;
-                I.b0[id] = rw.x;
-                bb += bv * bv;
-                rr += bv * bv;
+            const unsigned s0 = R * (unsigned)o.g.hx;
+            for (unsigned s = s0 + (unsigned)lane; s < s0 + (unsigned)o.g.hx; s += 32u) {
+                const double bv = b[s];
+                const float2 rw = split(bv);
+                r[s] = rw;
+                b0[s] = rw.x;
+                bb = __fma_rn(bv, bv, bb);
             }
-            continue;
-        }
-        double x_c = I.x[cl.s], x_b = 0.0;
-        float gu_b = 0.0f;
-        for (int l = 0; l < g.nz; ++l) {
-            const unsigned base = (unsigned)l * g.plane, id = base + cl.s;
-            const bool up = l < g.nz - 1;
-            const double x_a = up ? I.x[id + g.plane] : 0.0;
-            const float gu = I.o.gU[id];
-            double off = 0.0;
-            if (cl.i > 0) off += (double)I.o.gE[base + cl.sw] * I.x[base + cl.sw];
-            if (cl.i < g.nx - 1) off += (double)I.o.gE[id] * I.x[base + cl.se];
-            if (cl.j > 0) off += (double)I.o.gN[base + cl.ss] * I.x[base + cl.ss];
-            if (cl.j < g.ny - 1) off += (double)I.o.gN[id] * I.x[base + cl.sn];
-            if (l > 0) off += (double)gu_b * x_b;
-            if (up) off += (double)gu * x_a;
-            const double bv = I.b[id];
-            const double rv = bv - (I.diag[id] * x_c - off);
-            const float2 rw = dw_of(rv);
-            I.r[id] = rw;
-            I.b0[id] = rw.x;
-            rr += rv * rv;
-            bb += bv * bv;
-            x_b = x_c;
-            x_c = x_a;
-            gu_b = gu;
+        } else {
+            row64<1>(o, diag, x, R, lane, [&](unsigned k, bool valid, double ax, double) {
+                if (!valid) {
+                    r[k] = make_float2(0.0f, 0.0f);
+                    b0[k] = 0.0f;
+                    return;
+                }
+                const double bv = b[k], rv = bv - ax;
+                const float2 rw = split(rv);
+                r[k] = rw;
+                b0[k] = rw.x;
+                rr = __fma_rn(rv, rv, rr);
+                bb = __fma_rn(bv, bv, bb);
+            });
         }
     }
+    if (zero) rr = bb;
     block_sum2(rr, bb);
     if (publish_inst(rr, bb, red, p.ntasks, t.inst, p.inst_count[t.inst])) {
         double RR, BB;

@@ -29,24 +29,28 @@
 #include <cstdlib>
 
 #include "dw_dev.cuh"
+#include "f64_dev.cuh"
 #include "kernels.h"
 #include "reduce.cuh"
 
 namespace ct {
 
 using namespace dwdev;
+using namespace f64dev;
 
 namespace {
 
 // ---- FP64 residual from a double-word x: start and replacement -------------
 
-// r = b - (A + C/dt) x in FP64 with x = hi + lo, the stored FP64 diagonal;
+// r = b - (A + C/dt) x in FP64 from the folded base x, the stored FP64 diagonal;
 // stores r as a double word and b0 = r (float, the V-cycle's input). `start`:
 // the first residual of a solve (sets ||b||^2 and the start test); otherwise
 // the residual replacement (phase 2 begins, or the solve ends if already
-// converged).
-__global__ void __launch_bounds__(NT)
-    k_residual_x(OpView o, const double* __restrict__ diag, const double* __restrict__ b,
+// converged). One warp per row of one colour of one plane, as k_residual64, with
+// integer conversions: 640 x 640 x 10 from an x that is not zero 145 us, where a
+// thread per column with the hardware's conversions took 222.
+__global__ void __launch_bounds__(NT, 4)
+    k_residual_x(OpView o, unsigned n, const double* __restrict__ diag, const double* __restrict__ b,
                  const double* __restrict__ x, float2* __restrict__ r, float* __restrict__ b0,
                  int start, Ctl* ctl, double* part, int maxb, Cond cond) {
     pdl_enter();
@@ -60,51 +64,36 @@ __global__ void __launch_bounds__(NT)
     double rr = 0.0, bb = 0.0;
     // A solve that starts from x = 0 (every steady solve) has r = b exactly.
     const bool zero = start && ctl->x_zero;
-    for (unsigned s = blockIdx.x * NT + threadIdx.x; s < g.plane; s += gridDim.x * NT) {
-        const Col c = col_of_slot(g, s);
-        if (!c.valid) {
-            for (int l = 0; l < g.nz; ++l) {
-                r[(unsigned)l * g.plane + s] = make_float2(0.0f, 0.0f);
-                b0[(unsigned)l * g.plane + s] = 0.0f;
-            }
-            continue;
-        }
-        if (zero) {
-            for (int l = 0; l < g.nz; ++l) {
-                const unsigned id = (unsigned)l * g.plane + c.s;
-                const double bi = b[id];
-                const float2 rw = dw_of(bi);
-                r[id] = rw;
-                b0[id] = rw.x;
-                bb += bi * bi;
-            }
-            continue;
-        }
-        double x_c = x[c.s], x_b = 0.0;
-        float gu_b = 0.0f;
-        for (int l = 0; l < g.nz; ++l) {
-            const unsigned base = (unsigned)l * g.plane, id = base + c.s;
-            const bool up = l < g.nz - 1;
-            const double x_a = up ? x[id + g.plane] : 0.0;
-            const float gu = o.gU[id];
-            double off = 0.0;
-            if (c.i > 0) off += (double)o.gE[base + c.sw] * x[base + c.sw];
-            if (c.i < g.nx - 1) off += (double)o.gE[id] * x[base + c.se];
-            if (c.j > 0) off += (double)o.gN[base + c.ss] * x[base + c.ss];
-            if (c.j < g.ny - 1) off += (double)o.gN[id] * x[base + c.sn];
-            if (l > 0) off += (double)gu_b * x_b;
-            if (up) off += (double)gu * x_a;
-            const double bi = b[id];
-            const double ri = bi - (diag[id] * x_c - off);
-            const float2 rw = dw_of(ri);
-            r[id] = rw;
-            b0[id] = rw.x;
-            rr += ri * ri;
-            bb += bi * bi;
-            x_b = x_c;
-            x_c = x_a;
-            gu_b = gu;
-        }
+    if (zero) {
+        const double2* b2 = reinterpret_cast<const double2*>(b);
+        float4* r2 = reinterpret_cast<float4*>(r);
+        float2* b02 = reinterpret_cast<float2*>(b0);
+        stream_pipelined<2, double2>(
+            blockIdx.x * NT + threadIdx.x, n / 2, gridDim.x * NT, [&](unsigned k) { return b2[k]; },
+            [&](unsigned k, const double2& v) {
+                const float2 u = split(v.x), w = split(v.y);
+                r2[k] = make_float4(u.x, u.y, w.x, w.y);
+                b02[k] = make_float2(u.x, w.x);
+                bb = __fma_rn(v.x, v.x, bb);
+                bb = __fma_rn(v.y, v.y, bb);
+            });
+    } else {
+        const unsigned rows = 2u * (unsigned)g.ny * (unsigned)g.nz;
+        const int lane = (int)(threadIdx.x & 31u);
+        for (unsigned R = blockIdx.x * (NT / 32) + (threadIdx.x >> 5); R < rows; R += gridDim.x * (NT / 32))
+            row64<1>(o, diag, x, R, lane, [&](unsigned k, bool valid, double ax, double) {
+                if (!valid) {
+                    r[k] = make_float2(0.0f, 0.0f);
+                    b0[k] = 0.0f;
+                    return;
+                }
+                const double bi = b[k], ri = bi - ax;
+                const float2 rw = split(ri);
+                r[k] = rw;
+                b0[k] = rw.x;
+                rr = __fma_rn(ri, ri, rr);
+                bb = __fma_rn(bi, bi, bb);
+            });
     }
     if (zero) rr = bb;
     block_sum2(rr, bb);
@@ -341,11 +330,11 @@ void launch_fold(cudaStream_t st, unsigned n, double* xb, float2* xw, const Ctl*
                                                                check_done ? 1 : 0);
 }
 
-void launch_residual_x(cudaStream_t st, const OpView& o, const double* diag, const double* b,
+void launch_residual_x(cudaStream_t st, const OpView& o, unsigned n, const double* diag, const double* b,
                        const double* x, float2* r, float* b0, bool start, Ctl* ctl,
                        const Red& red, Cond cond) {
     static const int wb = wave_blocks(k_residual_x, 1 << 30);
-    launch_pdl(k_residual_x, std::min(red.blocks, wb), NT, 0, st, o, diag, b, x, r, b0, start ? 1 : 0, ctl, red.part,
+    launch_pdl(k_residual_x, std::min(red.blocks, wb), NT, 0, st, o, n, diag, b, x, r, b0, start ? 1 : 0, ctl, red.part,
                                             red.maxb, cond);
 }
 

@@ -169,7 +169,7 @@ void launch_record_keep(cudaStream_t st, const Ctl* ctl, double dt, StepEntry* t
 // ---- double-word outer PCG (FP32 pipes), k_dw.cu -----------------------------
 // r = b - A x in FP64 from the double-word x; start of a solve, or the residual
 // replacement that begins phase 2.
-void launch_residual_x(cudaStream_t st, const OpView& o, const double* diag, const double* b,
+void launch_residual_x(cudaStream_t st, const OpView& o, unsigned n, const double* diag, const double* b,
                        const double* x, float2* r, float* b0, bool start, Ctl* ctl,
                        const Red& red, Cond cond);
 // xb += xw in FP64, xw = 0 (skipped once the solve is done when check_done).

@@ -477,7 +477,7 @@ void Solver::enqueue_init(Cond cond) {
     if (dw) {
         enq("pcg_fold_x", (double)ncells * 32, [&] { launch_fold(cs, n, x, xwc, ctl, false); });
         enq("pcg_residual_fp64", (double)ncells * (36 + 8 + 8 + 4), [&] {
-            launch_residual_x(cs, op(), diag, b, x, rw(), (float*)b0, true, ctl,
+            launch_residual_x(cs, op(), n, diag, b, x, rw(), (float*)b0, true, ctl,
                               red_cols(SL_INIT), cond);
         });
         return;
@@ -492,7 +492,7 @@ void Solver::enqueue_replace(Cond cond) {
     if (x_lag()) enq("pcg_update_x", (double)ncells * 24, [&] { update_x(cs, 0); });  // phase 1's last
     enq("pcg_fold_x", (double)ncells * 32, [&] { launch_fold(cs, n, x, xwc, ctl, true); });
     enq("pcg_residual_fp64", (double)ncells * (36 + 8 + 8 + 4), [&] {
-        launch_residual_x(cs, op(), diag, b, x, rw(), b0, false, ctl, red_cols(SL_INIT), cond);
+        launch_residual_x(cs, op(), n, diag, b, x, rw(), b0, false, ctl, red_cols(SL_INIT), cond);
     });
 }
 
