@@ -189,15 +189,17 @@ __device__ __forceinline__ float2 az_dw(const CellZ<float, float2>& a) {
     return fast_two_sum(r.s, r.c);
 }
 
-// What the dots of one cell need beside its operands.
-struct DotItem {
-    float2 r, ap;
-};
-// v[0] += r.z, v[1] += z.Ap, v[2] += z.Az.
-__device__ __forceinline__ void dots_dw(DwAcc (&v)[3], const DotItem& m, float zc, float2 az) {
-    acc_mul_f(v[0], m.r, zc);
-    acc_mul_f(v[1], m.ap, zc);
-    acc_mul_f(v[2], az, zc);
+// w = A z of a pair; v[0] += r.z, v[1] += z.Ap, v[2] += z.w (r, Ap and z of a
+// padding slot are zero).
+__device__ __forceinline__ void dots_dw(DwAcc (&v)[3], const PairZ<float, float2>& a, float4 r, float4 ap, float2* w) {
+    const float2 w0 = az_dw(a.c[0]), w1 = a.second ? az_dw(a.c[1]) : make_float2(0.0f, 0.0f);
+    *reinterpret_cast<float4*>(w + a.k) = make_float4(w0.x, w0.y, w1.x, w1.y);
+    acc_mul_f(v[0], make_float2(r.x, r.y), a.c[0].zc);
+    acc_mul_f(v[1], make_float2(ap.x, ap.y), a.c[0].zc);
+    acc_mul_f(v[2], w0, a.c[0].zc);
+    acc_mul_f(v[0], make_float2(r.z, r.w), a.c[1].zc);
+    acc_mul_f(v[1], make_float2(ap.z, ap.w), a.c[1].zc);
+    acc_mul_f(v[2], w1, a.c[1].zc);
 }
 
 // The step of a pair of values: p = z + beta p, Ap = w + beta Ap (p = z and

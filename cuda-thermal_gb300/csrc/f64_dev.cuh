@@ -146,6 +146,22 @@ __device__ __forceinline__ double az64(const CellZ<T, double>& a) {
     return __fma_rn(a.dg, to_d(a.zc), -sum6(a.g, a.z));
 }
 
+// w = A z of a pair; v[0] += r.z, v[1] += z.Ap, v[2] += z.w.
+template <class T>
+__device__ __forceinline__ void dots64(double (&v)[3], const PairZ<T, double>& a, double2 r, double2 ap, double* w) {
+    const double z0 = to_d(a.c[0].zc), z1 = to_d(a.c[1].zc);
+    const double w0 = az64(a.c[0]), w1 = a.second ? az64(a.c[1]) : 0.0;
+    *reinterpret_cast<double2*>(w + a.k) = make_double2(w0, w1);
+    v[0] = __fma_rn(r.x, z0, v[0]);
+    v[1] = __fma_rn(z0, ap.x, v[1]);
+    v[2] = __fma_rn(z0, w0, v[2]);
+    if (a.second) {
+        v[0] = __fma_rn(r.y, z1, v[0]);
+        v[1] = __fma_rn(z1, ap.y, v[1]);
+        v[2] = __fma_rn(z1, w1, v[2]);
+    }
+}
+
 // ---- the FP64 operator apply, one warp per row (single solver and batch) ----
 
 // Operands of one cell, loaded before any is used (absent neighbours stay

@@ -136,8 +136,10 @@ __global__ void __launch_bounds__(NT, 4)
 }
 
 // w = (A + C/dt) z, r.z, z.Ap, z.w, then the instance's beta, p.Ap and alpha
-// (k_az_dw); items = rows of one colour and plane.
-__global__ void __launch_bounds__(NT, 4)
+// (k_az_dw); items = rows of one colour and plane, walked in pairs of slots. 16
+// stacks of 256 x 256 x 10: 115 us a launch, 127 compiled for 4 blocks per SM, 139
+// a cell a lane.
+__global__ void __launch_bounds__(NT, 3)
     kb_az_dw(Plan p, const BInst* __restrict__ bi, Ctl* ctl, BRed red, BCtl* bc, Cond cond) {
     pdl_enter();
     const Task t = p.tasks[blockIdx.x];
@@ -148,17 +150,16 @@ __global__ void __launch_bounds__(NT, 4)
     const float2 *const r = I.r, *const Ap = I.Ap;
     float2* const w = I.w;
     const bool first = c->iter == 0;  // no Ap yet
-    const int lane = (int)(threadIdx.x & 31u);
+    const float2* __restrict__ dgw = I.dgw;
+    const float* __restrict__ z = I.z;
+    const unsigned h = (unsigned)o.g.hx / 2u;  // pairs a row
     DwAcc v[3] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
-    for (unsigned R = t.begin + (threadIdx.x >> 5); R < t.end; R += NT / 32)
-        row_z<1>(
-            o, I.dgw, I.z, R, lane,
-            [&](unsigned k) { return DotItem{r[k], first ? make_float2(0.0f, 0.0f) : Ap[k]}; },
-            [&](unsigned k, const DotItem& m, const CellZ<float, float2>& a) {
-                const float2 az = az_dw(a);
-                w[k] = az;
-                dots_dw(v, m, a.zc, az);
-            });
+    for (unsigned q = t.begin * h + threadIdx.x; q < t.end * h; q += NT) {
+        PairZ<float, float2> a;
+        if (!load_pair(o, dgw, z, q, a)) continue;
+        const float4 rv = load_two(r, a.k), av = first ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : load_two(Ap, a.k);
+        dots_dw(v, a, rv, av, w);
+    }
     pdl_trigger();
     const unsigned count = (unsigned)p.inst_count[t.inst];
     if (publish_acc<3>(v, red.part, p.ntasks, blockIdx.x, &red.tickets[t.inst], count)) {

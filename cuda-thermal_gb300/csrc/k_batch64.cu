@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(NT, 4)
         double r, ap;
     };
     for (unsigned R = t.begin + (threadIdx.x >> 5); R < t.end; R += NT / 32)
-        row_z<1>(
+        row_z(
             o, I.diag, I.z, R, lane, [&](unsigned k) { return More{r[k], first ? 0.0 : Ap[k]}; },
             [&](unsigned k, const More& m, const CellZ<float, double>& a) {
                 const double az = az64(a), zc = to_d(a.zc);

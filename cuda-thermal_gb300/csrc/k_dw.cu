@@ -131,35 +131,29 @@ __global__ void __launch_bounds__(NT, 4)
 
 // ---- the iteration ------------------------------------------------------------
 
-constexpr int kRowZ = 1;   // cells a lane and step of k_az_dw
 constexpr int kStepU = 2;  // pairs a thread and step of k_step_dw
 
-// w = (A + C/dt) z, r.z, z.Ap and z.w in one pass (one warp per row of one colour
-// of one plane), then beta, p.Ap and alpha (next_scalars): the step below makes
+// w = (A + C/dt) z, r.z, z.Ap and z.w in one pass (two neighbouring slots of one
+// colour a thread, half the loads and indexing of a cell a lane), then beta, p.Ap and alpha (next_scalars): the step below makes
 // A p from w, so neither a dot pass nor an apply on p follows.
-// 640 x 640 x 10: 48.8 us (4.0 TB/s), and the step 43.8 us (6.0 TB/s), where the
+// 640 x 640 x 10: 44.8 us (4.4 TB/s; 48.8 a cell a lane, 52.8 at 3 blocks per SM),
+// and the step 43.8 us (6.0 TB/s), where the
 // dots, the p update, the apply on p and the update of x and r took 22.5 + 14.1 +
 // 47.1 + 36.1 us; the x update (16.1 us alone) hides beside the V-cycle's bottom.
-// A solve: 3.81 ms against 4.04.
 __global__ void __launch_bounds__(NT, 4)
     k_az_dw(OpView o, const float2* __restrict__ dgw, const float* __restrict__ z, const float2* __restrict__ r,
             const float2* __restrict__ Ap, float2* __restrict__ w, Ctl* ctl, double* part, int maxb, Cond cond) {
     pdl_enter();
     if (loop_done(ctl, cond)) return;
-    const Geo& g = o.g;
     const bool first = ctl->iter == 0;  // no Ap yet
-    const unsigned rows = 2u * (unsigned)g.ny * (unsigned)g.nz;
-    const int lane = (int)(threadIdx.x & 31u);
+    const unsigned n2 = o.g.plane * (unsigned)o.g.nz / 2u;
     DwAcc v[3] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
-    for (unsigned R = blockIdx.x * (NT / 32) + (threadIdx.x >> 5); R < rows; R += gridDim.x * (NT / 32))
-        row_z<kRowZ>(
-            o, dgw, z, R, lane,
-            [&](unsigned k) { return DotItem{r[k], first ? make_float2(0.0f, 0.0f) : Ap[k]}; },
-            [&](unsigned k, const DotItem& m, const CellZ<float, float2>& a) {
-                const float2 az = az_dw(a);
-                w[k] = az;
-                dots_dw(v, m, a.zc, az);
-            });
+    for (unsigned q = blockIdx.x * NT + threadIdx.x; q < n2; q += gridDim.x * NT) {
+        PairZ<float, float2> a;
+        if (!load_pair(o, dgw, z, q, a)) continue;
+        const float4 rv = load_two(r, a.k), av = first ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : load_two(Ap, a.k);
+        dots_dw(v, a, rv, av, w);
+    }
     pdl_trigger();
     if (publish_acc<3>(v, part, maxb, blockIdx.x, &ctl->ticket[SL_APPLY], gridDim.x)) {
         double t[3];
@@ -341,7 +335,8 @@ void launch_residual_x(cudaStream_t st, const OpView& o, unsigned n, const doubl
 void launch_az_dw(cudaStream_t st, const OpView& o, const float2* dgw, const float* z, const float2* r,
                   const float2* Ap, float2* w, Ctl* ctl, const Red& red, Cond cond) {
     static const int wb = wave_blocks(k_az_dw, 1 << 30);
-    launch_pdl(k_az_dw, std::min(red.maxb, wb), NT, 0, st, o, dgw, z, r, Ap, w, ctl, red.part, red.maxb, cond);
+    const int want = (int)blocks_of(o.g.plane * (size_t)o.g.nz / 2);
+    launch_pdl(k_az_dw, std::min(std::min(red.maxb, wb), want), NT, 0, st, o, dgw, z, r, Ap, w, ctl, red.part, red.maxb, cond);
 }
 
 void launch_step_dw(cudaStream_t st, unsigned n, const float* z, const float2* w, float2* p, float2* Ap, float2* x,

@@ -32,10 +32,14 @@ using namespace f64dev;
 namespace {
 
 constexpr int kRowU = 2;  // cells a lane and step of the rows of A p
-constexpr int kRowZ = 1;  // and of A z
 
 // w = (A + C/dt) z, r.z, z.Ap (the Ap of the iteration before), z.w; then beta,
-// p.Ap and alpha. One warp per row of one colour and plane, two cells a lane.
+// p.Ap and alpha. One warp per row of one colour and plane, a cell a lane; with
+// the FP64 V-cycle, whose sums leave the integer pipe free, a thread takes two
+// neighbouring slots with loads of two values (400 x 400 x 10: 42.7 us a launch
+// against 53; the float form is no faster in pairs at 800 x 800 and 1 % of an
+// iteration slower at 64 x 64 and 237 x 181, where half the threads wait twice as
+// long).
 //
 // The operator acts on z, not on p: the V-cycle's z is a float, so its products
 // with the float faces are exact in two floats and their sum runs on the FP32
@@ -50,28 +54,38 @@ constexpr int kRowZ = 1;  // and of A z
 // 98), against 107 + 37 for A p and the dots; the FP64 pipe is 60 % busy, memory
 // 44 %, issue 57 %, each warp going from one to the other.
 template <class T, bool FLEX>
-__global__ void __launch_bounds__(NT, 4)
+__global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 3 : 4)
     k_az64(OpView o, const double* __restrict__ diag, const T* __restrict__ z, const double* __restrict__ r,
            const double* __restrict__ Ap, double* __restrict__ w, Ctl* ctl, double* part, int maxb, Cond cond) {
     pdl_enter();
     if (loop_done(ctl, cond)) return;
     const bool first = ctl->iter == 0;  // no Ap yet
-    const unsigned rows = 2u * (unsigned)o.g.ny * (unsigned)o.g.nz;
-    const int lane = (int)(threadIdx.x & 31u);
     double v[3] = {0.0, 0.0, 0.0};
-    struct More {
-        double r, ap;
-    };
-    for (unsigned R = blockIdx.x * (NT / 32) + (threadIdx.x >> 5); R < rows; R += gridDim.x * (NT / 32))
-        row_z<kRowZ>(
-            o, diag, z, R, lane, [&](unsigned k) { return More{r[k], first ? 0.0 : Ap[k]}; },
-            [&](unsigned k, const More& m, const CellZ<T, double>& a) {
-                const double az = az64(a), zc = to_d(a.zc);
-                w[k] = az;
-                v[0] = __fma_rn(m.r, zc, v[0]);
-                v[1] = __fma_rn(zc, m.ap, v[1]);
-                v[2] = __fma_rn(zc, az, v[2]);
-            });
+    if constexpr (sizeof(T) == 8) {
+        const unsigned n2 = o.g.plane * (unsigned)o.g.nz / 2u;
+        for (unsigned q = blockIdx.x * NT + threadIdx.x; q < n2; q += gridDim.x * NT) {
+            PairZ<T, double> a;
+            if (!load_pair(o, diag, z, q, a)) continue;
+            const double2 rv = load_two(r, a.k), av = first ? make_double2(0.0, 0.0) : load_two(Ap, a.k);
+            dots64(v, a, rv, av, w);
+        }
+    } else {
+        const unsigned rows = 2u * (unsigned)o.g.ny * (unsigned)o.g.nz;
+        const int lane = (int)(threadIdx.x & 31u);
+        struct More {
+            double r, ap;
+        };
+        for (unsigned R = blockIdx.x * (NT / 32) + (threadIdx.x >> 5); R < rows; R += gridDim.x * (NT / 32))
+            row_z(
+                o, diag, z, R, lane, [&](unsigned k) { return More{r[k], first ? 0.0 : Ap[k]}; },
+                [&](unsigned k, const More& m, const CellZ<T, double>& a) {
+                    const double az = az64(a), zc = to_d(a.zc);
+                    w[k] = az;
+                    v[0] = __fma_rn(m.r, zc, v[0]);
+                    v[1] = __fma_rn(zc, m.ap, v[1]);
+                    v[2] = __fma_rn(zc, az, v[2]);
+                });
+    }
     pdl_trigger();
     if (publish_sums<3>(v, part, maxb, blockIdx.x, &ctl->ticket[SL_APPLY], gridDim.x)) {
         double t[3];
@@ -401,7 +415,9 @@ void launch_apply64(cudaStream_t st, const OpView& o, const double* diag, const 
 
 void launch_az64(cudaStream_t st, MgType mt, bool flexible, const OpView& o, const double* diag, const void* z,
                  const double* r, const double* Ap, double* w, Ctl* ctl, const Red& red, Cond cond) {
-    const int rows = 2 * o.g.ny * o.g.nz, want = std::max(1, (rows + NT / 32 - 1) / (NT / 32));
+    const int rows = 2 * o.g.ny * o.g.nz;
+    const int want = mt == MG_F64 ? (int)((o.g.plane * (unsigned)o.g.nz / 2u + NT - 1) / NT)
+                                  : std::max(1, (rows + NT / 32 - 1) / (NT / 32));
     auto go = [&](auto kern, int wb, auto* zt) {
         launch_pdl(kern, std::min(std::min(red.maxb, wb), want), NT, 0, st, o, diag, zt, r, Ap, w, ctl, red.part,
                    red.maxb, cond);

@@ -91,11 +91,10 @@ __device__ __forceinline__ void load_z(const OpView& o, const D* __restrict__ di
     }
 }
 
-// Row R = l * 2 ny + 2 j + colour: the calling warp strides over its slots, U
-// cells a lane and step; load(slot) brings whatever else f needs, with the
-// operands, and f(slot, that, operands) follows for each cell in order. Padding
-// slots are left alone.
-template <int U, class T, class D, class Load, class F>
+// Row R = l * 2 ny + 2 j + colour: the calling warp strides over its slots, a cell
+// a lane; load(slot) brings whatever else f needs, with the operands, and f(slot,
+// that, operands) follows. Padding slots are left alone.
+template <class T, class D, class Load, class F>
 __device__ __forceinline__ void row_z(const OpView& o, const D* __restrict__ diag, const T* __restrict__ z, unsigned R,
                                       int lane, Load&& load, F&& f) {
     const Geo& g = o.g;
@@ -108,25 +107,120 @@ __device__ __forceinline__ void row_z(const OpView& o, const D* __restrict__ dia
     const unsigned row = base + r * hx;
     const unsigned orow = base + (unsigned)(2 * j + (c ^ 1)) * hx;  // other colour, same j
     const bool hs = j > 0, hn = j < g.ny - 1, hd = l > 0, hu = (int)l < g.nz - 1;
-    for (unsigned t0 = (unsigned)lane; t0 < hx; t0 += 32u * U) {
-        CellZ<T, D> a[U];
-        decltype(load(0u)) more[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const unsigned t = t0 + 32u * u;
-            const int i = 2 * (int)t + e;
-            if (t < hx && i < g.nx) {
-                load_z(o, diag, z, row + t, t, orow, i, e, hs, hn, hd, hu, a[u]);
-                more[u] = load(row + t);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const unsigned t = t0 + 32u * u;
-            const int i = 2 * (int)t + e;
-            if (t < hx && i < g.nx) f(row + t, more[u], a[u]);
-        }
+    for (unsigned t = (unsigned)lane; t < hx; t += 32u) {
+        const int i = 2 * (int)t + e;
+        if (i >= g.nx) continue;
+        CellZ<T, D> a;
+        load_z(o, diag, z, row + t, t, orow, i, e, hs, hn, hd, hu, a);
+        const auto more = load(row + t);
+        f(row + t, more, a);
     }
+}
+
+template <class T>
+struct Two;
+template <>
+struct Two<float> {
+    typedef float2 type;
+};
+template <>
+struct Two<double> {
+    typedef double2 type;
+};
+template <>
+struct Two<float2> {
+    typedef float4 type;
+};
+template <class T>
+__device__ __forceinline__ typename Two<T>::type load_two(const T* __restrict__ v, unsigned k) {
+    return *reinterpret_cast<const typename Two<T>::type*>(v + k);
+}
+__device__ __forceinline__ double first_of(double2 v) { return v.x; }
+__device__ __forceinline__ double second_of(double2 v) { return v.y; }
+__device__ __forceinline__ float2 first_of(float4 v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 second_of(float4 v) { return make_float2(v.z, v.w); }
+
+// Two cells of A z: slots k and k + 1 of one colour of one row (k even: hx is a
+// multiple of 4), pair p of all planes in slot order, with loads of two values
+// where the neighbours lie side by side; of the other colour's row the pair needs
+// a third value to the west (even rows of the colour) or the east. second: slot
+// k + 1 holds a cell (not padding).
+template <class T, class D>
+struct PairZ {
+    CellZ<T, D> c[2];
+    unsigned k;
+    bool second;
+};
+// False where both slots are padding.
+template <class T, class D>
+__device__ __forceinline__ bool load_pair(const OpView& o, const D* __restrict__ diag, const T* __restrict__ z,
+                                          unsigned p, PairZ<T, D>& a) {
+    typedef typename Two<T>::type T2;
+    const Geo& g = o.g;
+    const unsigned hx = (unsigned)g.hx;
+    const unsigned F = p / hx, q = 2u * (p - F * hx);  // row of both colours, slot in it
+    const unsigned l = F / (unsigned)g.ny;
+    const int j = (int)(F - l * (unsigned)g.ny);
+    const int c = q >= hx ? 1 : 0, e = (j + c) & 1;
+    const unsigned t = q - (c ? hx : 0u), k = 2u * p;
+    const unsigned ok = c ? k - hx : k + hx;  // the other colour's slot t
+    const int i0 = 2 * (int)t + e, i1 = i0 + 2;
+    if (i0 >= g.nx) return false;
+    a.k = k;
+    a.second = i1 < g.nx;
+    const T2 zc = load_two(z, k), zo = load_two(z, ok);
+    const float2 go = load_two(o.gE, ok), ge = load_two(o.gE, k);
+    const auto dg = load_two(diag, k);
+    T zx = T(0);  // the third value of the other colour's row
+    float gx = 0.0f;
+    if (e == 0) {
+        if (t > 0) {
+            zx = z[ok - 1u];
+            gx = o.gE[ok - 1u];
+        }
+    } else if (t + 2u < hx) {
+        zx = z[ok + 2u];
+    }
+    T2 v[4];
+    float2 f[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        v[s].x = v[s].y = T(0);
+        f[s] = make_float2(0.0f, 0.0f);
+    }
+    if (j > 0) {
+        v[0] = load_two(z, ok - 2u * hx);
+        f[0] = load_two(o.gN, ok - 2u * hx);
+    }
+    if (j < g.ny - 1) {
+        v[1] = load_two(z, ok + 2u * hx);
+        f[1] = load_two(o.gN, k);
+    }
+    if (l > 0) {
+        v[2] = load_two(z, k - g.plane);
+        f[2] = load_two(o.gU, k - g.plane);
+    }
+    if ((int)l < g.nz - 1) {
+        v[3] = load_two(z, k + g.plane);
+        f[3] = load_two(o.gU, k);
+    }
+    CellZ<T, D>&u = a.c[0], &w = a.c[1];
+    u.zc = zc.x, w.zc = zc.y;
+    u.dg = first_of(dg), w.dg = second_of(dg);
+    u.z[0] = e ? zo.x : zx;
+    u.g[0] = e ? go.x : gx;
+    u.z[1] = e ? zo.y : zo.x;
+    u.g[1] = i0 < g.nx - 1 ? ge.x : 0.0f;
+    w.z[0] = e ? zo.y : zo.x;
+    w.g[0] = e ? go.y : go.x;
+    w.z[1] = e ? zx : zo.y;
+    w.g[1] = i1 < g.nx - 1 ? ge.y : 0.0f;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        u.z[2 + s] = v[s].x, w.z[2 + s] = v[s].y;
+        u.g[2 + s] = f[s].x, w.g[2 + s] = f[s].y;
+    }
+    return true;
 }
 
 // beta, p.Ap and alpha of the iteration that the V-cycle's z begins, from r.z,

@@ -64,3 +64,29 @@ def test_layered_field_equals_fp64(ct, batch):
             s.solve(1e-13, 300)
             out.append(s.get_x(0) if batch and out else s.get_x())
     assert np.abs(out[1] - out[0]).max() <= 2e-13 * np.abs(out[0]).max()
+
+
+# A z in pairs of slots (FP64 V-cycle, double words) against the float form's cell
+# a lane: one column to rows of a few slots, odd and even widths and heights of
+# either parity, the third neighbour at both ends. Solved to 1e-12 the fields agree
+# to rounding (1e-16 times the 1e3 of diagonal over row sum), ten times over for
+# the iterations' sums.
+@pytest.mark.parametrize("nx,ny", [(1, 1), (2, 3), (3, 2), (7, 5), (8, 4), (9, 6), (15, 16), (16, 15), (17, 18), (66, 33)])
+def test_pairs_equal_cells(ct, nx, ny):
+    m = tsv_stack(ct, nx, ny)
+    out = []
+    for prec in ("MG_FP32_FLEX", "MG_FP64", "MG_FP32_FLEX_DW", "batch"):
+        if prec == "batch":
+            with ct.GpuBatch([m], precision=ct.Precision.MG_FP32_FLEX_DW) as b:
+                b.set_x_zero()
+                b.set_rhs_steady()
+                b.solve(1e-12, 200)
+                out.append(b.get_x(0))
+            continue
+        with ct.GpuPcg(m, ct.Precond.Multigrid, getattr(ct.Precision, prec)) as s:
+            s.set_x_zero()
+            s.set_rhs_steady()
+            s.solve(1e-12, 200)
+            out.append(s.get_x())
+    for T in out[1:]:
+        assert np.abs(T - out[0]).max() <= 1e-12 * np.abs(out[0]).max()
