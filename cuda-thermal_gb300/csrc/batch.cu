@@ -671,7 +671,7 @@ void Batch::vcycle(Bucket& b, cudaStream_t s, Cond cond) {
             [&] { sweep(b, s, d, 0, true, false, cond); });
         enq(s, "b_sweep" + lvl, N * 20,
             [&] { sweep(b, s, d, 1, false, false, cond); });
-        enq(s, "b_restrict" + lvl, N * 25, [&] { launch_b_restrict(s, b.restr[(size_t)d], L, C, ctl); });
+        enq(s, "b_restrict" + lvl, N * 11, [&] { launch_b_restrict(s, b.restr[(size_t)d], L, C, ctl); });
     }
     double smb = 0;
     for (int i : b.inst) {

@@ -87,15 +87,12 @@ struct Cond {
 };
 
 // One multigrid level as the kernels see it (split layout). T = float or
-// double: the V-cycle precision. Faces and capacities are always float. dg is
-// the cell's diagonal (faces + C/dt) as the residual of the restriction
-// rounds it, made with the column factors by set_dt.
+// double: the V-cycle precision. Faces and capacities are always float.
 template <class T>
 struct LevelView {
     Geo g;
     const float *gE, *gN, *gU, *gB, *cap;
     T *fcp, *finv;
-    T* dg;
     T *x, *b;
 };
 

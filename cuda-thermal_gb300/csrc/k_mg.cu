@@ -215,16 +215,8 @@ __global__ void __launch_bounds__(32 * MZ)
     if (on) L.x[(unsigned)l * g.plane + s] = sv[l][tx];
 }
 
-// Restriction F -> C, one thread per coarse cell and plane (blockIdx.y is
-// the plane; k_restrict), or per coarse cell and pair of consecutive planes
-// (k_restrict2: both sums before either store, so the planes' shared
-// operands, a child's x one plane up being the next plane's own, are loaded
-// once). Pairs pay on large fine levels (800 x 800: 46 us against 49 us),
-// single planes on small ones (25 x 25: 8.8 us against 10.5 us, twice the
-// threads for a latency-bound launch). k_restrict2 is compiled for 4 blocks
-// per SM (64 registers): 38.8 us at 800 x 800, against 39.5 us with 80
-// registers and 46.8 / 53.7 us with 48 / 40; the load round trips of a
-// thread, not the number of resident warps, bound it.
+// Restriction F -> C, one thread per coarse cell and plane (blockIdx.y is the
+// plane).
 template <class T>
 __global__ void __launch_bounds__(NT)
     k_restrict(LevelView<T> F, LevelView<T> C, const Ctl* ctl, Cond cond) {
@@ -239,17 +231,6 @@ __global__ void __launch_bounds__(NT)
     if (loop_done(flags, cond) || !on) return;
     pdl_trigger();
     C.b[(unsigned)l * cg.plane + scol(cg, I, J)] = sum;
-}
-
-template <class T>
-__global__ void __launch_bounds__(NT, 4)
-    k_restrict2(LevelView<T> F, LevelView<T> C, const Ctl* ctl, Cond cond) {
-    pdl_enter();
-    if (loop_done(ctl, cond)) return;
-    pdl_trigger();  // several waves: the dependent launches as the last one starts
-    const unsigned q = blockIdx.x * NT + threadIdx.x;
-    if (q >= (unsigned)C.g.nx * (unsigned)C.g.ny) return;
-    restrict_pair<T, false>(F, C, q, 2 * (int)blockIdx.y);
 }
 
 // Restriction F -> C fused with C's first sweep (x = 0, red columns). A
@@ -419,13 +400,8 @@ void launch_sweep(cudaStream_t st, const LevelView<T>& L, int color, bool zero_x
 template <class T>
 void launch_restrict(cudaStream_t st, const LevelView<T>& F, const LevelView<T>& C, const Ctl* ctl,
                      Cond cond) {
-    if ((unsigned)F.g.nx * (unsigned)F.g.ny > kSweepBfColumns) {
-        const dim3 grid(blocks_for((unsigned)C.g.nx * C.g.ny), (unsigned)(C.g.nz + 1) / 2);
-        launch_pdl(k_restrict2<T>, grid, NT, 0, st, F, C, ctl, cond);
-    } else {
-        const dim3 grid(blocks_for((unsigned)C.g.nx * C.g.ny), (unsigned)C.g.nz);
-        launch_pdl(k_restrict<T>, grid, NT, 0, st, F, C, ctl, cond);
-    }
+    const dim3 grid(blocks_for((unsigned)C.g.nx * C.g.ny), (unsigned)C.g.nz);
+    launch_pdl(k_restrict<T>, grid, NT, 0, st, F, C, ctl, cond);
 }
 
 template <class T>

@@ -14,8 +14,8 @@
 // cluster (`nd` distributed levels, coarse row J with the fine rows 2J and
 // 2J + 1); the levels below (at most kTailBottomCells) are one CTA's, which takes
 // no rows of the others where the cluster has a CTA to spare. A CTA keeps its
-// rows of b, x, 1/pivot, gU, gE, gN and the diagonal, brought in by one tensor
-// copy an array, with a halo row of x on each side and one of gN to the south. A
+// rows of b, x, 1/pivot, gU, gE and gN, brought in by one tensor copy an array,
+// with a halo row of x on each side and one of gN to the south. A
 // sweep sends its boundary rows straight into the neighbours' halos (st.async,
 // counted by an mbarrier of the receiver that only this sweep uses), so
 // neighbours wait for each other's data and nothing else: 0.2 us, against 0.5
@@ -221,9 +221,9 @@ __device__ __forceinline__ void tail_recur(const Cta& c, const TailLevel& L, int
     }
 }
 
-// Restriction of level k: one task per coarse cell and plane, the sum of its
-// (up to four) children's residuals, j then i, consecutive cells on consecutive
-// lanes. far: the coarse b lies in another CTA's shared memory (at `far`,
+// Restriction of level k (mgdev::restrict_sum: the faces times the black
+// neighbours' x at the two red children): one task per coarse cell and plane,
+// consecutive cells on consecutive lanes. far: the coarse b lies in another CTA's shared memory (at `far`,
 // counted by far_bar), by global rows.
 __device__ __forceinline__ void tail_restrict(const Cta& c, const TailLevel& L, const TailLevel& C, int j0,
                                               unsigned far, unsigned far_bar) {
@@ -233,38 +233,28 @@ __device__ __forceinline__ void tail_restrict(const Cta& c, const TailLevel& L, 
     const int* const tab = tail_ints() + L.tcell;
     for (int l = c.warp; l < nz; l += c.warps) {
         const int lp = l * pl, lx = L.x + l * xpl + RS, le = L.ge + lp, ln = L.gn + lp + (l + 1) * gnh;
-        const int lu = L.gu + lp, ld = L.dg + lp, lb = L.b + lp;
-        const bool dn = l > 0, up = l < nz - 1;
-        const int od = dn ? xpl : 0, ou = up ? xpl : 0, pd = dn ? pl : 0;
 #pragma unroll 1
         for (int q0 = c.lane; q0 < ncell + c.lane; q0 += 32) {
             const int q = min(q0, ncell - 1), w = tab[2 * q], at = tab[2 * q + 1], rl = entry_row(w);
             const bool hi = entry_bit(w, 0), hw = entry_bit(w, 1), hj = 2 * (J0 + rl) + 1 < L.ny;
             // the children's slots: (2I, 2J) red, (2I + 1, 2J) black, and a row up;
-            // a child row past the level's reads the row below (not used)
+            // a child row past the level's reads the row below (weight zero)
             const int c00 = entry_own(w), c10 = c00 + hx, R1 = 2 * rl + 1 < rows ? RS : 0;
             const int c01 = c10 + R1, c11 = c00 + R1;
-            const float x00 = sm[lx + c00], x10 = sm[lx + c10], x01 = sm[lx + c01], x11 = sm[lx + c11];
-            const float gE00 = sm[le + c00], gN00 = sm[ln + c00], gE01 = sm[le + c01], gN10 = sm[ln + c10];
-            auto res = [&](int p, float xc, float gw, float xw, float xe, float gs, float xs, float xn) {
-                const float gup = sm[lu + p], gdn = sm[lu + p - pd];
-                float off = __fmaf_rn(gw, xw, 0.0f);
-                off = __fmaf_rn(sm[le + p], xe, off);
-                off = __fmaf_rn(gs, xs, off);
-                off = __fmaf_rn(sm[ln + p], xn, off);
-                off = __fmaf_rn(dn ? gdn : 0.0f, sm[lx + p - od], off);
-                off = __fmaf_rn(up ? gup : 0.0f, sm[lx + p + ou], off);
-                return __fsub_rn(sm[lb + p], __fmaf_rn(sm[ld + p], xc, -off));
-            };
-            const bool hs = gnh || rl > 0;
-            const float gw0 = sm[le + c10 - 1], gw1 = sm[le + c11 - 1], gs0 = sm[ln + c10 - RS], gs1 = sm[ln + c00 - RS];
-            float v = res(c00, x00, hw ? gw0 : 0.0f, sm[lx + c10 - 1], x10, hs ? gs0 : 0.0f, sm[lx + c10 - RS], x01);
-            const float r10 = res(c10, x10, gE00, x00, sm[lx + c00 + 1], hs ? gs1 : 0.0f, sm[lx + c00 - RS], x11);
-            const float r01 = res(c01, x01, hw ? gw1 : 0.0f, sm[lx + c11 - 1], x11, gN00, x00, sm[lx + c11 + RS]);
-            const float r11 = res(c11, x11, gE01, x01, sm[lx + c01 + 1], gN10, x10, sm[lx + c01 + RS]);
-            v = hi ? __fadd_rn(v, r10) : v;
-            v = hj ? __fadd_rn(v, r01) : v;
-            v = hi && hj ? __fadd_rn(v, r11) : v;
+            const bool hs = gnh || rl > 0, both = hi && hj;
+            const float x10 = sm[lx + c10], x01 = sm[lx + c01], xw = sm[lx + c10 - 1], xs = sm[lx + c10 - RS];
+            const float xe = sm[lx + c01 + 1], xn = sm[lx + c10 + 2 * R1];
+            const float gw = sm[le + c10 - 1], ge = sm[le + c00], gs = sm[ln + c10 - RS], gn = sm[ln + c00];
+            const float gw1 = sm[le + c01], ge1 = sm[le + c11], gs1 = sm[ln + c10], gn1 = sm[ln + c11];
+            float v = __fmaf_rn(hw ? gw : 0.0f, xw, 0.0f);
+            v = __fmaf_rn(hi ? ge : 0.0f, x10, v);
+            v = __fmaf_rn(hs ? gs : 0.0f, xs, v);
+            v = __fmaf_rn(hj ? gn : 0.0f, x01, v);
+            float u = __fmaf_rn(both ? gw1 : 0.0f, x01, 0.0f);
+            u = __fmaf_rn(both ? ge1 : 0.0f, xe, u);
+            u = __fmaf_rn(both ? gs1 : 0.0f, x10, u);
+            u = __fmaf_rn(both ? gn1 : 0.0f, xn, u);
+            v = __fadd_rn(v, u);
             if (q0 == q && J0 + rl < C.ny) {
                 const int b = C.b + l * cpl + at;
                 if (far)
@@ -309,7 +299,7 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
         halo.north = remote(base, (unsigned)rank + 1u);
         halo.north_bar = remote(bar_base, (unsigned)rank + 1u);
     }
-    // The operator, factors and diagonal do not change during a solve: their
+    // The operator and factors do not change during a solve: their
     // copies are issued before the wait for the preceding kernel, those of the
     // first sweep on a barrier of their own; a level split by rows by tensor
     // copies (rows outside it come as zeros), a whole one by plain ones.
@@ -322,10 +312,10 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
     }
     __syncwarp();
     if (lane == 0)
-        for (int a = warp; a < 5 * (k_hi - k_lo); a += warps) {
-            const int kk = a / 5, arr = a - 5 * kk, k = k_lo + kk;
+        for (int a = warp; a < 4 * (k_hi - k_lo); a += warps) {
+            const int kk = a >> 2, arr = a & 3, k = k_lo + kk;
             const TailLevel& L = P.L[k];
-            const int dst = arr == 0 ? L.fi : arr == 1 ? L.gu : arr == 2 ? L.ge : arr == 3 ? L.gn : L.dg;
+            const int dst = arr == 0 ? L.fi : arr == 1 ? L.gu : arr == 2 ? L.ge : L.gn;
             uint64_t* const bar = arr < 2 && k == k_lo ? bar0 : bar1;
             const int j0 = rank * L.rows;
             if (k < nd)
@@ -357,7 +347,7 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
     const bool first = k_lo == 0 && k_hi > 0;  // holds rows of the first level
     if (tid == 0 && first) {
         tma::mbar_arrive_expect_tx(barb, (unsigned)(P.L[0].rows * 2 * P.L[0].hx * nz) * 4u);
-        tma::load_3d(sm + P.L[0].b, &maps[0].m[5], 0, nd > 0 ? rank * P.L[0].rows : 0, 0, barb);
+        tma::load_3d(sm + P.L[0].b, &maps[0].m[4], 0, nd > 0 ? rank * P.L[0].rows : 0, 0, barb);
     }
     const bool closed = loop_done(ctl, cond);  // the same in every thread of the cluster
     bool ok = tma::mbar_wait(bar0, 0u);        // (the level descriptors come with the tables)
@@ -544,12 +534,11 @@ bool plan_tail(const LevelView<float>* views, int n, int ctas, bool apart, size_
         L.ge = take(w, pl);
         L.gnh = k < nd ? 2 * L.hx : 0;  // (a whole level has no row to its south)
         L.gn = take(w, pl + (size_t)L.gnh * nz);
-        L.dg = take(w, pl);
     }
     for (int k = 0; k < n; ++k) {
         const TailLevel& L = p.L[k];
         const unsigned one = (unsigned)(L.rows * 2 * L.hx * nz) * 4u;
-        (k < nd ? p.dist_bytes : p.bottom_bytes) += 5 * one + (unsigned)(L.gnh * nz) * 4u;
+        (k < nd ? p.dist_bytes : p.bottom_bytes) += 4 * one + (unsigned)(L.gnh * nz) * 4u;
         if (k == 0) p.first_bytes = 2 * one;
         if (k == nd) p.bottom_first_bytes = 2 * one;
     }
@@ -603,11 +592,11 @@ bool make_tail_maps(const TailPlan& p, const LevelView<float>* views, TailMaps* 
     for (int k = 0; k < p.n; ++k) {
         const LevelView<float>& v = views[k];
         const unsigned RS = 2u * (unsigned)v.g.hx, rows = (unsigned)p.L[k].rows, nz = (unsigned)p.nz;
-        const float* src[6] = {v.finv, v.gU, v.gE, v.gN, v.dg, v.b};
+        const float* src[5] = {v.finv, v.gU, v.gE, v.gN, v.b};
         std::memset(&maps[k], 0, sizeof maps[k]);
-        for (int a = 0; a < 5; ++a) maps[k].whole[a] = src[a];
+        for (int a = 0; a < 4; ++a) maps[k].whole[a] = src[a];
         if (k >= p.nd && k > 0) continue;  // (the first level's b is always a tensor copy)
-        for (int a = 0; a < 6; ++a)
+        for (int a = 0; a < 5; ++a)
             if (!encode_tail_map(&maps[k].m[a], src[a], v.g, RS, a == 3 ? rows + 1u : rows, nz)) return false;
     }
     return true;

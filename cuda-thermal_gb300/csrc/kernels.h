@@ -199,9 +199,6 @@ void launch_factor(cudaStream_t st, const LevelView<T>& L, T inv_dt);
 // V-cycle), so lateral neighbours are not read. xc: when not null, the
 // coarser level's x is added to every neighbour value read (prolongation
 // fused into the sweep).
-// Fine levels of more than this many columns restrict by pairs of planes
-// (k_restrict2), smaller ones by single planes (k_restrict).
-constexpr unsigned kSweepBfColumns = 128u * 128u;
 // Levels of at most this many columns sweep with one thread per column and
 // plane (k_sweep_split); larger FP32 levels are staged by bulk tensor copies
 // (at 800 x 800: the 200 x 200 level split 6.96 ms per solve against 7.07 ms
@@ -274,14 +271,13 @@ struct TailLevels {
 constexpr int kSmallThreads = 512;        // the bottom kernel's launch bound (and the batch's blocks)
 constexpr int kSmallThreadsSolver = 256;  // the single solver's bottom block
 constexpr int kSmallSmemMax = 200 * 1024;
-// Bytes one level takes there: gE, gN, gU (float), dg, fcp, finv, x, b (elem
-// bytes each), every array rounded up to 16
-// bytes. The device carving of the block's shared memory, its size at launch
+// Bytes one level takes there: gE, gN, gU (float), fcp, finv, x, b (elem bytes
+// each), every array rounded up to 16 bytes. The device carving of the block's shared memory, its size at launch
 // and the choice of the first level held there all use this one sum.
 __host__ __device__ inline size_t small_round16(size_t b) { return (b + 15) & ~size_t(15); }
 __host__ __device__ inline size_t small_level_bytes(const Geo& g, size_t elem) {
     const size_t ln = (size_t)g.plane * (size_t)g.nz;
-    return 3 * small_round16(ln * 4) + 5 * small_round16(ln * elem);
+    return 3 * small_round16(ln * 4) + 4 * small_round16(ln * elem);
 }
 // The coarse end of the single solver's FP32 V-cycle in one cluster launch
 // (k_tail.cu): `n` levels, finest first; the first nd are split by rows over
@@ -297,12 +293,12 @@ constexpr int kTailCtas = 16;            // CTAs of the cluster, at most
 // 1024 x 16 964.6 us, 967 at 1000 and 975 at 4096 (its 16 x 16 level on one CTA).
 constexpr int kTailBottomCells = 2560;
 struct TailLevel {
-    int x, b, fi, gu, ge, gn, dg;  // the level's arrays
+    int x, b, fi, gu, ge, gn;      // the level's arrays
     int tcol, tpar, tcell;         // its tables: columns, black columns' parents, coarse cells
     int hx, rows, nx, ny;
     int ncol, ncell;  // slots of one colour, coarse cells of the rows
     int gnh;          // floats of gN's halo row (0: none)
-    int pad;
+    int pad[2];
 };
 constexpr int kTailDescriptors = 32;  // where the descriptors lie (a west neighbour of the first slot stays inside)
 struct TailPlan {
@@ -317,12 +313,12 @@ struct TailPlan {
     unsigned plane;        // its plane stride
     TailLevel L[kTailLevels];
 };
-// One level's arrays: 1/pivot, gU, gE, gN, diagonal, b. A distributed level's as
+// One level's arrays: 1/pivot, gU, gE, gN, b. A distributed level's as
 // tensor maps, whole rows (both colours) of all planes (gN with one row more);
 // the others' as they lie.
 struct TailMaps {
-    CUtensorMap m[6];
-    const float* whole[16];  // (five, padded to the maps' alignment)
+    CUtensorMap m[5];
+    const float* whole[16];  // (four, padded to the maps' alignment)
 };
 // Lays out levels views[0 .. n) for a cluster of at most `ctas` CTAs, the bottom
 // levels on a CTA of their own (apart) or with the first rows; false if they do

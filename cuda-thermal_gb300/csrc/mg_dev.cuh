@@ -241,119 +241,49 @@ __device__ __forceinline__ void sweep_column(const LevelView<T>& L, const LevelV
     }
 }
 
-// b - (A + C/dt) x of a cell on operands already loaded, in op_apply's order
-// (src/operator3d.h:108-112): its diagonal dg times x minus the neighbour terms
-// (west, east, south, north, down, up). dg is the diagonal this sum would
-// form (faces west to down, then C/dt fused), stored by set_dt: seven
-// additions, six of them on the FP64 pipe's critical path in FP64, and two
-// operands (C and the bottom face) fewer per cell than forming it here.
-template <class T>
-__device__ __forceinline__ T residual_of(T b, T dg, T xc, T xw, T xe, T xs, T xn, T xd, T xu, float gew, float gee,
-                                         float gns, float gnn, float gu, float gd, bool w, bool e, bool so, bool no,
-                                         bool down, bool up) {
-    T off = 0;
-    if (w) off += face<T>(gew) * xw;
-    if (e) off += face<T>(gee) * xe;
-    if (so) off += face<T>(gns) * xs;
-    if (no) off += face<T>(gnn) * xn;
-    if (down) off += face<T>(gd) * xd;
-    if (up) off += face<T>(gu) * xu;
-    return b - (dg * xc - off);
-}
-
-// The same at fine cell (i, j, l); an absent neighbour reads the cell itself.
-template <class T, bool CG>
-__device__ __forceinline__ T residual_at(const LevelView<T>& F, int i, int j, int l) {
-    const Geo& fg = F.g;
-    const Nbr n = neighbours<false>(fg, fg, i, j, i >> 1, (i + j) & 1);
-    const unsigned base = (unsigned)l * fg.plane, id = base + n.s;
-    const bool down = l > 0, up = l < fg.nz - 1;
-    const unsigned sw = n.w ? base + n.sw : id, se = n.e ? base + n.se : id;
-    const unsigned ss = n.so ? base + n.ss : id, sn = n.no ? base + n.sn : id;
-    const unsigned sd = down ? id - fg.plane : id, su = up ? id + fg.plane : id;
-    return residual_of<T>(ldm<CG>(F.b + id), F.dg[id], ldm<CG>(F.x + id), ldm<CG>(F.x + sw), ldm<CG>(F.x + se),
-                          ldm<CG>(F.x + ss), ldm<CG>(F.x + sn), ldm<CG>(F.x + sd), ldm<CG>(F.x + su), F.gE[sw],
-                          F.gE[id], F.gN[ss], F.gN[id], F.gU[id], F.gU[sd], n.w, n.e, n.so, n.no, down, up);
-}
-
-// The four children of an interior coarse cell at once: their x, faces and
-// the eight outside neighbours are loaded once each (48 values instead of
-// four residual_at's 60, with the index arithmetic shared), and each child's
-// residual is residual_at's, operation for operation.
-template <class T, bool CG>
-__device__ __forceinline__ T restrict_sum4(const LevelView<T>& F, int I, int J, int l) {
-    const Geo& g = F.g;
-    const int i0 = 2 * I, j0 = 2 * J;
-    const bool w = i0 > 0, e = i0 + 2 < g.nx, so = j0 > 0, no = j0 + 2 < g.ny;
-    const bool down = l > 0, up = l < g.nz - 1;
-    const unsigned base = (unsigned)l * g.plane;
-    const unsigned c00 = base + scol(g, i0, j0), c10 = base + scol(g, i0 + 1, j0);
-    const unsigned c01 = base + scol(g, i0, j0 + 1), c11 = base + scol(g, i0 + 1, j0 + 1);
-    // outside neighbours (an absent one reads the child beside it; unused)
-    const unsigned w0 = w ? base + scol(g, i0 - 1, j0) : c00, w1 = w ? base + scol(g, i0 - 1, j0 + 1) : c01;
-    const unsigned e0 = e ? base + scol(g, i0 + 2, j0) : c10, e1 = e ? base + scol(g, i0 + 2, j0 + 1) : c11;
-    const unsigned s0 = so ? base + scol(g, i0, j0 - 1) : c00, s1 = so ? base + scol(g, i0 + 1, j0 - 1) : c10;
-    const unsigned n0 = no ? base + scol(g, i0, j0 + 2) : c01, n1 = no ? base + scol(g, i0 + 1, j0 + 2) : c11;
-    const unsigned dn = down ? g.plane : 0u, upo = up ? g.plane : 0u;
-    const T x00 = ldm<CG>(F.x + c00), x10 = ldm<CG>(F.x + c10), x01 = ldm<CG>(F.x + c01), x11 = ldm<CG>(F.x + c11);
-    const T xw0 = ldm<CG>(F.x + w0), xw1 = ldm<CG>(F.x + w1), xe0 = ldm<CG>(F.x + e0), xe1 = ldm<CG>(F.x + e1);
-    const T xs0 = ldm<CG>(F.x + s0), xs1 = ldm<CG>(F.x + s1), xn0 = ldm<CG>(F.x + n0), xn1 = ldm<CG>(F.x + n1);
-    const T d00 = ldm<CG>(F.x + c00 - dn), d10 = ldm<CG>(F.x + c10 - dn);
-    const T d01 = ldm<CG>(F.x + c01 - dn), d11 = ldm<CG>(F.x + c11 - dn);
-    const T u00 = ldm<CG>(F.x + c00 + upo), u10 = ldm<CG>(F.x + c10 + upo);
-    const T u01 = ldm<CG>(F.x + c01 + upo), u11 = ldm<CG>(F.x + c11 + upo);
-    const float gEw0 = F.gE[w0], gE00 = F.gE[c00], gE10 = F.gE[c10];
-    const float gEw1 = F.gE[w1], gE01 = F.gE[c01], gE11 = F.gE[c11];
-    const float gNs0 = F.gN[s0], gN00 = F.gN[c00], gNs1 = F.gN[s1], gN10 = F.gN[c10];
-    const float gN01 = F.gN[c01], gN11 = F.gN[c11];
-    const float gu00 = F.gU[c00], gu10 = F.gU[c10], gu01 = F.gU[c01], gu11 = F.gU[c11];
-    // down face: gU of the plane below (unused at the bottom plane)
-    const float gd00 = F.gU[c00 - dn], gd10 = F.gU[c10 - dn], gd01 = F.gU[c01 - dn], gd11 = F.gU[c11 - dn];
-    T sum = 0;
-    sum += residual_of<T>(ldm<CG>(F.b + c00), F.dg[c00], x00, xw0, x10, xs0, x01, d00, u00, gEw0, gE00, gNs0, gN00, gu00, gd00,
-                          w, true, so, true, down, up);
-    sum += residual_of<T>(ldm<CG>(F.b + c10), F.dg[c10], x10, x00, xe0, xs1, x11, d10, u10, gE00, gE10, gNs1, gN10, gu10, gd10,
-                          true, e, so, true, down, up);
-    sum += residual_of<T>(ldm<CG>(F.b + c01), F.dg[c01], x01, xw1, x11, x00, xn0, d01, u01, gEw1, gE01, gN00, gN01, gu01, gd01,
-                          w, true, true, no, down, up);
-    sum += residual_of<T>(ldm<CG>(F.b + c11), F.dg[c11], x11, x01, xe1, x10, xn1, d11, u11, gE01, gE11, gN10, gN11, gu11, gd11,
-                          true, e, true, no, down, up);
-    return sum;
-}
-
-// Restriction (src/pcg3d_cpu.cpp:87-100) of coarse cell (I, J, l): the sum
-// over the (up to 4) children, j then i, of the fine residual.
+// Restriction (src/pcg3d_cpu.cpp:87-100) of coarse cell (I, J, l): the sum over
+// its (up to 4) children of the fine residual b - (A + C/dt) x, x being the
+// iterate of the V-cycle's way down: the red columns solved from x = 0, then the
+// black ones. A black column was solved with the red x it still has: its residual
+// is zero. A red column was solved with zeros beside it: of its residual the
+// lateral terms of the black x that came since are left. So the residual is the
+// faces times the black neighbours' x at the two red children, (2I, 2J) and
+// (2I + 1, 2J + 1): 10 bytes a fine cell in FP32 where b, x, the diagonal and
+// every face are 24, and no difference of large terms (the vertical ones are up to
+// 1e4 of the lateral).
+// The residual of all four children on all operands took 35.5 us at 800 x 800 x 10
+// (23.0 so) and, in FP64, 47 at 400 x 400 x 10 (13.1); an iteration 382 -> 359 and
+// 388 -> 318.
 template <class T, bool CG>
 __device__ __forceinline__ T restrict_sum(const LevelView<T>& F, int I, int J, int l) {
-    const Geo& fg = F.g;
-    if (2 * I + 1 < fg.nx && 2 * J + 1 < fg.ny) return restrict_sum4<T, CG>(F, I, J, l);
-    const int i1 = min(2 * I + 2, fg.nx), j1 = min(2 * J + 2, fg.ny);
-    T sum = 0;
-    for (int j = 2 * J; j < j1; ++j)
-        for (int i = 2 * I; i < i1; ++i) sum += residual_at<T, CG>(F, i, j, l);
-    return sum;
+    const Geo& g = F.g;
+    const int i0 = 2 * I, j0 = 2 * J;
+    const bool w = i0 > 0, e = i0 + 1 < g.nx, so = j0 > 0, no = j0 + 1 < g.ny;
+    const bool both = e && no, e2 = both && i0 + 2 < g.nx, n2 = both && j0 + 2 < g.ny;
+    const unsigned base = (unsigned)l * g.plane, hx = (unsigned)g.hx;
+    // slots: red (2I, 2J), black (2I + 1, 2J); black (2I, 2J + 1), red (2I + 1, 2J + 1)
+    const unsigned c00 = base + 4u * (unsigned)J * hx + (unsigned)I, c10 = c00 + hx;
+    const unsigned c11 = no ? c00 + 2u * hx : c00, c01 = no ? c10 + 2u * hx : c10;
+    // (an absent neighbour reads a cell beside it, with a zero face)
+    const unsigned a_w = w ? c10 - 1u : c10, a_s = so ? c10 - 2u * hx : c10;
+    const unsigned a_e = e2 ? c01 + 1u : c01, a_n = n2 ? c10 + 4u * hx : c10;
+    const T x10 = ldm<CG>(F.x + c10), x01 = ldm<CG>(F.x + c01);
+    const T xw = ldm<CG>(F.x + a_w), xs = ldm<CG>(F.x + a_s), xe = ldm<CG>(F.x + a_e), xn = ldm<CG>(F.x + a_n);
+    const float gw = F.gE[a_w], ge = F.gE[c00], gs = F.gN[a_s], gn = F.gN[c00];
+    const float hw = F.gE[c01], he = F.gE[c11], hs = F.gN[c10], hn = F.gN[c11];
+    T sum = 0, two = 0;
+    sum += (w ? face<T>(gw) : T(0)) * xw;
+    sum += (e ? face<T>(ge) : T(0)) * x10;
+    sum += (so ? face<T>(gs) : T(0)) * xs;
+    sum += (no ? face<T>(gn) : T(0)) * x01;
+    two += (both ? face<T>(hw) : T(0)) * x01;
+    two += (e2 ? face<T>(he) : T(0)) * xe;
+    two += (both ? face<T>(hs) : T(0)) * x10;
+    two += (n2 ? face<T>(hn) : T(0)) * xn;
+    return sum + two;
 }
 
-// Coarse cell q = J cnx + I of the planes l and l + 1 (when it exists):
-// both sums before either store, so the shared vertical operands are loaded
-// once.
-template <class T, bool CG>
-__device__ __forceinline__ void restrict_pair(const LevelView<T>& F, const LevelView<T>& C,
-                                              unsigned q, int l) {
-    const Geo& cg = C.g;
-    const int J = (int)(q / (unsigned)cg.nx), I = (int)(q - (unsigned)J * cg.nx);
-    const unsigned cs = scol(cg, I, J);
-    const T s0 = restrict_sum<T, CG>(F, I, J, l);
-    if (l + 1 < cg.nz) {
-        const T s1 = restrict_sum<T, CG>(F, I, J, l + 1);
-        C.b[(unsigned)l * cg.plane + cs] = s0;
-        C.b[(unsigned)(l + 1) * cg.plane + cs] = s1;
-    } else {
-        C.b[(unsigned)l * cg.plane + cs] = s0;
-    }
-}
-
-// The same stored as coarse b; q = J cnx + I.
+// Coarse cell q = J cnx + I, stored as coarse b.
 template <class T, bool CG>
 __device__ __forceinline__ void restrict_cell(const LevelView<T>& F, const LevelView<T>& C, unsigned q,
                                               int l) {
@@ -383,7 +313,7 @@ __device__ __forceinline__ void gather_rhs(const LevelView<T>& L, const LevelVie
 }
 
 // Level views of the shared-memory bottom: a level's arrays lie at base in
-// the order gE, gN, gU, dg, fcp, finv, x, b, each rounded up to 16 bytes
+// the order gE, gN, gU, fcp, finv, x, b, each rounded up to 16 bytes
 // (small_level_bytes adds the same sizes). The views are rebuilt from the
 // block's base and a byte offset wherever they are used, never stored as
 // pointers, so every pointer visibly points into shared memory and the
@@ -402,7 +332,6 @@ __device__ __forceinline__ LevelView<T> small_view(unsigned char* base, const Ge
     S.gE = (const float*)take(ln * 4u);
     S.gN = (const float*)take(ln * 4u);
     S.gU = (const float*)take(ln * 4u);
-    S.dg = (T*)take(ln * (unsigned)sizeof(T));
     S.fcp = (T*)take(ln * (unsigned)sizeof(T));
     S.finv = (T*)take(ln * (unsigned)sizeof(T));
     S.x = (T*)take(ln * (unsigned)sizeof(T));
@@ -441,7 +370,7 @@ __device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, unsigned cha
             soff[k] = off;
             off += (unsigned)small_level_bytes(g, sizeof(T));
             const unsigned ln = g.plane * (unsigned)g.nz;
-            total += 3u * ln * 4u + 3u * ln * (unsigned)sizeof(T);
+            total += 3u * ln * 4u + 2u * ln * (unsigned)sizeof(T);
         }
         tma::mbar_init(&bar, 1);
         tma::mbar_init(&barb, 1);
@@ -450,9 +379,9 @@ __device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, unsigned cha
     }
     __syncthreads();
     if (threadIdx.x < 32u) {
-        // copy c of level k = c / 6: gE, gN, gU, dg, fcp, finv
-        for (int c = (int)threadIdx.x; c < 6 * nl; c += 32) {
-            const int k = c / 6, a = c - 6 * k;
+        // copy c of level k = c / 5: gE, gN, gU, fcp, finv
+        for (int c = (int)threadIdx.x; c < 5 * nl; c += 32) {
+            const int k = c / 5, a = c - 5 * k;
             const LevelView<T>& G = tl.L[k];
             const LevelView<T> S = small_view<T>(smem + soff[k], sg[k]);
             const unsigned ln = sg[k].plane * (unsigned)sg[k].nz;
@@ -460,8 +389,7 @@ __device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, unsigned cha
             if (a == 0) tma::bulk_load((void*)S.gE, G.gE, fb, &bar);
             else if (a == 1) tma::bulk_load((void*)S.gN, G.gN, fb, &bar);
             else if (a == 2) tma::bulk_load((void*)S.gU, G.gU, fb, &bar);
-            else if (a == 3) tma::bulk_load(S.dg, G.dg, tb, &bar);
-            else if (a == 4) tma::bulk_load(S.fcp, G.fcp, tb, &bar);
+            else if (a == 3) tma::bulk_load(S.fcp, G.fcp, tb, &bar);
             else tma::bulk_load(S.finv, G.finv, tb, &bar);
         }
     }

@@ -47,11 +47,8 @@ __device__ __forceinline__ T face_sum_rn(const LevelView<T>& L, int i, int j, in
     return RN<T>::add(d, RN<T>::of(l > 0 ? L.gU[id - g.plane] : L.gB[s]));
 }
 
-// Thomas factors of natural column q = j nx + i of a level, and its cells'
-// diagonals for the restriction (dg). Both diagonals are the face sum plus
-// C/dt; the factorisation adds the rounded product (mg_factor_column's
-// arithmetic), the restriction's residual the product fused. The factors are
-// written through restrict pointers, so the operand loads of the next planes
+// Thomas factors of natural column q = j nx + i of a level (mg_factor_column's
+// arithmetic, src/mg3d.h:46-61). The factors are written through restrict pointers, so the operand loads of the next planes
 // may be issued before this plane's stores.
 template <class T>
 __device__ __forceinline__ void factor_column(const LevelView<T>& L, T inv_dt, unsigned q) {
@@ -60,7 +57,6 @@ __device__ __forceinline__ void factor_column(const LevelView<T>& L, T inv_dt, u
     const unsigned s = scol(g, i, j);
     T* __restrict__ finv = L.finv;
     T* __restrict__ fcp = L.fcp;
-    T* __restrict__ dg = L.dg;
     const float* __restrict__ gU = L.gU;
     T cp_prev = 0;
 #pragma unroll 4
@@ -68,7 +64,6 @@ __device__ __forceinline__ void factor_column(const LevelView<T>& L, T inv_dt, u
         const unsigned id = (unsigned)l * g.plane + s;
         const T faces = face_sum_rn(L, i, j, l), cap = RN<T>::of(L.cap[id]);
         const T d = RN<T>::add(faces, RN<T>::mul(cap, inv_dt));
-        dg[id] = RN<T>::fma(cap, inv_dt, faces);
         const T lower = l > 0 ? -RN<T>::of(gU[id - g.plane]) : T(0);
         const T upper = l < g.nz - 1 ? -RN<T>::of(gU[id]) : T(0);
         const T inv = RN<T>::div(T(1), RN<T>::sub(d, RN<T>::mul(lower, cp_prev)));

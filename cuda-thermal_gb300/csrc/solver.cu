@@ -161,7 +161,6 @@ ct_status Solver::create(const ct_model* m_in, ct_precond pc_, ct_precision prec
             }
             L.o_fcp = ar.take(ln * tsize);
             L.o_finv = ar.take(ln * tsize);
-            L.o_dg = ar.take(ln * tsize);
             L.o_x = ar.take(ln * tsize);
             L.o_b = ar.take(ln * tsize);
             L.o_dx = ar.take(L.dx.size() * 8);
@@ -458,7 +457,7 @@ void Solver::vcycle(size_t k, Cond cond, bool first_sweep_done) {
     // bound, and the block's serial line-solve tail costs more (measured at
     // 800 x 800: 78 us fused against 51 + 13 us) than the launch it saves.
     const bool fuse = fuse_sweep0 && k > 0 && k + 1 != small_k0 && L.g.nz <= 32;
-    const double b_restrict = cells * (3 * t + 12) + cells / 4 * t;
+    const double b_restrict = cells * (t / 2 + 8) + cells / 4 * t;
     const double cc = (double)C.g.nx * C.g.ny * C.g.nz;
     if (fuse)
         enq(("mg_restrict_sweep0" + lvl).c_str(), b_restrict + cc / 2 * (3 * t + 4),

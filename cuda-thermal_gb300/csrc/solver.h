@@ -27,7 +27,7 @@ struct Arena {
 // Host-side record of one multigrid level.
 struct Level {
     Geo g;
-    size_t o_gE, o_gN, o_gU, o_gB, o_cap, o_fcp, o_finv, o_dg, o_x, o_b, o_dx, o_dy;
+    size_t o_gE, o_gN, o_gU, o_gB, o_cap, o_fcp, o_finv, o_x, o_b, o_dx, o_dy;
     std::vector<double> dx, dy;  // cell widths (m), for the coarsening
     bool tma = false;            // sweeps staged by bulk tensor copies (maps per colour)
     SweepMaps maps[2];
@@ -167,7 +167,6 @@ class Solver {
         v.cap = at<float>(L.o_cap);
         v.fcp = at<T>(L.o_fcp);
         v.finv = at<T>(L.o_finv);
-        v.dg = at<T>(L.o_dg);
         v.x = at<T>(L.o_x);
         v.b = at<T>(L.o_b);
         return v;
