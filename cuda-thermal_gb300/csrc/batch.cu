@@ -495,7 +495,8 @@ ct_status Batch::tune_bucket(Bucket& b) {
                 ins_g.push_back(i);
                 items_g.push_back((unsigned)g.ny * (unsigned)g.hx);
             }
-            restr_items.push_back((unsigned)c.nx * (unsigned)c.ny * (unsigned)c.nz);
+            restr_items.push_back(((unsigned)c.nx + kRestrictWide - 1u) / kRestrictWide * (unsigned)c.ny *
+                                  (unsigned)c.nz);
         }
         auto time_of = [&](auto&& launch) -> float {
             launch();  // warm

@@ -356,9 +356,9 @@ __global__ void __launch_bounds__(NT)
         sweep_column<float, MZ, ZERO, PRO, false>(L, C, color, q);
 }
 
-// Compiled for 4 blocks per SM (64 registers): level 0 of the 256-instance
-// batch 296 us per launch against 429 us with the compiler's own choice (also
-// 64 registers), as for the single solver's k_restrict2.
+// Coarse cells of one instance, kRestrictWide a thread; compiled for 4 blocks per SM
+// (48 stacks, the finest level: 28.9 us a launch against 34.1 with the compiler's own
+// choice).
 __global__ void __launch_bounds__(NT, 4)
     kb_restrict(Plan p, const LevelView<float>* __restrict__ views,
                 const LevelView<float>* __restrict__ cviews, const Ctl* ctl) {
@@ -368,10 +368,11 @@ __global__ void __launch_bounds__(NT, 4)
     if (inst_done(c)) return;
     const LevelView<float> L = views[t.inst];
     const LevelView<float> C = cviews[t.inst];
-    const unsigned ccols = (unsigned)C.g.nx * (unsigned)C.g.ny;
+    constexpr unsigned W = kRestrictWide;
+    const unsigned ccols = ((unsigned)C.g.nx + W - 1u) / W * (unsigned)C.g.ny;
     for (unsigned w = t.begin + threadIdx.x; w < t.end; w += NT) {
         const int l = (int)(w / ccols);
-        restrict_cell<float, false>(L, C, w - (unsigned)l * ccols, l);
+        restrict_wide_store<float, W>(L, C, w - (unsigned)l * ccols, l);
     }
 }
 

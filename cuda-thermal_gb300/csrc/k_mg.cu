@@ -233,6 +233,20 @@ __global__ void __launch_bounds__(NT)
     C.b[(unsigned)l * cg.plane + scol(cg, I, J)] = sum;
 }
 
+// The same on large FP32 levels, W cells a thread (restrict_wide): 800 x 800 x 10
+// 14.7 us (17.5 with two cells, 23.0 with one), 1024 x 1024 x 16 34.0 (38.9, 47.6);
+// in FP64 one cell a thread is the faster (400 x 400 x 10: 13.1 against 17.0).
+template <int W>
+__global__ void __launch_bounds__(NT)
+    k_restrict_wide(LevelView<float> F, LevelView<float> C, const Ctl* ctl, Cond cond) {
+    pdl_enter();
+    if (loop_done(ctl, cond)) return;
+    pdl_trigger();  // several waves: the dependent launches as the last one starts
+    const unsigned q = blockIdx.x * NT + threadIdx.x;
+    if (q >= ((unsigned)C.g.nx + W - 1u) / W * (unsigned)C.g.ny) return;
+    restrict_wide_store<float, W>(F, C, q, (int)blockIdx.y);
+}
+
 // Restriction F -> C fused with C's first sweep (x = 0, red columns). A
 // block is 32 coarse columns x nz planes, one thread per coarse cell and
 // plane; each thread also stages its cell's b and, for a red column,
@@ -400,6 +414,14 @@ void launch_sweep(cudaStream_t st, const LevelView<T>& L, int color, bool zero_x
 template <class T>
 void launch_restrict(cudaStream_t st, const LevelView<T>& F, const LevelView<T>& C, const Ctl* ctl,
                      Cond cond) {
+    if constexpr (sizeof(T) == 4) {
+        if ((unsigned)F.g.nx * (unsigned)F.g.ny > kRestrictWideColumns) {
+            constexpr int W = kRestrictWide;
+            const dim3 wide(blocks_for(((unsigned)C.g.nx + W - 1u) / W * (unsigned)C.g.ny), (unsigned)C.g.nz);
+            launch_pdl(k_restrict_wide<W>, wide, NT, 0, st, F, C, ctl, cond);
+            return;
+        }
+    }
     const dim3 grid(blocks_for((unsigned)C.g.nx * C.g.ny), (unsigned)C.g.nz);
     launch_pdl(k_restrict<T>, grid, NT, 0, st, F, C, ctl, cond);
 }

@@ -199,6 +199,12 @@ void launch_factor(cudaStream_t st, const LevelView<T>& L, T inv_dt);
 // V-cycle), so lateral neighbours are not read. xc: when not null, the
 // coarser level's x is added to every neighbour value read (prolongation
 // fused into the sweep).
+// FP32 levels of more than this many columns restrict kRestrictWide coarse cells a
+// thread, smaller ones one (237 x 181 x 13: 6.7 us against 7.6; at 100 x 100 the
+// launch's latency either way). The batch does on every level (48 stacks, the finest
+// level: 28 us, 30.8 with two cells, 36.9 with one; the third 8.5, 8.6, 9.4).
+constexpr unsigned kRestrictWideColumns = 128u * 128u;
+constexpr int kRestrictWide = 4;
 // Levels of at most this many columns sweep with one thread per column and
 // plane (k_sweep_split); larger FP32 levels are staged by bulk tensor copies
 // (at 800 x 800: the 200 x 200 level split 6.96 ms per solve against 7.07 ms

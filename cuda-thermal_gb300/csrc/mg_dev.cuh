@@ -241,6 +241,24 @@ __device__ __forceinline__ void sweep_column(const LevelView<T>& L, const LevelV
     }
 }
 
+// The two red children's terms of restrict_sum from operands already loaded: west,
+// east, south, north of (2I, 2J), then of (2I + 1, 2J + 1).
+template <class T>
+__device__ __forceinline__ T red_residuals(bool w, bool e, bool so, bool no, bool both, bool e2, bool n2, float gw,
+                                           float ge, float gs, float gn, float hw, float he, float hs, float hn, T xw,
+                                           T x10, T xs, T x01, T xe, T xn) {
+    T sum = 0, two = 0;
+    sum += (w ? face<T>(gw) : T(0)) * xw;
+    sum += (e ? face<T>(ge) : T(0)) * x10;
+    sum += (so ? face<T>(gs) : T(0)) * xs;
+    sum += (no ? face<T>(gn) : T(0)) * x01;
+    two += (both ? face<T>(hw) : T(0)) * x01;
+    two += (e2 ? face<T>(he) : T(0)) * xe;
+    two += (both ? face<T>(hs) : T(0)) * x10;
+    two += (n2 ? face<T>(hn) : T(0)) * xn;
+    return sum + two;
+}
+
 // Restriction (src/pcg3d_cpu.cpp:87-100) of coarse cell (I, J, l): the sum over
 // its (up to 4) children of the fine residual b - (A + C/dt) x, x being the
 // iterate of the V-cycle's way down: the red columns solved from x = 0, then the
@@ -271,16 +289,55 @@ __device__ __forceinline__ T restrict_sum(const LevelView<T>& F, int I, int J, i
     const T xw = ldm<CG>(F.x + a_w), xs = ldm<CG>(F.x + a_s), xe = ldm<CG>(F.x + a_e), xn = ldm<CG>(F.x + a_n);
     const float gw = F.gE[a_w], ge = F.gE[c00], gs = F.gN[a_s], gn = F.gN[c00];
     const float hw = F.gE[c01], he = F.gE[c11], hs = F.gN[c10], hn = F.gN[c11];
-    T sum = 0, two = 0;
-    sum += (w ? face<T>(gw) : T(0)) * xw;
-    sum += (e ? face<T>(ge) : T(0)) * x10;
-    sum += (so ? face<T>(gs) : T(0)) * xs;
-    sum += (no ? face<T>(gn) : T(0)) * x01;
-    two += (both ? face<T>(hw) : T(0)) * x01;
-    two += (e2 ? face<T>(he) : T(0)) * xe;
-    two += (both ? face<T>(hs) : T(0)) * x10;
-    two += (n2 ? face<T>(hn) : T(0)) * xn;
-    return sum + two;
+    return red_residuals<T>(w, e, so, no, both, e2, n2, gw, ge, gs, gn, hw, he, hs, hn, xw, x10, xs, x01, xe, xn);
+}
+
+// W coarse cells (I .. I + W - 1, J) of plane l at once, I a multiple of W: their
+// operands lie side by side, so a load brings W of them, and a black column's x
+// and faces serve the cells on both its sides.
+template <class T, int W>
+struct alignas(W * sizeof(T)) Lane {
+    T v[W];
+};
+template <class T, int W>
+__device__ __forceinline__ void restrict_wide(const LevelView<T>& F, int I, int J, int l, T (&s)[W]) {
+    const Geo& g = F.g;
+    const int i0 = 2 * I, j0 = 2 * J;
+    const bool so = j0 > 0, no = j0 + 1 < g.ny, nn = j0 + 2 < g.ny;
+    const unsigned hx = (unsigned)g.hx, base = (unsigned)l * g.plane;
+    const unsigned c00 = base + 4u * (unsigned)J * hx + (unsigned)I, c10 = c00 + hx;
+    const unsigned c11 = no ? c00 + 2u * hx : c00, c01 = no ? c10 + 2u * hx : c10;
+    const unsigned a_s = so ? c10 - 2u * hx : c10, a_n = nn ? c10 + 4u * hx : c10;
+    auto xs_at = [&](unsigned k) { return *reinterpret_cast<const Lane<T, W>*>(F.x + k); };
+    auto f_at = [&](const float* f, unsigned k) { return *reinterpret_cast<const Lane<float, W>*>(f + k); };
+    const Lane<T, W> x10 = xs_at(c10), x01 = xs_at(c01), xs = xs_at(a_s), xn = xs_at(a_n);
+    const Lane<float, W> ge = f_at(F.gE, c00), gb = f_at(F.gE, c10), hw = f_at(F.gE, c01), he = f_at(F.gE, c11);
+    const Lane<float, W> gs = f_at(F.gN, a_s), gn = f_at(F.gN, c00), hs = f_at(F.gN, c10), hn = f_at(F.gN, c11);
+    const bool w0 = I > 0, e0 = i0 + 2 * W < g.nx;  // a column beyond the first and the last cell
+    const T xw = w0 ? F.x[c10 - 1u] : T(0), xe = no && e0 ? F.x[c01 + (unsigned)W] : T(0);
+    const float gw = w0 ? F.gE[c10 - 1u] : 0.0f;
+#pragma unroll
+    for (int c = 0; c < W; ++c) {
+        const bool e = i0 + 2 * c + 1 < g.nx, both = e && no;
+        const bool e2 = both && i0 + 2 * c + 2 < g.nx, n2 = both && nn;
+        s[c] = red_residuals<T>(c > 0 || w0, e, so, no, both, e2, n2, c > 0 ? gb.v[c > 0 ? c - 1 : 0] : gw, ge.v[c],
+                                gs.v[c], gn.v[c], hw.v[c], he.v[c], hs.v[c], hn.v[c],
+                                c > 0 ? x10.v[c > 0 ? c - 1 : 0] : xw, x10.v[c], xs.v[c], x01.v[c],
+                                c + 1 < W ? x01.v[c + 1 < W ? c + 1 : 0] : xe, xn.v[c]);
+    }
+}
+// ... stored as coarse b (cells past the row's end left alone).
+template <class T, int W>
+__device__ __forceinline__ void restrict_wide_store(const LevelView<T>& F, const LevelView<T>& C, unsigned q, int l) {
+    const Geo& cg = C.g;
+    const unsigned groups = ((unsigned)cg.nx + W - 1u) / W;
+    const int J = (int)(q / groups), I = (int)(q - (unsigned)J * groups) * W;
+    T s[W];
+    restrict_wide<T, W>(F, I, J, l, s);
+    T* const row = C.b + (unsigned)l * cg.plane + 2u * (unsigned)J * (unsigned)cg.hx + (unsigned)(I >> 1);
+#pragma unroll
+    for (int c = 0; c < W; ++c)
+        if (I + c < cg.nx) row[(((c + J) & 1) ? cg.hx : 0) + (c >> 1)] = s[c];
 }
 
 // Coarse cell q = J cnx + I, stored as coarse b.
