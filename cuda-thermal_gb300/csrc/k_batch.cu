@@ -368,11 +368,14 @@ __global__ void __launch_bounds__(NT, 4)
     if (inst_done(c)) return;
     const LevelView<float> L = views[t.inst];
     const LevelView<float> C = cviews[t.inst];
-    constexpr unsigned W = kRestrictWide;
-    const unsigned ccols = ((unsigned)C.g.nx + W - 1u) / W * (unsigned)C.g.ny;
+    constexpr int W = kRestrictWide;
+    const unsigned groups = ((unsigned)C.g.nx + W - 1u) / W;
     for (unsigned w = t.begin + threadIdx.x; w < t.end; w += NT) {
-        const int l = (int)(w / ccols);
-        restrict_wide_store<float, W>(L, C, w - (unsigned)l * ccols, l);
+        const unsigned row = w / groups, l = row / (unsigned)C.g.ny;
+        const int J = (int)(row - l * (unsigned)C.g.ny), I = (int)(w - row * groups) * (int)W;
+        float s[W];
+        restrict_wide<float, W>(L, wide_faces<float, W>(L, I, J, (int)l), I, J, (int)l, s);
+        store_wide<float, W>(C, I, J, (int)l, s);
     }
 }
 

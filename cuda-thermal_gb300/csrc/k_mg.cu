@@ -136,8 +136,6 @@ __global__ void __launch_bounds__(NT, (ZERO && sizeof(T) == 4 && MZ > 0 && MZ <=
 template <class T, int MZ, bool ZERO, bool PRO>
 __global__ void __launch_bounds__(32 * MZ)
     k_sweep_split(LevelView<T> L, int color, LevelView<T> C, const Ctl* ctl, Cond cond) {
-    pdl_enter();
-    const int2 flags = loop_flags(ctl);  // tested after the gathers are issued
     __shared__ T sv[MZ][32], sfi[MZ][32], sfc[MZ][32];
     __shared__ float sgu[MZ][32];
     const Geo& g = L.g;
@@ -147,23 +145,59 @@ __global__ void __launch_bounds__(32 * MZ)
     const int j = (int)(q / (unsigned)g.hx), t = (int)(q - (unsigned)j * g.hx);
     const int i = 2 * t + ((j + color) & 1);
     const bool on = q < (unsigned)g.ny * (unsigned)g.hx && i < g.nx;
-    unsigned s = 0;
+    const Nbr n = neighbours<PRO>(g, C.g, i, j, t, color);
+    const unsigned s = n.s, base = (unsigned)l * g.plane, id = base + s;
     T rhs = 0, fi = 0, fc = 0;
-    float gu = 0.0f;
+    float gu = 0.0f, gw = 0.0f, ge = 0.0f, gs = 0.0f, gn = 0.0f;
+    // before the wait for the preceding kernel (kernels.h): the operator and the
+    // factors, on the way up b, and ahead of the prolongation x as well
+    const bool b_early = PRO || (!ZERO && color == 0);
+    T xw = 0, xe = 0, xs = 0, xn = 0;
+    auto load_x = [&] {
+        if (n.w) xw = L.x[base + n.sw];
+        if (n.e) xe = L.x[base + n.se];
+        if (n.so) xs = L.x[base + n.ss];
+        if (n.no) xn = L.x[base + n.sn];
+    };
     if (on) {
-        const Nbr n = neighbours<PRO>(g, C.g, i, j, t, color);
-        s = n.s;
-        const unsigned id = (unsigned)l * g.plane + n.s;
-        rhs = L.b[id];
-        if (!ZERO) rhs = rhs + lat_sum<T, PRO, false>(L, C, n, l);
         fi = L.finv[id];
         gu = L.gU[id];
-        // the x = 0 sweep recomputes fcp as factor_column rounded it (one
-        // operand stream less); the others load it
-        fc = ZERO ? fcp_of(gu, fi) : L.fcp[id];
+        if (!ZERO) {
+            fc = L.fcp[id];
+            if (n.w) gw = L.gE[base + n.sw];
+            ge = L.gE[id];
+            if (n.so) gs = L.gN[base + n.ss];
+            gn = L.gN[id];
+        }
+        if (b_early) rhs = L.b[id];
+        if (PRO) load_x();
+    }
+    pdl_enter();
+    pdl_trigger();
+    const int2 flags = loop_flags(ctl);  // tested after the gathers are issued
+    if (on) {
+        if (!b_early) rhs = L.b[id];
+        if (!ZERO) {
+            if (PRO) {
+                const T* const cx = C.x + (unsigned)l * C.g.plane;
+                if (n.w) xw = xw + cx[n.pw];
+                if (n.e) xe = xe + cx[n.pe];
+                if (n.so) xs = xs + cx[n.ps];
+                if (n.no) xn = xn + cx[n.pn];
+            } else {
+                load_x();
+            }
+            T sum = 0;  // lat_sum's order
+            if (n.w) sum += face<T>(gw) * xw;
+            if (n.e) sum += face<T>(ge) * xe;
+            if (n.so) sum += face<T>(gs) * xs;
+            if (n.no) sum += face<T>(gn) * xn;
+            rhs = rhs + sum;
+        } else {
+            fc = fcp_of(gu, fi);  // as factor_column rounded it (one operand stream less)
+        }
     }
     if (loop_done(flags, cond)) return;  // the same for every thread of the grid
-    pdl_trigger();
     if (on) {
         sv[l][tx] = rhs;
         sfi[l][tx] = fi;
@@ -220,16 +254,17 @@ __global__ void __launch_bounds__(32 * MZ)
 template <class T>
 __global__ void __launch_bounds__(NT)
     k_restrict(LevelView<T> F, LevelView<T> C, const Ctl* ctl, Cond cond) {
-    pdl_enter();
-    const int2 flags = loop_flags(ctl);  // tested after the sums' loads are issued
     const unsigned q = blockIdx.x * NT + threadIdx.x;
     const Geo& cg = C.g;
     const bool on = q < (unsigned)cg.nx * (unsigned)cg.ny;
     const int J = on ? (int)(q / (unsigned)cg.nx) : 0, I = on ? (int)(q - (unsigned)J * cg.nx) : 0;
     const int l = (int)blockIdx.y;
-    const T sum = on ? restrict_sum<T, false>(F, I, J, l) : T(0);
-    if (loop_done(flags, cond) || !on) return;
+    const RedFaces f = red_faces(F, I, J, l);  // before the wait: not written during a solve
+    pdl_enter();
     pdl_trigger();
+    const int2 flags = loop_flags(ctl);  // tested after the sums' loads are issued
+    const T sum = on ? restrict_sum<T, false>(F, f, I, J, l) : T(0);
+    if (loop_done(flags, cond) || !on) return;
     C.b[(unsigned)l * cg.plane + scol(cg, I, J)] = sum;
 }
 
@@ -239,12 +274,17 @@ __global__ void __launch_bounds__(NT)
 template <int W>
 __global__ void __launch_bounds__(NT)
     k_restrict_wide(LevelView<float> F, LevelView<float> C, const Ctl* ctl, Cond cond) {
-    pdl_enter();
-    if (loop_done(ctl, cond)) return;
-    pdl_trigger();  // several waves: the dependent launches as the last one starts
+    const unsigned groups = ((unsigned)C.g.nx + W - 1u) / W;
     const unsigned q = blockIdx.x * NT + threadIdx.x;
-    if (q >= ((unsigned)C.g.nx + W - 1u) / W * (unsigned)C.g.ny) return;
-    restrict_wide_store<float, W>(F, C, q, (int)blockIdx.y);
+    const bool on = q < groups * (unsigned)C.g.ny;
+    const int J = on ? (int)(q / groups) : 0, I = on ? (int)(q - (unsigned)J * groups) * W : 0, l = (int)blockIdx.y;
+    const WideFaces<W> f = wide_faces<float, W>(F, I, J, l);  // before the wait, as k_restrict
+    pdl_enter();
+    pdl_trigger();  // several waves: the dependent launches as the last one starts
+    if (loop_done(ctl, cond) || !on) return;
+    float s[W];
+    restrict_wide<float, W>(F, f, I, J, l, s);
+    store_wide<float, W>(C, I, J, l, s);
 }
 
 // Restriction F -> C fused with C's first sweep (x = 0, red columns). A
@@ -257,8 +297,6 @@ __global__ void __launch_bounds__(NT)
 template <class T, int MZ>
 __global__ void __launch_bounds__(32 * MZ)
     k_restrict_sweep0(LevelView<T> F, LevelView<T> C, const Ctl* ctl, Cond cond) {
-    pdl_enter();
-    const int2 flags = loop_flags(ctl);  // tested after the sums' loads are issued
     __shared__ T sb[MZ][32], sfi[MZ][32];
     __shared__ float sgu[MZ][32];
     const Geo& cg = C.g;
@@ -271,15 +309,16 @@ __global__ void __launch_bounds__(32 * MZ)
     const unsigned id = (unsigned)l * cg.plane + cs;
     T sum = 0, fi = 0;
     float gu = 0.0f;
-    if (on) {
-        sum = restrict_sum<T, false>(F, I, J, l);
-        if (red) {
-            fi = C.finv[id];
-            gu = C.gU[id];
-        }
+    const RedFaces f = red_faces(F, I, J, l);  // before the wait, as the factors
+    if (red) {
+        fi = C.finv[id];
+        gu = C.gU[id];
     }
-    if (loop_done(flags, cond)) return;  // the same for every thread of the grid
+    pdl_enter();
     pdl_trigger();
+    const int2 flags = loop_flags(ctl);  // tested after the sums' loads are issued
+    if (on) sum = restrict_sum<T, false>(F, f, I, J, l);
+    if (loop_done(flags, cond)) return;  // the same for every thread of the grid
     if (on) {
         C.b[id] = sum;
         if (red) {

@@ -344,6 +344,7 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
     for (int i = tid; i < P.x4; i += 32 * warps) reinterpret_cast<float4*>(sm + P.x)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     cluster_arrive();  // this CTA's shared memory may be written by its peers after this
     pdl_enter();
+    pdl_trigger();  // the dependent's blocks load what this kernel does not write
     const bool first = k_lo == 0 && k_hi > 0;  // holds rows of the first level
     if (tid == 0 && first) {
         tma::mbar_arrive_expect_tx(barb, (unsigned)(P.L[0].rows * 2 * P.L[0].hx * nz) * 4u);
@@ -433,7 +434,6 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
         ok = ok && tma::mbar_wait(bar1, 0u);
     }
     cluster_arrive();  // no CTA leaves before its peers have sent what they send
-    pdl_trigger();
     if (!closed && first) {  // the first level's x, whole rows (padding is zero)
         const TailLevel& F = tail_level(0);
         const int RS = 2 * F.hx, j0 = c.row0(0), row4 = (nd > 0 ? min(F.rows, F.ny - j0) : F.ny) * RS / 4;

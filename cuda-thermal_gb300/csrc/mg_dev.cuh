@@ -259,6 +259,38 @@ __device__ __forceinline__ T red_residuals(bool w, bool e, bool so, bool no, boo
     return sum + two;
 }
 
+// The faces of restrict_sum at coarse cell (I, J, l) and where they and the black
+// x beside them lie (an absent neighbour reads a cell beside it).
+struct RedFaces {
+    float gw, ge, gs, gn, hw, he, hs, hn;
+};
+struct RedSlots {
+    bool w, e, so, no, both, e2, n2;
+    unsigned c00, c10, c01, c11, a_w, a_s, a_e, a_n;
+};
+__device__ __forceinline__ RedSlots red_slots(const Geo& g, int I, int J, int l) {
+    RedSlots r;
+    const int i0 = 2 * I, j0 = 2 * J;
+    r.w = i0 > 0, r.e = i0 + 1 < g.nx, r.so = j0 > 0, r.no = j0 + 1 < g.ny;
+    r.both = r.e && r.no, r.e2 = r.both && i0 + 2 < g.nx, r.n2 = r.both && j0 + 2 < g.ny;
+    const unsigned hx = (unsigned)g.hx;
+    // red (2I, 2J), black (2I + 1, 2J); black (2I, 2J + 1), red (2I + 1, 2J + 1)
+    r.c00 = (unsigned)l * g.plane + 4u * (unsigned)J * hx + (unsigned)I;
+    r.c10 = r.c00 + hx;
+    r.c11 = r.no ? r.c00 + 2u * hx : r.c00;
+    r.c01 = r.no ? r.c10 + 2u * hx : r.c10;
+    r.a_w = r.w ? r.c10 - 1u : r.c10;
+    r.a_s = r.so ? r.c10 - 2u * hx : r.c10;
+    r.a_e = r.e2 ? r.c01 + 1u : r.c01;
+    r.a_n = r.n2 ? r.c10 + 4u * hx : r.c10;
+    return r;
+}
+template <class T>
+__device__ __forceinline__ RedFaces red_faces(const LevelView<T>& F, int I, int J, int l) {
+    const RedSlots r = red_slots(F.g, I, J, l);
+    return RedFaces{F.gE[r.a_w], F.gE[r.c00], F.gN[r.a_s], F.gN[r.c00], F.gE[r.c01], F.gE[r.c11], F.gN[r.c10], F.gN[r.c11]};
+}
+
 // Restriction (src/pcg3d_cpu.cpp:87-100) of coarse cell (I, J, l): the sum over
 // its (up to 4) children of the fine residual b - (A + C/dt) x, x being the
 // iterate of the V-cycle's way down: the red columns solved from x = 0, then the
@@ -273,23 +305,12 @@ __device__ __forceinline__ T red_residuals(bool w, bool e, bool so, bool no, boo
 // (23.0 so) and, in FP64, 47 at 400 x 400 x 10 (13.1); an iteration 382 -> 359 and
 // 388 -> 318.
 template <class T, bool CG>
-__device__ __forceinline__ T restrict_sum(const LevelView<T>& F, int I, int J, int l) {
-    const Geo& g = F.g;
-    const int i0 = 2 * I, j0 = 2 * J;
-    const bool w = i0 > 0, e = i0 + 1 < g.nx, so = j0 > 0, no = j0 + 1 < g.ny;
-    const bool both = e && no, e2 = both && i0 + 2 < g.nx, n2 = both && j0 + 2 < g.ny;
-    const unsigned base = (unsigned)l * g.plane, hx = (unsigned)g.hx;
-    // slots: red (2I, 2J), black (2I + 1, 2J); black (2I, 2J + 1), red (2I + 1, 2J + 1)
-    const unsigned c00 = base + 4u * (unsigned)J * hx + (unsigned)I, c10 = c00 + hx;
-    const unsigned c11 = no ? c00 + 2u * hx : c00, c01 = no ? c10 + 2u * hx : c10;
-    // (an absent neighbour reads a cell beside it, with a zero face)
-    const unsigned a_w = w ? c10 - 1u : c10, a_s = so ? c10 - 2u * hx : c10;
-    const unsigned a_e = e2 ? c01 + 1u : c01, a_n = n2 ? c10 + 4u * hx : c10;
-    const T x10 = ldm<CG>(F.x + c10), x01 = ldm<CG>(F.x + c01);
-    const T xw = ldm<CG>(F.x + a_w), xs = ldm<CG>(F.x + a_s), xe = ldm<CG>(F.x + a_e), xn = ldm<CG>(F.x + a_n);
-    const float gw = F.gE[a_w], ge = F.gE[c00], gs = F.gN[a_s], gn = F.gN[c00];
-    const float hw = F.gE[c01], he = F.gE[c11], hs = F.gN[c10], hn = F.gN[c11];
-    return red_residuals<T>(w, e, so, no, both, e2, n2, gw, ge, gs, gn, hw, he, hs, hn, xw, x10, xs, x01, xe, xn);
+__device__ __forceinline__ T restrict_sum(const LevelView<T>& F, const RedFaces& f, int I, int J, int l) {
+    const RedSlots r = red_slots(F.g, I, J, l);
+    const T x10 = ldm<CG>(F.x + r.c10), x01 = ldm<CG>(F.x + r.c01), xw = ldm<CG>(F.x + r.a_w), xs = ldm<CG>(F.x + r.a_s);
+    const T xe = ldm<CG>(F.x + r.a_e), xn = ldm<CG>(F.x + r.a_n);
+    return red_residuals<T>(r.w, r.e, r.so, r.no, r.both, r.e2, r.n2, f.gw, f.ge, f.gs, f.gn, f.hw, f.he, f.hs, f.hn, xw,
+                            x10, xs, x01, xe, xn);
 }
 
 // W coarse cells (I .. I + W - 1, J) of plane l at once, I a multiple of W: their
@@ -299,41 +320,61 @@ template <class T, int W>
 struct alignas(W * sizeof(T)) Lane {
     T v[W];
 };
+template <int W>
+struct WideFaces {
+    Lane<float, W> ge, gb, hw, he, gs, gn, hs, hn;
+    float gw;
+};
+// Where the rows lie: red and black of row 2J, red and black of row 2J + 1, the
+// black rows to the south and north (an absent one reads a row beside it).
+struct WideRows {
+    bool so, no, nn;
+    unsigned c00, c10, c11, c01, a_s, a_n;
+};
+__device__ __forceinline__ WideRows wide_rows(const Geo& g, int I, int J, int l) {
+    WideRows r;
+    const int j0 = 2 * J;
+    const unsigned hx = (unsigned)g.hx;
+    r.so = j0 > 0, r.no = j0 + 1 < g.ny, r.nn = j0 + 2 < g.ny;
+    r.c00 = (unsigned)l * g.plane + 4u * (unsigned)J * hx + (unsigned)I;
+    r.c10 = r.c00 + hx;
+    r.c11 = r.no ? r.c00 + 2u * hx : r.c00;
+    r.c01 = r.no ? r.c10 + 2u * hx : r.c10;
+    r.a_s = r.so ? r.c10 - 2u * hx : r.c10;
+    r.a_n = r.nn ? r.c10 + 4u * hx : r.c10;
+    return r;
+}
 template <class T, int W>
-__device__ __forceinline__ void restrict_wide(const LevelView<T>& F, int I, int J, int l, T (&s)[W]) {
+__device__ __forceinline__ WideFaces<W> wide_faces(const LevelView<T>& F, int I, int J, int l) {
+    const WideRows r = wide_rows(F.g, I, J, l);
+    auto at = [&](const float* f, unsigned k) { return *reinterpret_cast<const Lane<float, W>*>(f + k); };
+    return WideFaces<W>{at(F.gE, r.c00), at(F.gE, r.c10), at(F.gE, r.c01), at(F.gE, r.c11), at(F.gN, r.a_s),
+                        at(F.gN, r.c00), at(F.gN, r.c10), at(F.gN, r.c11), I > 0 ? F.gE[r.c10 - 1u] : 0.0f};
+}
+template <class T, int W>
+__device__ __forceinline__ void restrict_wide(const LevelView<T>& F, const WideFaces<W>& f, int I, int J, int l,
+                                              T (&s)[W]) {
     const Geo& g = F.g;
-    const int i0 = 2 * I, j0 = 2 * J;
-    const bool so = j0 > 0, no = j0 + 1 < g.ny, nn = j0 + 2 < g.ny;
-    const unsigned hx = (unsigned)g.hx, base = (unsigned)l * g.plane;
-    const unsigned c00 = base + 4u * (unsigned)J * hx + (unsigned)I, c10 = c00 + hx;
-    const unsigned c11 = no ? c00 + 2u * hx : c00, c01 = no ? c10 + 2u * hx : c10;
-    const unsigned a_s = so ? c10 - 2u * hx : c10, a_n = nn ? c10 + 4u * hx : c10;
-    auto xs_at = [&](unsigned k) { return *reinterpret_cast<const Lane<T, W>*>(F.x + k); };
-    auto f_at = [&](const float* f, unsigned k) { return *reinterpret_cast<const Lane<float, W>*>(f + k); };
-    const Lane<T, W> x10 = xs_at(c10), x01 = xs_at(c01), xs = xs_at(a_s), xn = xs_at(a_n);
-    const Lane<float, W> ge = f_at(F.gE, c00), gb = f_at(F.gE, c10), hw = f_at(F.gE, c01), he = f_at(F.gE, c11);
-    const Lane<float, W> gs = f_at(F.gN, a_s), gn = f_at(F.gN, c00), hs = f_at(F.gN, c10), hn = f_at(F.gN, c11);
+    const int i0 = 2 * I;
+    const WideRows r = wide_rows(g, I, J, l);
+    auto at = [&](unsigned k) { return *reinterpret_cast<const Lane<T, W>*>(F.x + k); };
+    const Lane<T, W> x10 = at(r.c10), x01 = at(r.c01), xs = at(r.a_s), xn = at(r.a_n);
     const bool w0 = I > 0, e0 = i0 + 2 * W < g.nx;  // a column beyond the first and the last cell
-    const T xw = w0 ? F.x[c10 - 1u] : T(0), xe = no && e0 ? F.x[c01 + (unsigned)W] : T(0);
-    const float gw = w0 ? F.gE[c10 - 1u] : 0.0f;
+    const T xw = w0 ? F.x[r.c10 - 1u] : T(0), xe = r.no && e0 ? F.x[r.c01 + (unsigned)W] : T(0);
 #pragma unroll
     for (int c = 0; c < W; ++c) {
-        const bool e = i0 + 2 * c + 1 < g.nx, both = e && no;
-        const bool e2 = both && i0 + 2 * c + 2 < g.nx, n2 = both && nn;
-        s[c] = red_residuals<T>(c > 0 || w0, e, so, no, both, e2, n2, c > 0 ? gb.v[c > 0 ? c - 1 : 0] : gw, ge.v[c],
-                                gs.v[c], gn.v[c], hw.v[c], he.v[c], hs.v[c], hn.v[c],
-                                c > 0 ? x10.v[c > 0 ? c - 1 : 0] : xw, x10.v[c], xs.v[c], x01.v[c],
-                                c + 1 < W ? x01.v[c + 1 < W ? c + 1 : 0] : xe, xn.v[c]);
+        const int b = c > 0 ? c - 1 : 0, d = c + 1 < W ? c + 1 : c;
+        const bool e = i0 + 2 * c + 1 < g.nx, both = e && r.no;
+        const bool e2 = both && i0 + 2 * c + 2 < g.nx, n2 = both && r.nn;
+        s[c] = red_residuals<T>(c > 0 || w0, e, r.so, r.no, both, e2, n2, c > 0 ? f.gb.v[b] : f.gw, f.ge.v[c], f.gs.v[c],
+                                f.gn.v[c], f.hw.v[c], f.he.v[c], f.hs.v[c], f.hn.v[c], c > 0 ? x10.v[b] : xw, x10.v[c],
+                                xs.v[c], x01.v[c], c + 1 < W ? x01.v[d] : xe, xn.v[c]);
     }
 }
-// ... stored as coarse b (cells past the row's end left alone).
+// The sums stored as coarse b (cells past the row's end left alone).
 template <class T, int W>
-__device__ __forceinline__ void restrict_wide_store(const LevelView<T>& F, const LevelView<T>& C, unsigned q, int l) {
+__device__ __forceinline__ void store_wide(const LevelView<T>& C, int I, int J, int l, const T (&s)[W]) {
     const Geo& cg = C.g;
-    const unsigned groups = ((unsigned)cg.nx + W - 1u) / W;
-    const int J = (int)(q / groups), I = (int)(q - (unsigned)J * groups) * W;
-    T s[W];
-    restrict_wide<T, W>(F, I, J, l, s);
     T* const row = C.b + (unsigned)l * cg.plane + 2u * (unsigned)J * (unsigned)cg.hx + (unsigned)(I >> 1);
 #pragma unroll
     for (int c = 0; c < W; ++c)
@@ -346,7 +387,7 @@ __device__ __forceinline__ void restrict_cell(const LevelView<T>& F, const Level
                                               int l) {
     const Geo& cg = C.g;
     const int J = (int)(q / (unsigned)cg.nx), I = (int)(q - (unsigned)J * cg.nx);
-    C.b[(unsigned)l * cg.plane + scol(cg, I, J)] = restrict_sum<T, CG>(F, I, J, l);
+    C.b[(unsigned)l * cg.plane + scol(cg, I, J)] = restrict_sum<T, CG>(F, red_faces(F, I, J, l), I, J, l);
 }
 
 
