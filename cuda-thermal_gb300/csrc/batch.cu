@@ -70,6 +70,9 @@ constexpr unsigned kRowChunkDw = 64;
 // Candidate tiles of the autotuner (columns per block for the sweeps, coarse
 // cells per block for the restriction).
 constexpr unsigned kSweepTiles[] = {256, 512, 1024, 2048};
+// ... once more with a block per 32 of a tile's columns, a thread a column and plane
+// (the last candidate).
+constexpr unsigned kSplitTile = 256;
 // ... and tiles per block of the staged sweeps (k_sweep_tma.cu).
 constexpr unsigned kTmaTiles[] = {1, 2, 4, 8};
 constexpr unsigned kRestrictTiles[] = {256, 512, 1024, 2048, 4096};
@@ -480,6 +483,8 @@ ct_status Batch::tune_bucket(Bucket& b) {
     CT_BK(cudaEventCreate(&e0));
     CT_BK(cudaEventCreate(&e1));
     ct_status s = CT_OK;
+    std::vector<unsigned> grid_tiles(std::begin(kSweepTiles), std::end(kSweepTiles));
+    if (b.mz <= 32) grid_tiles.push_back(kSplitTile);
     for (int d = 0; d < b.depth && s == CT_OK; ++d) {
         // staged instances (all of them in mode 1, the fitting ones in mode 2)
         // and grid-swept ones (all in mode 0, the rest in mode 2)
@@ -525,11 +530,13 @@ ct_status Batch::tune_bucket(Bucket& b) {
             if (tma && fixed_tma) cands.push_back(fixed_tma);
             else if (tma) cands.assign(std::begin(kTmaTiles), std::end(kTmaTiles));
             else if (fixed) cands.push_back(fixed);
-            else cands.assign(std::begin(kSweepTiles), std::end(kSweepTiles));
+            else cands = grid_tiles;
             float best = 1e30f;
-            for (unsigned tile : cands) {
+            for (size_t c = 0; c < cands.size(); ++c) {
+                const unsigned tile = cands[c];
                 Plan p;
                 if ((s = upload_plan(make_plan(ni, ins, items, tile), &p)) != CT_OK) break;
+                if (!tma && c >= std::size(kSweepTiles)) p.split = (int)(tile / 32u);
                 CT_BK(cudaStreamSynchronize(st));
                 const float t = cands.size() == 1 ? 0.0f : time_of([&] {
                     if (tma)
@@ -562,10 +569,12 @@ ct_status Batch::tune_bucket(Bucket& b) {
             const float staged = part_best[0] + (ins_g.empty() ? 0.0f : part_best[1]);
             std::vector<unsigned> cands;
             if (fixed) cands.push_back(fixed);
-            else cands.assign(std::begin(kSweepTiles), std::end(kSweepTiles));
-            for (unsigned tile : cands) {
+            else cands = grid_tiles;
+            for (size_t c = 0; c < cands.size(); ++c) {
+                const unsigned tile = cands[c];
                 Plan p;
                 if ((s = upload_plan(make_plan(ni, b.inst, items, tile), &p)) != CT_OK) break;
+                if (c >= std::size(kSweepTiles)) p.split = (int)(tile / 32u);
                 CT_BK(cudaStreamSynchronize(st));
                 const float t = time_of([&] {
                     launch_b_sweep(b.st, p, views[(size_t)d], views[(size_t)d], 1, false, false, b.mz, ctl);
@@ -600,10 +609,12 @@ ct_status Batch::tune_bucket(Bucket& b) {
             });
             std::vector<unsigned> cands;
             if (fixed) cands.push_back(fixed);
-            else cands.assign(std::begin(kSweepTiles), std::end(kSweepTiles));
-            for (unsigned tile : cands) {
+            else cands = grid_tiles;
+            for (size_t c = 0; c < cands.size(); ++c) {
+                const unsigned tile = cands[c];
                 Plan p;
                 if ((s = upload_plan(make_plan(ni, b.inst, items, tile), &p)) != CT_OK) break;
+                if (c >= std::size(kSweepTiles)) p.split = (int)(tile / 32u);
                 CT_BK(cudaStreamSynchronize(st));
                 const float t = time_of([&] {
                     launch_b_sweep(b.st, p, views[(size_t)d], views[(size_t)d], 0, true, false, b.mz, ctl);

@@ -28,6 +28,7 @@ struct Plan {
     int ntasks;
     const int* inst_first;  // per instance: first block of the instance (reducing stages)
     const int* inst_count;  // per instance: number of its blocks (0 = not in this stage)
+    int split;              // > 0: that many blocks a task, 32 columns each, a thread a column and plane (grid sweeps)
 };
 
 // One instance's fine-level arrays (split layout). The double-word mode

@@ -356,6 +356,31 @@ __global__ void __launch_bounds__(NT)
         sweep_column<float, MZ, ZERO, PRO, false>(L, C, color, q);
 }
 
+// The same with one thread per column and plane (split_columns), 32 columns a block:
+// the small levels, where a thread's nz planes of loads are the launch (48 stacks,
+// the second to fifth level: 25, 15, 11, 8 us a launch against 32, 18, 17, 16 with a
+// thread a column). The tuner times it beside the other forms.
+template <int MZ, bool ZERO, bool PRO>
+__global__ void __launch_bounds__(32 * MZ)
+    kb_sweep_split(Plan p, const LevelView<float>* __restrict__ views, const LevelView<float>* __restrict__ cviews,
+                   int color, const Ctl* ctl) {
+    __shared__ SplitShared<float, MZ> S;
+    const unsigned task = blockIdx.x / (unsigned)p.split;
+    const Task t = p.tasks[task];
+    const unsigned q = t.begin + (blockIdx.x - task * (unsigned)p.split) * 32u;
+    if (q >= t.end) return;
+    const LevelView<float> L = views[t.inst];
+    const LevelView<float> C = PRO ? cviews[t.inst] : L;
+    split_columns<float, MZ, ZERO, PRO>(
+        L, C, color, q + threadIdx.x, t.end, S,
+        [&] {
+            pdl_enter();
+            pdl_trigger();
+            return *(volatile const int*)&ctl[t.inst].done;
+        },
+        [](int done) { return done != 0; });
+}
+
 // Coarse cells of one instance, kRestrictWide a thread; compiled for 4 blocks per SM
 // (48 stacks, the finest level: 28.9 us a launch against 34.1 with the compiler's own
 // choice).
@@ -440,6 +465,28 @@ void launch_b_rhs_transient(cudaStream_t st, const Plan& p, const BInst* bi, con
 void launch_b_sweep(cudaStream_t st, const Plan& p, const LevelView<float>* views,
                     const LevelView<float>* cviews, int color, bool zero_x, bool prolong, int mz,
                     const Ctl* ctl) {
+#define CT_BSPLIT(MZ)                                                                                        \
+    do {                                                                                                     \
+        const dim3 block(32, (unsigned)mz);                                                                  \
+        if (zero_x)                                                                                          \
+            launch_pdl(kb_sweep_split<MZ, true, false>, p.ntasks * p.split, block, 0, st, p, views, cviews, color, ctl);  \
+        else if (prolong)                                                                                    \
+            launch_pdl(kb_sweep_split<MZ, false, true>, p.ntasks * p.split, block, 0, st, p, views, cviews, color, ctl);  \
+        else                                                                                                 \
+            launch_pdl(kb_sweep_split<MZ, false, false>, p.ntasks * p.split, block, 0, st, p, views, cviews, color, ctl); \
+    } while (0)
+    if (p.split) {  // (at most 32 planes)
+        if (mz <= 8)
+            CT_BSPLIT(8);
+        else if (mz <= 12)
+            CT_BSPLIT(12);
+        else if (mz <= 16)
+            CT_BSPLIT(16);
+        else
+            CT_BSPLIT(32);
+        return;
+    }
+#undef CT_BSPLIT
 #define CT_BSWEEP(MZ)                                                                          \
     do {                                                                                       \
         if (zero_x)                                                                            \

@@ -124,129 +124,19 @@ __global__ void __launch_bounds__(NT, (ZERO && sizeof(T) == 4 && MZ > 0 && MZ <=
     sweep_column<T, MZ, ZERO, PRO, false>(L, C, color, q);
 }
 
-// Sweep of a small level (L2-resident, latency-bound) with one thread per
-// column and plane: a block is 32 columns of the active colour x nz planes.
-// Each thread gathers its plane's right-hand side (b plus lat_sum, the same
-// operations as sweep_column) and the column's factors into shared memory;
-// after one block barrier, one thread per column runs sweep_column's
-// recurrence there, and after a second the block writes x plane by plane.
-// Same operations in the same order as k_sweep, so the same bits, but a
-// thread issues one plane's loads instead of nz planes' (k_sweep: 6.5-7.8 us
-// per launch on the 100 x 100 to 25 x 25 levels of an 800 x 800 stack).
+// Sweep of a small level, a block per 32 columns (split_columns).
 template <class T, int MZ, bool ZERO, bool PRO>
 __global__ void __launch_bounds__(32 * MZ)
     k_sweep_split(LevelView<T> L, int color, LevelView<T> C, const Ctl* ctl, Cond cond) {
-    __shared__ T sv[MZ][32], sfi[MZ][32], sfc[MZ][32];
-    __shared__ float sgu[MZ][32];
-    const Geo& g = L.g;
-    const unsigned tx = threadIdx.x;
-    const int l = (int)threadIdx.y;
-    const unsigned q = blockIdx.x * 32u + tx;
-    const int j = (int)(q / (unsigned)g.hx), t = (int)(q - (unsigned)j * g.hx);
-    const int i = 2 * t + ((j + color) & 1);
-    const bool on = q < (unsigned)g.ny * (unsigned)g.hx && i < g.nx;
-    const Nbr n = neighbours<PRO>(g, C.g, i, j, t, color);
-    const unsigned s = n.s, base = (unsigned)l * g.plane, id = base + s;
-    T rhs = 0, fi = 0, fc = 0;
-    float gu = 0.0f, gw = 0.0f, ge = 0.0f, gs = 0.0f, gn = 0.0f;
-    // before the wait for the preceding kernel (kernels.h): the operator and the
-    // factors, on the way up b, and ahead of the prolongation x as well
-    const bool b_early = PRO || (!ZERO && color == 0);
-    T xw = 0, xe = 0, xs = 0, xn = 0;
-    auto load_x = [&] {
-        if (n.w) xw = L.x[base + n.sw];
-        if (n.e) xe = L.x[base + n.se];
-        if (n.so) xs = L.x[base + n.ss];
-        if (n.no) xn = L.x[base + n.sn];
-    };
-    if (on) {
-        fi = L.finv[id];
-        gu = L.gU[id];
-        if (!ZERO) {
-            fc = L.fcp[id];
-            if (n.w) gw = L.gE[base + n.sw];
-            ge = L.gE[id];
-            if (n.so) gs = L.gN[base + n.ss];
-            gn = L.gN[id];
-        }
-        if (b_early) rhs = L.b[id];
-        if (PRO) load_x();
-    }
-    pdl_enter();
-    pdl_trigger();
-    const int2 flags = loop_flags(ctl);  // tested after the gathers are issued
-    if (on) {
-        if (!b_early) rhs = L.b[id];
-        if (!ZERO) {
-            if (PRO) {
-                const T* const cx = C.x + (unsigned)l * C.g.plane;
-                if (n.w) xw = xw + cx[n.pw];
-                if (n.e) xe = xe + cx[n.pe];
-                if (n.so) xs = xs + cx[n.ps];
-                if (n.no) xn = xn + cx[n.pn];
-            } else {
-                load_x();
-            }
-            T sum = 0;  // lat_sum's order
-            if (n.w) sum += face<T>(gw) * xw;
-            if (n.e) sum += face<T>(ge) * xe;
-            if (n.so) sum += face<T>(gs) * xs;
-            if (n.no) sum += face<T>(gn) * xn;
-            rhs = rhs + sum;
-        } else {
-            fc = fcp_of(gu, fi);  // as factor_column rounded it (one operand stream less)
-        }
-    }
-    if (loop_done(flags, cond)) return;  // the same for every thread of the grid
-    if (on) {
-        sv[l][tx] = rhs;
-        sfi[l][tx] = fi;
-        sfc[l][tx] = fc;
-        sgu[l][tx] = gu;
-    }
-    __syncthreads();
-    const int nz = g.nz;
-    if (on && l == 0) {
-        // the recurrence of sweep_column, on shared memory; FP32 up to 16 planes
-        // on registers, all MZ planes without a test (the ones past nz hold
-        // nothing and reach nothing): one warp runs it while the block waits, so
-        // its instruction count is the kernel's time. 237 x 181 x 10: an
-        // iteration of 105.2 us against 109.4 with the loop over shared memory;
-        // 501 x 333 x 10: 167.1 against 169.8
-        if constexpr (sizeof(T) == 4 && MZ <= 16) {
-            T v[MZ], c[MZ], prev = 0, lower = 0;
-#pragma unroll
-            for (int k = 0; k < MZ; ++k) {
-                prev = (sv[k][tx] - lower * prev) * sfi[k][tx];
-                v[k] = prev;
-                c[k] = sfc[k][tx];
-                lower = -sgu[k][tx];
-            }
-#pragma unroll
-            for (int k = MZ - 2; k >= 0; --k) {
-                const T n = v[k] - c[k] * v[k + 1];
-                v[k] = k < nz - 1 ? n : v[k];
-            }
-#pragma unroll
-            for (int k = 0; k < MZ; ++k)
-                if (k < nz) sv[k][tx] = v[k];
-        } else {
-            T prev = 0;
-#pragma unroll 4
-            for (int k = 0; k < nz; ++k) {
-                const T lower = k > 0 ? -face<T>(sgu[k - 1][tx]) : T(0);
-                prev = (sv[k][tx] - lower * prev) * sfi[k][tx];
-                sv[k][tx] = prev;
-            }
-#pragma unroll 4
-            for (int k = nz - 2; k >= 0; --k) {
-                prev = sv[k][tx] - sfc[k][tx] * prev;
-                sv[k][tx] = prev;
-            }
-        }
-    }
-    __syncthreads();
-    if (on) L.x[(unsigned)l * g.plane + s] = sv[l][tx];
+    __shared__ SplitShared<T, MZ> S;
+    split_columns<T, MZ, ZERO, PRO>(
+        L, C, color, blockIdx.x * 32u + threadIdx.x, (unsigned)L.g.ny * (unsigned)L.g.hx, S,
+        [&] {
+            pdl_enter();
+            pdl_trigger();
+            return loop_flags(ctl);
+        },
+        [&](int2 flags) { return loop_done(flags, cond); });
 }
 
 // Restriction F -> C, one thread per coarse cell and plane (blockIdx.y is the
