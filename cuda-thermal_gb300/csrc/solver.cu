@@ -120,8 +120,8 @@ ct_status Solver::create(const ct_model* m_in, ct_precond pc_, ct_precision prec
         CT_CK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
     }
     cs = st;
-    CT_CK(cudaMallocHost(&h_ctl, sizeof(Ctl)));
-    std::memset(h_ctl, 0, sizeof(Ctl));
+    h_ctl = std::make_unique<Ctl>();
+    std::memset(h_ctl.get(), 0, sizeof(Ctl));
 
     // Level sizes (src/mg3d.h:159-181) and the arena layout.
     Arena ar;
@@ -668,7 +668,7 @@ ct_status Solver::solve(double tol, int maxit, ct_stats* out) {
     c.x_zero = x_zero ? 1 : 0;
     x_zero = false;
     *h_ctl = c;
-    CT_CK(cudaMemcpyAsync(ctl, h_ctl, sizeof(Ctl), cudaMemcpyHostToDevice, st));
+    CT_CK(cudaMemcpyAsync(ctl, h_ctl.get(), sizeof(Ctl), cudaMemcpyHostToDevice, st));
     const Cond none{0, 0};
     cs = st;
     if (have_cond && !prof) {
@@ -685,7 +685,7 @@ ct_status Solver::solve(double tol, int maxit, ct_stats* out) {
             enqueue_init(none);
         int launched = 0, k = graphs ? 2 : 1;
         while (true) {
-            CT_CK(cudaMemcpyAsync(h_ctl, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
+            CT_CK(cudaMemcpyAsync(h_ctl.get(), ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
             CT_CK(cudaStreamSynchronize(st));
             if (h_ctl->done || launched > maxit + 2) break;
             if (h_ctl->phase_end) {
@@ -809,7 +809,7 @@ ct_status Solver::copies_wait() {
 }
 
 ct_status Solver::finish_solve(ct_stats* out) {
-    CT_CK(cudaMemcpyAsync(h_ctl, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
+    CT_CK(cudaMemcpyAsync(h_ctl.get(), ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
     CT_CK(cudaStreamSynchronize(st));
     if (h_ctl->bb_zero) {  // no heat in: x = 0 (src/pcg3d_cpu.cpp:146)
         CT_CK(cudaMemsetAsync(x, 0, (size_t)n * 8, st));
@@ -1117,7 +1117,7 @@ ct_status ct_true_relres(ct_solver* s, double* out) {
     ct::Solver& v = s->impl;
     ct::launch_true_residual(v.st, v.op(), v.P, v.x_as_double(nullptr), v.ctl, v.red_cols(ct::SL_AUX));
     CT_CUDA(cudaGetLastError());
-    CT_CUDA(cudaMemcpyAsync(v.h_ctl, v.ctl, sizeof(ct::Ctl), cudaMemcpyDeviceToHost, v.st));
+    CT_CUDA(cudaMemcpyAsync(v.h_ctl.get(), v.ctl, sizeof(ct::Ctl), cudaMemcpyDeviceToHost, v.st));
     CT_CUDA(cudaStreamSynchronize(v.st));
     *out = std::sqrt(v.h_ctl->aux0 / v.h_ctl->aux1);
     return CT_OK;
@@ -1129,7 +1129,7 @@ ct_status ct_solver_step_record(ct_solver* s, double dt, ct_step_record* out) {
     ct::Solver& v = s->impl;
     ct::launch_step_record(v.st, v.op(), v.x_as_double(nullptr), v.xold, v.ctl, v.red_cols(ct::SL_AUX));
     CT_CUDA(cudaGetLastError());
-    CT_CUDA(cudaMemcpyAsync(v.h_ctl, v.ctl, sizeof(ct::Ctl), cudaMemcpyDeviceToHost, v.st));
+    CT_CUDA(cudaMemcpyAsync(v.h_ctl.get(), v.ctl, sizeof(ct::Ctl), cudaMemcpyDeviceToHost, v.st));
     CT_CUDA(cudaStreamSynchronize(v.st));
     out->T_max = v.h_ctl->aux0;
     out->q_out = v.h_ctl->aux1;

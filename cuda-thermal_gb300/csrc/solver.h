@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <string>
+#include <memory>
 #include <vector>
 
 #include "build.h"
@@ -77,7 +78,10 @@ class Solver {
     float2* dgw = nullptr;  // double-word diagonal (dw)
     float2* xwc = nullptr;  // double-word correction of x (dw); x is then its FP64 base
     Ctl* ctl = nullptr;
-    Ctl* h_ctl = nullptr;  // pinned mirror
+    // host mirror of the control block, in pageable memory: pinning and unpinning a
+    // page cost 0.12 + 0.19 ms of a 2 ms one-call solve, and a copy of 250 bytes to
+    // pageable memory 1.7 us more than to pinned (10.4 against 8.7)
+    std::unique_ptr<Ctl> h_ctl;
     std::vector<Level> lv;
     int maxb = 0;
     double inv_dt = 0;
@@ -136,7 +140,6 @@ class Solver {
             if (g) cudaGraphExecDestroy(g);
         if (base) cudaFree(base);
         if (rec_table) cudaFree(rec_table);
-        if (h_ctl) cudaFreeHost(h_ctl);
         for (int i = 0; i < 2; ++i) {
             for (cudaEvent_t e : {ev_in_copied[i], ev_in_used[i], ev_out_ready[i], ev_out_copied[i]})
                 if (e) cudaEventDestroy(e);
