@@ -159,12 +159,20 @@ __device__ __forceinline__ void gather_acc(const double* part, int stride, unsig
     DwAcc a[N];
 #pragma unroll
     for (int q = 0; q < N; ++q) a[q] = DwAcc{0.0f, 0.0f};
-    for (unsigned k = threadIdx.x; k < count; k += NT) {
+    // four slots' loads in flight, as gather_sums
+    for (unsigned k0 = threadIdx.x; k0 < count; k0 += 4 * NT) {
+        float2 p[4][N];
 #pragma unroll
-        for (int q = 0; q < N; ++q) {
-            const float2 u = __ldcg(pp + (size_t)q * stride + first + k);
-            acc_add(a[q], u.x, u.y);
-        }
+        for (unsigned u = 0; u < 4; ++u)
+#pragma unroll
+            for (int q = 0; q < N; ++q)
+                p[u][q] = k0 + u * NT < count ? __ldcg(pp + (size_t)q * stride + first + k0 + u * NT)
+                                              : make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (unsigned u = 0; u < 4; ++u)
+            if (k0 + u * NT < count)
+#pragma unroll
+                for (int q = 0; q < N; ++q) acc_add(a[q], p[u][q].x, p[u][q].y);
     }
     block_sum_acc<N>(a);
     if (threadIdx.x == 0) {

@@ -127,9 +127,21 @@ __device__ __forceinline__ void gather_sums(const double* part, int stride, unsi
     double v[N];
 #pragma unroll
     for (int q = 0; q < N; ++q) v[q] = 0.0;
-    for (unsigned k = threadIdx.x; k < count; k += NT)
+    // four slots' loads in flight (up to 4 NT blocks: one round trip to L2; 237 x 181
+    // x 13, with 588 blocks in A z: 94.7 us an iteration against 95.5)
+    for (unsigned k0 = threadIdx.x; k0 < count; k0 += 4 * NT) {
+        double p[4][N];
 #pragma unroll
-        for (int q = 0; q < N; ++q) v[q] += __ldcg(part + (size_t)q * stride + first + k);
+        for (unsigned u = 0; u < 4; ++u)
+#pragma unroll
+            for (int q = 0; q < N; ++q)
+                p[u][q] = k0 + u * NT < count ? __ldcg(part + (size_t)q * stride + first + k0 + u * NT) : 0.0;
+#pragma unroll
+        for (unsigned u = 0; u < 4; ++u)
+            if (k0 + u * NT < count)
+#pragma unroll
+                for (int q = 0; q < N; ++q) v[q] += p[u][q];
+    }
     const double a = block_sums<N>(v);
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (w < N && lane == 0) t[w] = a;
