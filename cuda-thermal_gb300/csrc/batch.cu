@@ -58,7 +58,7 @@ namespace {
     } while (0)
 
 // Items per block of the stages whose tile is not tuned.
-constexpr unsigned kVecChunk = 4096;   // value pairs (fold, update, dot, p, rhs)
+constexpr unsigned kVecChunk = 4096;   // value pairs (fold, step, rhs)
 // fine rows of one colour and plane per block of the operator apply: the
 // FP64 apply is FP64-pipe-bound, and per-block reduction overhead weighs less
 // on longer tables (256 instances, two cells per lane: 16 / 32 / 64 / 128 rows

@@ -245,7 +245,8 @@ __global__ void __launch_bounds__(NT)
     }
 }
 
-// Pairs of values: b = P + C/dt x (x = FP64 base, folded), x_old = x.
+// Pairs of values: b = P + C/dt x (x = FP64 base, folded), x_old = x; conversions
+// on the integer pipe, as in set_dt (f64_dev.cuh).
 __global__ void __launch_bounds__(NT)
     kb_rhs_transient(Plan p, const BInst* __restrict__ bi, const Ctl* ctl) {
     const Task t = p.tasks[blockIdx.x];
@@ -259,8 +260,8 @@ __global__ void __launch_bounds__(NT)
     for (unsigned k = t.begin + threadIdx.x; k < t.end; k += NT) {
         const double2 xv = x[k], pv = P[k];
         const float2 cv = cap[k];
-        b[k] = make_double2(__dadd_rn(pv.x, __dmul_rn(__dmul_rn((double)cv.x, inv_dt), xv.x)),
-                            __dadd_rn(pv.y, __dmul_rn(__dmul_rn((double)cv.y, inv_dt), xv.y)));
+        b[k] = make_double2(__dadd_rn(pv.x, __dmul_rn(__dmul_rn(widen(cv.x), inv_dt), xv.x)),
+                            __dadd_rn(pv.y, __dmul_rn(__dmul_rn(widen(cv.y), inv_dt), xv.y)));
         xold[k] = xv;
     }
 }

@@ -1,6 +1,6 @@
 // k_fp64.cu - the FP64 outer PCG of the multigrid modes (CT_MG_FP32_FLEX,
-// CT_MG_FP32, CT_MG_FP64): residual, operator apply, x/r update, dot
-// products and p update, all in IEEE double arithmetic as the reference's
+// CT_MG_FP32, CT_MG_FP64): residual, A z with the dot products, the step of p,
+// Ap and r, and the x update, all in IEEE double arithmetic as the reference's
 // outer iteration is (Real = double, src/pcg3d.h:18-22; k_residual,
 // k_apply, k_update_xr, k_mg_dot, k_update_p_mg, src/pcg3d_gpu.cu:159-256).
 //
@@ -51,8 +51,8 @@ constexpr int kRowU = 2;  // cells a lane and step of the rows of A p
 // 82 us a launch (105 compiled for two cells a lane
 // and the compiler's 101 registers, 94 / 82 / 87 for one cell at 2 / 5 / 6 blocks
 // per SM against 4; the next cells' loads ahead of this one's arithmetic 84 to
-// 98), against 107 + 37 for A p and the dots; the FP64 pipe is 60 % busy, memory
-// 44 %, issue 57 %, each warp going from one to the other.
+// 98), against 107 + 37 for A p and the dots; the FP64 pipe is 62 % busy, memory
+// 43 %, issue 64 %, each warp going from one to the other.
 template <class T, bool FLEX>
 __global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 3 : 4)
     k_az64(OpView o, const double* __restrict__ diag, const T* __restrict__ z, const double* __restrict__ r,
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(NT)
 // beside the next V-cycle); alpha is kept in ctl->alpha_x for it. The x update
 // that was pending at entry has run by then: none is pending when the loop has
 // ended.
-// 4 FP64 instructions and 60 B a cell. 800 x 800 x 10: 73 us (5.6 TB/s), against
+// 4 FP64 instructions and 64 B a cell. 800 x 800 x 10: 73 us (5.6 TB/s), against
 // 22 + 37 for the p update and the update of r alone.
 template <class T>
 struct Pair;

@@ -81,9 +81,9 @@ __global__ void k_coarsen(Geo fg, const float* __restrict__ fgE, const float* __
         for (int j = j0; j <= j1; ++j)
             for (int i = i0; i <= i1; ++i) {
                 const unsigned fs = scol(fg, i, j);
-                gu = __dadd_rn(gu, (double)fgU[fb + fs]);
-                cp = __dadd_rn(cp, (double)fcap[fb + fs]);
-                if (l == 0) gb = __dadd_rn(gb, (double)fgB[fs]);
+                gu = __dadd_rn(gu, f64dev::widen(fgU[fb + fs]));
+                cp = __dadd_rn(cp, f64dev::widen(fcap[fb + fs]));
+                if (l == 0) gb = __dadd_rn(gb, f64dev::widen(fgB[fs]));
             }
         const unsigned cs = scol(cg, I, J);
         cgU[cb + cs] = __double2float_rn(gu);
@@ -92,14 +92,14 @@ __global__ void k_coarsen(Geo fg, const float* __restrict__ fgE, const float* __
         float e = 0.0f, nn = 0.0f;
         if (I < cg.nx - 1) {  // fine faces between columns 2I+1 and 2I+2
             double sum = 0;
-            for (int j = j0; j <= j1; ++j) sum = __dadd_rn(sum, (double)fgE[fb + scol(fg, 2 * I + 1, j)]);
+            for (int j = j0; j <= j1; ++j) sum = __dadd_rn(sum, f64dev::widen(fgE[fb + scol(fg, 2 * I + 1, j)]));
             const double df = __dmul_rn(0.5, __dadd_rn(fdx[2 * I + 1], fdx[2 * I + 2]));
             const double dc = __dmul_rn(0.5, __dadd_rn(cdx[I], cdx[I + 1]));
             e = __double2float_rn(__ddiv_rn(__dmul_rn(sum, df), dc));
         }
         if (J < cg.ny - 1) {  // fine faces between rows 2J+1 and 2J+2
             double sum = 0;
-            for (int i = i0; i <= i1; ++i) sum = __dadd_rn(sum, (double)fgN[fb + scol(fg, i, 2 * J + 1)]);
+            for (int i = i0; i <= i1; ++i) sum = __dadd_rn(sum, f64dev::widen(fgN[fb + scol(fg, i, 2 * J + 1)]));
             const double df = __dmul_rn(0.5, __dadd_rn(fdy[2 * J + 1], fdy[2 * J + 2]));
             const double dc = __dmul_rn(0.5, __dadd_rn(cdy[J], cdy[J + 1]));
             nn = __double2float_rn(__ddiv_rn(__dmul_rn(sum, df), dc));

@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstdlib>
 
+#include "f64_dev.cuh"
 #include "kernels.h"
 #include "tma.cuh"
 #include "reduce.cuh"
@@ -304,7 +305,7 @@ __global__ void k_rhs_transient(unsigned n, const float* __restrict__ cap, doubl
     for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const double xv = x[k];
         // b = P + C/dt x, rounded as the reference rounds it (src/pcg3d_cpu.cpp:64)
-        b[k] = __dadd_rn(P[k], __dmul_rn(__dmul_rn((double)cap[k], inv_dt), xv));
+        b[k] = __dadd_rn(P[k], __dmul_rn(__dmul_rn(f64dev::widen(cap[k]), inv_dt), xv));
         xold[k] = xv;
     }
 }
@@ -375,11 +376,12 @@ __global__ void __launch_bounds__(NT)
     for (unsigned s = blockIdx.x * NT + threadIdx.x; s < g.plane; s += gridDim.x * NT) {
         const Col c = col_of_slot(g, s);
         if (!c.valid) continue;
+#pragma unroll 4
         for (int l = 0; l < g.nz; ++l) {
             const unsigned id = (unsigned)l * g.plane + s;
             const double xv = x[id];
             tmax = fmax(tmax, xv);
-            qst += (double)o.cap[id] * (xv - xold[id]);
+            qst += f64dev::widen(o.cap[id]) * (xv - xold[id]);
         }
         const unsigned top = (unsigned)(g.nz - 1) * g.plane + s;
         qout += (double)o.gU[top] * x[top];

@@ -77,6 +77,7 @@ __device__ __forceinline__ void factor_column(const LevelView<T>& L, T inv_dt, u
 // the fine operator in FP64 — west, east, south, north, up, down or bottom
 // sink, summed in that order — which does not change with dt.
 __device__ __forceinline__ void faces_column(const OpView& o, unsigned q, double* __restrict__ dface) {
+    using f64dev::widen;
     const Geo& g = o.g;
     const int j = (int)(q / (unsigned)g.nx), i = (int)(q - (unsigned)j * g.nx);
     const unsigned s = scol(g, i, j);
@@ -84,12 +85,12 @@ __device__ __forceinline__ void faces_column(const OpView& o, unsigned q, double
     for (int l = 0; l < g.nz; ++l) {
         const unsigned base = (unsigned)l * g.plane, id = base + s;
         double d = 0.0;
-        if (i > 0) d = __dadd_rn(d, (double)o.gE[base + scol(g, i - 1, j)]);
-        if (i < g.nx - 1) d = __dadd_rn(d, (double)o.gE[id]);
-        if (j > 0) d = __dadd_rn(d, (double)o.gN[base + scol(g, i, j - 1)]);
-        if (j < g.ny - 1) d = __dadd_rn(d, (double)o.gN[id]);
-        d = __dadd_rn(d, (double)o.gU[id]);
-        d = __dadd_rn(d, l > 0 ? (double)o.gU[id - g.plane] : (double)o.gB[s]);
+        if (i > 0) d = __dadd_rn(d, widen(o.gE[base + scol(g, i - 1, j)]));
+        if (i < g.nx - 1) d = __dadd_rn(d, widen(o.gE[id]));
+        if (j > 0) d = __dadd_rn(d, widen(o.gN[base + scol(g, i, j - 1)]));
+        if (j < g.ny - 1) d = __dadd_rn(d, widen(o.gN[id]));
+        d = __dadd_rn(d, widen(o.gU[id]));
+        d = __dadd_rn(d, l > 0 ? widen(o.gU[id - g.plane]) : widen(o.gB[s]));
         dface[id] = d;
     }
 }
@@ -98,9 +99,13 @@ __device__ __forceinline__ void faces_column(const OpView& o, unsigned q, double
 // sum plus C/dt, the last term of op_diag's sum, so the same bits as summing
 // it all here (and 1/d for Jacobi, the double-word copy for the double-word
 // mode, where requested).
+// Conversions by integer operations here and in faces_column and k_coarsen: at the
+// FP64 rate they were half of these kernels (800 x 800 x 10: coarse operators 0.35 ->
+// 0.26 ms, faces and factors 0.23 -> 0.17; a step of 16 stacks 4.78 -> 4.70).
 __device__ __forceinline__ void diag_column(const OpView& o, const double* __restrict__ dface, double inv_dt,
                                             unsigned q, double* __restrict__ diag, double* __restrict__ invd,
                                             float2* __restrict__ dgw) {
+    using f64dev::widen;
     const Geo& g = o.g;
     const int j = (int)(q / (unsigned)g.nx), i = (int)(q - (unsigned)j * g.nx);
     const unsigned s = scol(g, i, j);
@@ -108,12 +113,11 @@ __device__ __forceinline__ void diag_column(const OpView& o, const double* __res
 #pragma unroll 4
     for (int l = 0; l < g.nz; ++l) {
         const unsigned id = (unsigned)l * g.plane + s;
-        const double d = __dadd_rn(dface[id], __dmul_rn((double)cap[id], inv_dt));
+        const double d = __dadd_rn(dface[id], __dmul_rn(widen(cap[id]), inv_dt));
         diag[id] = d;
         if (invd) invd[id] = __drcp_rn(d);
         if (dgw) {
-            const float h = __double2float_rn(d);
-            dgw[id] = make_float2(h, __double2float_rn(d - (double)h));
+            dgw[id] = f64dev::split(d);
         }
     }
 }

@@ -454,8 +454,9 @@ void Solver::vcycle(size_t k, Cond cond, bool first_sweep_done) {
     // The coarse level's first sweep rides along with the restriction unless
     // the shared-memory bottom starts there,
     // or the restriction is from the finest level: there it is bandwidth
-    // bound, and the block's serial line-solve tail costs more (measured at
-    // 800 x 800: 78 us fused against 51 + 13 us) than the launch it saves.
+    // bound, and the block's serial line-solve tail costs about the launch it
+    // saves (an iteration fused: 501 x 333 - 1.4 %, 800 x 800 - 0.2 %, 1024 x
+    // 1024 + 0.5 %, FP64 400 x 400 + 4 %).
     const bool fuse = fuse_sweep0 && k > 0 && k + 1 != small_k0 && L.g.nz <= 32;
     const double b_restrict = cells * (t / 2 + 8) + cells / 4 * t;
     const double cc = (double)C.g.nx * C.g.ny * C.g.nz;
