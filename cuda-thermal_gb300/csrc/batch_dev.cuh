@@ -17,14 +17,14 @@ __device__ __forceinline__ void inst_stop(Ctl* c, BCtl* bc, const Cond& cond) {
     if (atomicSub(&bc->active, 1) == 1 && cond.use) cudaGraphSetConditional(cond.h, 0u);
 }
 
-// The block's (a, b) go to its slot of the stage; true in the instance's
-// last block.
+// The block's (a, b) of a task go to its slot of the stage; true in the block of
+// the instance's last task.
 __device__ __forceinline__ bool publish_inst(double a, double b, const BRed& red, int ntasks,
-                                             int inst, int count) {
+                                             int inst, int count, int task) {
     __shared__ int last;
     if (threadIdx.x == 0) {
-        red.part[blockIdx.x] = a;
-        red.part[ntasks + blockIdx.x] = b;
+        red.part[task] = a;
+        red.part[ntasks + task] = b;
         __threadfence();
         const unsigned t = atomicAdd(&red.tickets[inst], 1u);
         last = (t == (unsigned)count - 1u) ? 1 : 0;

@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(NT)
     }
     if (zero) rr = bb;
     block_sum2(rr, bb);
-    if (publish_inst(rr, bb, red, p.ntasks, t.inst, p.inst_count[t.inst])) {
+    if (publish_inst(rr, bb, red, p.ntasks, t.inst, p.inst_count[t.inst], (int)blockIdx.x)) {
         double RR, BB;
         gather_inst(red, p.ntasks, t.inst, p.inst_first[t.inst], p.inst_count[t.inst], RR, BB);
         if (threadIdx.x == 0) {
