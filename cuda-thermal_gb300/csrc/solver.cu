@@ -576,6 +576,14 @@ ct_status Solver::record_graphs() {
               cudaGraphConditionalHandleCreate(&h1, graph, 1u, cudaGraphCondAssignDefault) == cudaSuccess;
     if (ok && dw)
         ok = cudaGraphConditionalHandleCreate(&h2, graph, 1u, cudaGraphCondAssignDefault) == cudaSuccess;
+    // Iterations in the loop's body. A body costs 5 us beside its kernels; a body whose
+    // loop has ended before it is through, the entries of the kernels left. Where the
+    // cluster holds the whole V-cycle those are three launches an iteration, and four
+    // iterations a body pay (16 x 16 x 10: 11 iterations 429 -> 374 us a solve, 395 with
+    // two; 64 x 64 x 10: 12 in 602 -> 553, 570; 3 to 6 of a transient 245 -> 244 at
+    // worst), two in the double-word mode's two loops. Elsewhere one does: 400 x 400 x 10
+    // in FP64 307 us an iteration, 313 with two.
+    const int per_body = small_k0 == 0 && tail.n > 0 ? (dw ? 2 : 4) : 1;
     // Adds a WHILE node after the captured work so far and captures its body.
     auto add_while = [&](cudaGraphConditionalHandle h) -> bool {
         cudaStreamCaptureStatus cst;
@@ -595,7 +603,7 @@ ct_status Solver::record_graphs() {
                                           cudaStreamCaptureModeThreadLocal) != cudaSuccess)
             return false;
         cs = st_body;
-        enqueue_body(Cond{h, 1});
+        for (int u = 0; u < per_body; ++u) enqueue_body(Cond{h, 1});
         cs = st;
         cudaGraph_t bg = nullptr;
         if (cudaStreamEndCapture(st_body, &bg) != cudaSuccess) return false;
