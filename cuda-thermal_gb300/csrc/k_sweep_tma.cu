@@ -101,7 +101,8 @@ __device__ __forceinline__ void issue_plane(const SweepMaps* m, float* sm, uint6
 // have arrived. No block-wide barrier inside the loop, so warps drift apart
 // and cover one another's waits. A wait that runs out raises `abort`, which
 // ends every other wait.
-template <int TT, int TJ, int NS, int MZ, bool ZERO, bool PRO>
+// MAPS_GLOBAL: the maps lie in global memory (tma.cuh, acquire_map).
+template <int TT, int TJ, int NS, int MZ, bool ZERO, bool PRO, bool MAPS_GLOBAL>
 __device__ __forceinline__ bool sweep_tiles_ws(const SweepMaps* m, const LevelView<float>& L,
                                                const LevelView<float>& C, int color,
                                                const TileList& tl, float* sm, uint64_t* full,
@@ -126,6 +127,18 @@ __device__ __forceinline__ bool sweep_tiles_ws(const SweepMaps* m, const LevelVi
     __syncthreads();
     if (warp == TJ) {  // producer
         if (lane == 0) {
+            if (MAPS_GLOBAL) {
+                acquire_map(&m->b);
+                acquire_map(&m->fi);
+                acquire_map(&m->gu);
+                if (!ZERO) {
+                    acquire_map(&m->ge);
+                    acquire_map(&m->gn);
+                    acquire_map(&m->ox);
+                    acquire_map(&m->oge);
+                    acquire_map(&m->ogn);
+                }
+            }
             for (int w = 0; w < nitems; ++w) {
                 const int s = w % NS;
                 if (w >= NS && !mbar_wait_or_abort(&empty[s], (unsigned)(w / NS - 1) & 1u, abort)) break;
@@ -260,7 +273,7 @@ __global__ void __launch_bounds__(TT * TJ + 32, MZ <= 16 ? kSweepWsBlocks : 2)
     const int ntiles = ((g.hx + TT - 1) / TT) * ((g.ny + TJ - 1) / TJ);
     const int count = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     const TileList tl{(int)blockIdx.x, (int)gridDim.x, count};
-    if (!sweep_tiles_ws<TT, TJ, NS, MZ, ZERO, PRO>(&m, L, C, color, tl, sm, full, empty, &flags[0],
+    if (!sweep_tiles_ws<TT, TJ, NS, MZ, ZERO, PRO, false>(&m, L, C, color, tl, sm, full, empty, &flags[0],
                                                      &flags[1]) &&
         threadIdx.x == 0)
         fail_wait(ctl, cond);
@@ -282,7 +295,7 @@ __global__ void __launch_bounds__(TT * TJ + 32, MZ <= 16 ? kSweepWsBlocks : 2)
     const LevelView<float> L = views[t.inst];
     const LevelView<float> C = PRO ? cviews[t.inst] : L;
     const TileList tl{(int)t.begin, 1, (int)(t.end - t.begin)};
-    if (!sweep_tiles_ws<TT, TJ, NS, MZ, ZERO, PRO>(&maps[t.inst], L, C, color, tl, sm, full, empty, &flags[0],
+    if (!sweep_tiles_ws<TT, TJ, NS, MZ, ZERO, PRO, true>(&maps[t.inst], L, C, color, tl, sm, full, empty, &flags[0],
                                                    &flags[1]) &&
         threadIdx.x == 0) {
         atomicExch(&c->err, 1);

@@ -318,9 +318,10 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
             const int dst = arr == 0 ? L.fi : arr == 1 ? L.gu : arr == 2 ? L.ge : L.gn;
             uint64_t* const bar = arr < 2 && k == k_lo ? bar0 : bar1;
             const int j0 = rank * L.rows;
-            if (k < nd)
+            if (k < nd) {
+                tma::acquire_map(&maps[k].m[arr]);
                 tma::load_3d(sm + dst, &maps[k].m[arr], 0, arr == 3 ? j0 - 1 : j0, 0, bar);
-            else
+            } else
                 tma::bulk_load(sm + dst, maps[k].whole[arr], (unsigned)(L.rows * 2 * L.hx * nz) * 4u, bar);
         }
     // what the peers will send: halo rows a sweep, the bottom's b and x
@@ -343,9 +344,10 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
     // zeros beside the zero weights, and they go back out with x)
     for (int i = tid; i < P.x4; i += 32 * warps) reinterpret_cast<float4*>(sm + P.x)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     cluster_arrive();  // this CTA's shared memory may be written by its peers after this
+    const bool first = k_lo == 0 && k_hi > 0;  // holds rows of the first level
+    if (tid == 0 && first) tma::acquire_map(&maps[0].m[4]);
     pdl_enter();
     pdl_trigger();  // the dependent's blocks load what this kernel does not write
-    const bool first = k_lo == 0 && k_hi > 0;  // holds rows of the first level
     if (tid == 0 && first) {
         tma::mbar_arrive_expect_tx(barb, (unsigned)(P.L[0].rows * 2 * P.L[0].hx * nz) * 4u);
         tma::load_3d(sm + P.L[0].b, &maps[0].m[4], 0, nd > 0 ? rank * P.L[0].rows : 0, 0, barb);
