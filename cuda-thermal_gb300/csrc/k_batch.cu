@@ -131,6 +131,9 @@ __global__ void __launch_bounds__(NT, 4)
                     inst_stop(c, bc, cond);
                 }
             }
+            // block_sum2's shared arrays: warp 0 reads gather_inst's sums after that
+            // sum's only barrier, and the next task's sums go to the same place
+            __syncthreads();
         }
     }
 }
