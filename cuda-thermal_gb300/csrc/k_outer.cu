@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(NT)
 // ---- setup and bookkeeping ------------------------------------------------
 
 __global__ void k_to_split_f(Geo g, int planes, const float* __restrict__ in,
-                             float* __restrict__ out) {
+                             float* __restrict__ out, Edge edge) {
     const size_t nxy = (size_t)g.nx * g.ny;
     const size_t n = nxy * (size_t)planes;
     for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n;
@@ -239,7 +239,8 @@ __global__ void k_to_split_f(Geo g, int planes, const float* __restrict__ in,
         const int l = (int)(c / nxy);
         const size_t rem = c - (size_t)l * nxy;
         const int j = (int)(rem / g.nx), i = (int)(rem - (size_t)j * g.nx);
-        out[(size_t)l * g.plane + scol(g, i, j)] = in[c];
+        const bool none = (edge == EDGE_EAST && i == g.nx - 1) || (edge == EDGE_NORTH && j == g.ny - 1);
+        out[(size_t)l * g.plane + scol(g, i, j)] = none ? 0.0f : in[c];
     }
 }
 
@@ -470,8 +471,8 @@ void launch_update_p(cudaStream_t st, unsigned n, const double* r, const double*
     k_update_p<<<std::min(grid_for(n / 2), (unsigned)wb), NT, 0, st>>>(n / 2, r, invd, p, ctl, cond);
 }
 
-void launch_to_split_f(cudaStream_t st, const Geo& g, int planes, const float* nat, float* split) {
-    k_to_split_f<<<grid_for((size_t)g.nx * g.ny * planes), NT, 0, st>>>(g, planes, nat, split);
+void launch_to_split_f(cudaStream_t st, const Geo& g, int planes, const float* nat, float* split, Edge edge) {
+    k_to_split_f<<<grid_for((size_t)g.nx * g.ny * planes), NT, 0, st>>>(g, planes, nat, split, edge);
 }
 
 void launch_to_split_d(cudaStream_t st, const Geo& g, const double* nat, double* split) {

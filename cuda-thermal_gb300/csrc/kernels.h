@@ -140,7 +140,12 @@ cudaError_t launch_conv_selftest(cudaStream_t st, unsigned long long n, unsigned
                                  unsigned long long* mismatches);
 
 // ---- setup and auxiliary kernels, k_outer.cu ------------------------------
-void launch_to_split_f(cudaStream_t st, const Geo& g, int planes, const float* nat, float* split);
+// edge: the face array (gE, gN) whose last column's or row's entries are no faces
+// of the grid; they are stored as zero whatever the caller's array holds there
+// (k_tail.cu multiplies by them where the others test for the edge).
+enum Edge { EDGE_NONE = 0, EDGE_EAST, EDGE_NORTH };
+void launch_to_split_f(cudaStream_t st, const Geo& g, int planes, const float* nat, float* split,
+                       Edge edge = EDGE_NONE);
 void launch_to_split_d(cudaStream_t st, const Geo& g, const double* nat, double* split);
 void launch_to_natural_d(cudaStream_t st, const Geo& g, const double* split, double* nat);
 // diag = op_diag (FP64, no contraction); invd = 1 / diag when invd != null.

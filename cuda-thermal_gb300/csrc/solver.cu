@@ -295,9 +295,10 @@ ct_status Solver::create(const ct_model* m_in, ct_precond pc_, ct_precision prec
         float* natf = reinterpret_cast<float*>(nat);
         const float* src[4] = {m->gE, m->gN, m->gU, m->cap};
         float* dst[4] = {gE, gN, gU, cap};
+        const Edge edge[4] = {EDGE_EAST, EDGE_NORTH, EDGE_NONE, EDGE_NONE};
         for (int a = 0; a < 4; ++a) {
             CT_CK(cudaMemcpyAsync(natf, src[a], ncells * 4, cudaMemcpyHostToDevice, st));
-            launch_to_split_f(st, g0, g0.nz, natf, dst[a]);
+            launch_to_split_f(st, g0, g0.nz, natf, dst[a], edge[a]);
         }
         CT_CK(cudaMemcpyAsync(natf, m->gB, (size_t)m->nx * m->ny * 4, cudaMemcpyHostToDevice, st));
         launch_to_split_f(st, g0, 1, natf, gB);
