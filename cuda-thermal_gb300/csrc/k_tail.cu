@@ -32,6 +32,7 @@
 // one thread per column runs the Thomas recurrence on registers. Arithmetic and
 // order are the grid kernels' (k_mg.cu): same bits.
 #include <algorithm>
+#include <climits>
 #include <cstring>
 
 #include "kernels.h"
@@ -74,8 +75,8 @@ __device__ __forceinline__ void send4(unsigned a, float4 v, unsigned bar) {
                  : "memory");
 }
 // Bounded wait for what peers send (the first phase of `bar`).
-__device__ __forceinline__ bool receive(uint64_t* bar) {
-    for (unsigned k = 0; k < tma::kWaitLimit; ++k) {
+__device__ __forceinline__ bool receive(uint64_t* bar, unsigned limit) {
+    for (unsigned k = 0; k < limit; ++k) {
         unsigned ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -353,22 +354,26 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
         tma::load_3d(sm + P.L[0].b, &maps[0].m[4], 0, nd > 0 ? rank * P.L[0].rows : 0, 0, barb);
     }
     const bool closed = loop_done(ctl, cond);  // the same in every thread of the cluster
-    bool ok = tma::mbar_wait(bar0, 0u);        // (the level descriptors come with the tables)
-    if (tid == 0 && nd > 0 && ((rank * P.rd) & 1)) {  // the coarse offsets for an odd first coarse row
+    // A thread whose wait for the tables (the level descriptors come with them) runs
+    // out does no work below: it would take offsets from what never landed. It keeps
+    // to the barriers, whose number the parameters give.
+    const bool landed = tma::mbar_wait(bar0, 0u, P.polls);
+    bool ok = landed;
+    if (landed && tid == 0 && nd > 0 && ((rank * P.rd) & 1)) {  // the coarse offsets for an odd first coarse row
         TailLevel& L = const_cast<TailLevel&>(tail_level(nd - 1));
         L.tpar += 2 * L.ncol;
         L.tcell += 2 * L.ncell;
     }
     Cta c;
-    c.nz = nz;
-    c.tid = tid;
+    c.nz = landed ? nz : 0;
+    c.tid = landed ? tid : INT_MAX;
     c.lane = lane;
     c.rank = rank;
     c.nd = nd;
     c.warp = warp;
     c.warps = warps;
     auto rows_of = [&](int k) { return k < nd ? min(tail_level(k).rows, tail_level(k).ny - c.row0(k)) : tail_level(k).ny; };
-    ok = ok && (!first || tma::mbar_wait(barb, 0u));
+    ok = ok && (!first || tma::mbar_wait(barb, 0u, P.polls));
     cluster_wait();
     if (!closed) {
         // down: red from x = 0, black, restriction
@@ -377,17 +382,17 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
             const bool spread = k < nd;
             const TailLevel& L = tail_level(k);
             const int j0 = c.row0(k), nr = rows_of(k);
-            if (k == nd && nd > 0) ok = ok && receive(bard);
+            if (k == nd && nd > 0) ok = ok && receive(bard, P.polls);
             tail_recur<MZ, true>(c, L, nr, 0, halo, spread, 4 * k);
-            if (k == k_lo) ok = ok && tma::mbar_wait(bar1, 0u);
+            if (k == k_lo) ok = ok && tma::mbar_wait(bar1, 0u, P.polls);
             if (k == n - 1) break;
             __syncthreads();
-            if (spread) ok = ok && receive(&barh[4 * k]);
+            if (spread) ok = ok && receive(&barh[4 * k], P.polls);
             tail_gather<false>(c, L, nr, 1, 0, 0);
             __syncthreads();
             tail_recur<MZ, false>(c, L, nr, 1, halo, spread, 4 * k + 1);
             __syncthreads();
-            if (spread) ok = ok && receive(&barh[4 * k + 1]);
+            if (spread) ok = ok && receive(&barh[4 * k + 1], P.polls);
             tail_restrict(c, L, tail_level(k + 1), j0, k == nd - 1 ? far : 0u, far_bar);
             __syncthreads();
         }
@@ -409,7 +414,7 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
                     if (d < P.dist) {
                         const unsigned to = remote(base, (unsigned)d) + 4u * (unsigned)(P.xd + (r0 - j) * RC);
                         const unsigned tb = remote(tma::smem_addr(baru), (unsigned)d);
-                        for (int l = warp; l < nz; l += warps) {
+                        for (int l = warp; l < c.nz; l += warps) {
                             const float4* const from = reinterpret_cast<const float4*>(sm + N.x + l * xcp + (r0 + 1) * RC);
 #pragma unroll 4
                             for (int s = lane >> 4; s < n4; s += 2) send4(to + 4u * (unsigned)(l * xdpl) + 16u * (unsigned)s, from[s], tb);
@@ -417,7 +422,7 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
                     }
                 }
                 if (!dist) break;
-                ok = ok && receive(baru);
+                ok = ok && receive(baru, P.polls);
                 xc = P.xd;
                 xcp = (P.rd + 2) * 2 * N.hx;
             }
@@ -425,15 +430,15 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
             __syncthreads();
             tail_recur<MZ, false>(c, L, nr, 1, halo, spread, 4 * k + 2);
             __syncthreads();
-            if (spread) ok = ok && receive(&barh[4 * k + 2]);
+            if (spread) ok = ok && receive(&barh[4 * k + 2], P.polls);
             tail_gather<false>(c, L, nr, 0, 0, 0);
             __syncthreads();
             tail_recur<MZ, false>(c, L, nr, 0, halo, spread && k > 0, 4 * k + 3);
             __syncthreads();
-            if (spread && k > 0) ok = ok && receive(&barh[4 * k + 3]);
+            if (spread && k > 0) ok = ok && receive(&barh[4 * k + 3], P.polls);
         }
     } else {
-        ok = ok && tma::mbar_wait(bar1, 0u);
+        ok = ok && tma::mbar_wait(bar1, 0u, P.polls);
     }
     cluster_arrive();  // no CTA leaves before its peers have sent what they send
     if (!closed && first) {  // the first level's x, whole rows (padding is zero)
@@ -441,22 +446,32 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
         const int RS = 2 * F.hx, j0 = c.row0(0), row4 = (nd > 0 ? min(F.rows, F.ny - j0) : F.ny) * RS / 4;
         const float4* const x4 = reinterpret_cast<const float4*>(sm + F.x + RS);
         const int xpl4 = (F.rows + 2) * RS / 4;
-        for (int l = warp; l < nz; l += warps)
+        for (int l = warp; l < c.nz; l += warps)
             for (int i = lane; i < row4; i += 32)
                 reinterpret_cast<float4*>(P.x0 + (size_t)l * P.plane + (size_t)j0 * RS)[i] = x4[l * xpl4 + i];
     }
     cluster_wait();
     if (__syncthreads_or(ok ? 0 : 1) && tid == 0) {
         // A bounded wait ran out: the phases ran on whatever was there (every
-        // access stays in bounds). Record it and stop the solve, only now that
-        // every CTA of the cluster has read the stop flag, and let the copies
-        // land before leaving.
+        // access stays in bounds: without the tables there are none). Record it and
+        // stop the solve, only now that every CTA of the cluster has read the stop
+        // flag. Before this CTA's shared memory goes, what is in flight to it lands:
+        // its copies, and what its peers sent (all of them are past their sends).
         atomicExch(&ctl->err, 1);
         ctl->breakdown = 1;
         stop_loop(ctl, cond);
-        tma::mbar_wait(bar0, 0u);
-        tma::mbar_wait(bar1, 0u);
-        if (first) tma::mbar_wait(barb, 0u);
+        const unsigned polls = P.polls / 64u + 1u;
+        tma::mbar_wait(bar0, 0u, polls);
+        tma::mbar_wait(bar1, 0u, polls);
+        if (first) tma::mbar_wait(barb, 0u, polls);
+        if (!closed && nd > 0) {
+            if (bottom) receive(bard, polls);
+            if (dist) {
+                receive(baru, polls);
+                for (int i = 0; i < 4 * nd; ++i)
+                    if (i != 3) receive(&barh[i], polls);  // (the first level's last sweep sends nothing)
+            }
+        }
     }
 }
 
@@ -474,6 +489,7 @@ bool plan_tail(const LevelView<float>* views, int n, int ctas, bool apart, size_
     p.n = n;
     p.nd = nd;
     p.nz = nz;
+    p.polls = tma::kWaitLimit;
     p.x0 = views[0].x;
     p.plane = views[0].g.plane;
     const int most = apart ? ctas - 1 : ctas;

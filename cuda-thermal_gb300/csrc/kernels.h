@@ -327,6 +327,7 @@ struct TailPlan {
     int tab, table_bytes;  // the descriptors and tables
     unsigned first_bytes, bottom_first_bytes, dist_bytes, bottom_bytes;  // copies: 1/pivot and gU of the first level, all
     int smem;              // bytes
+    unsigned polls;        // of one wait before it gives up
     float* x0;             // the first level's x in global memory
     unsigned plane;        // its plane stride
     TailLevel L[kTailLevels];

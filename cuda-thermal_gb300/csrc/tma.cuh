@@ -67,8 +67,8 @@ __device__ __forceinline__ bool mbar_wait_or_abort(uint64_t* bar, unsigned parit
 }
 
 // Bounded wait for the phase with the given parity to complete.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
-    for (unsigned k = 0; k < kWaitLimit; ++k)
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, unsigned limit = kWaitLimit) {
+    for (unsigned k = 0; k < limit; ++k)
         if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
