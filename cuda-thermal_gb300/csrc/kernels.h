@@ -50,13 +50,15 @@ inline int wave_blocks(K kernel, int cap) {
 // its predecessor (each block of the predecessor releases it as it exits);
 // every such kernel calls pdl_enter() (wait until the predecessor grid has
 // completed and its memory is visible) before it touches what that grid writes,
-// and pdl_trigger() only after it: so when a kernel starts, every grid before its
-// predecessor has completed, and what those wrote, and what no kernel of the loop
-// writes, may be loaded before the wait. The latency-bound kernels do (the split
-// sweeps and the restrictions: operator, factors, on the way up b, ahead of the
-// prolongation x), and let their dependent start at once: 237 x 181 x 13 100.0 ->
-// 93.5 us an iteration, 400 x 400 x 10 in FP64 321.7 -> 304.8, 800 x 800 x 10 351 ->
-// 341. The staged sweeps gain nothing (their blocks fill the SMs until they leave).
+// and pdl_trigger() only after it. The wait is what makes memory visible, so only
+// what no kernel of the loop writes (operator, factors, tables) may be loaded ahead
+// of it. The latency-bound kernels do that (the split sweeps and the restrictions),
+// and let their dependent start at once: 237 x 181 x 13 100 -> 95 us an iteration,
+// 400 x 400 x 10 in FP64 322 -> 300, 800 x 800 x 10 351 -> 342. b and x, which an
+// older kernel of the loop wrote, gain nothing by it (95.4 ahead of the wait and
+// 95.7 after, 305.6 and 300.0, 342.8 and 344.8): their loads are in flight together
+// with the coarse corrections'. The staged sweeps gain nothing either (their blocks
+// fill the SMs until they leave).
 // Without the launch attribute both instructions are no-ops. CT_PDL=0 turns the
 // attribute off.
 bool pdl_enabled();

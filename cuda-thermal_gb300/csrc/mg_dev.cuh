@@ -272,15 +272,7 @@ __device__ __forceinline__ bool split_columns(const LevelView<T>& L, const Level
     T rhs = 0, fi = 0, fc = 0;
     float gu = 0.0f, gw = 0.0f, ge = 0.0f, gs = 0.0f, gn = 0.0f;
     // before the wait for the preceding kernel (kernels.h): the operator and the
-    // factors, on the way up b, and ahead of the prolongation x as well
-    const bool b_early = PRO || (!ZERO && color == 0);
-    T xw = 0, xe = 0, xs = 0, xn = 0;
-    auto load_x = [&] {
-        if (n.w) xw = L.x[base + n.sw];
-        if (n.e) xe = L.x[base + n.se];
-        if (n.so) xs = L.x[base + n.ss];
-        if (n.no) xn = L.x[base + n.sn];
-    };
+    // factors, which no kernel of the loop writes
     if (on) {
         fi = L.finv[id];
         gu = L.gU[id];
@@ -291,21 +283,22 @@ __device__ __forceinline__ bool split_columns(const LevelView<T>& L, const Level
             if (n.so) gs = L.gN[base + n.ss];
             gn = L.gN[id];
         }
-        if (b_early) rhs = L.b[id];
-        if (PRO) load_x();
     }
     const auto flags = enter();
     if (on) {
-        if (!b_early) rhs = L.b[id];
+        rhs = L.b[id];
         if (!ZERO) {
+            T xw = 0, xe = 0, xs = 0, xn = 0;
+            if (n.w) xw = L.x[base + n.sw];
+            if (n.e) xe = L.x[base + n.se];
+            if (n.so) xs = L.x[base + n.ss];
+            if (n.no) xn = L.x[base + n.sn];
             if (PRO) {
                 const T* const cx = C.x + (unsigned)l * C.g.plane;
                 if (n.w) xw = xw + cx[n.pw];
                 if (n.e) xe = xe + cx[n.pe];
                 if (n.so) xs = xs + cx[n.ps];
                 if (n.no) xn = xn + cx[n.pn];
-            } else {
-                load_x();
             }
             T sum = 0;  // lat_sum's order
             if (n.w) sum += face<T>(gw) * xw;
