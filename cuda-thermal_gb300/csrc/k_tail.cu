@@ -272,8 +272,8 @@ __device__ __forceinline__ int row_columns(int nx, int j, int color) { return (n
 
 template <int MZ>
 __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarps : MZ), 1)
-    k_tail(const __grid_constant__ TailPlan P, const TailMaps* __restrict__ maps, const int* __restrict__ table, Ctl* ctl,
-           Cond cond) {
+    k_tail(const __grid_constant__ TailPlan P, const __grid_constant__ TailMaps maps, const int* __restrict__ table,
+           Ctl* ctl, Cond cond) {
     float* const sm = tail_smem();
     // the first sweep's factors and the tables; everything else of the operator;
     // the first level's b; the bottom's b (from the distributed levels); the
@@ -319,11 +319,10 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
             const int dst = arr == 0 ? L.fi : arr == 1 ? L.gu : arr == 2 ? L.ge : L.gn;
             uint64_t* const bar = arr < 2 && k == k_lo ? bar0 : bar1;
             const int j0 = rank * L.rows;
-            if (k < nd) {
-                tma::acquire_map(&maps[k].m[arr]);
-                tma::load_3d(sm + dst, &maps[k].m[arr], 0, arr == 3 ? j0 - 1 : j0, 0, bar);
-            } else
-                tma::bulk_load(sm + dst, maps[k].whole[arr], (unsigned)(L.rows * 2 * L.hx * nz) * 4u, bar);
+            if (k < nd)
+                tma::load_3d(sm + dst, &maps.m[k][arr], 0, arr == 3 ? j0 - 1 : j0, 0, bar);
+            else
+                tma::bulk_load(sm + dst, maps.whole[k][arr], (unsigned)(L.rows * 2 * L.hx * nz) * 4u, bar);
         }
     // what the peers will send: halo rows a sweep, the bottom's b and x
     if (warp == warps - 1 && nd > 0) {
@@ -346,12 +345,11 @@ __global__ void __launch_bounds__(32 * (MZ < 4 ? 4 : MZ > kTailWarps ? kTailWarp
     for (int i = tid; i < P.x4; i += 32 * warps) reinterpret_cast<float4*>(sm + P.x)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     cluster_arrive();  // this CTA's shared memory may be written by its peers after this
     const bool first = k_lo == 0 && k_hi > 0;  // holds rows of the first level
-    if (tid == 0 && first) tma::acquire_map(&maps[0].m[4]);
     pdl_enter();
     pdl_trigger();  // the dependent's blocks load what this kernel does not write
     if (tid == 0 && first) {
         tma::mbar_arrive_expect_tx(barb, (unsigned)(P.L[0].rows * 2 * P.L[0].hx * nz) * 4u);
-        tma::load_3d(sm + P.L[0].b, &maps[0].m[4], 0, nd > 0 ? rank * P.L[0].rows : 0, 0, barb);
+        tma::load_3d(sm + P.L[0].b, &maps.m[0][4], 0, nd > 0 ? rank * P.L[0].rows : 0, 0, barb);
     }
     const bool closed = loop_done(ctl, cond);  // the same in every thread of the cluster
     // A thread whose wait for the tables (the level descriptors come with them) runs
@@ -607,15 +605,15 @@ void fill_tail_table(const TailPlan& p, int* table) {
 }
 
 bool make_tail_maps(const TailPlan& p, const LevelView<float>* views, TailMaps* maps) {
+    std::memset(maps, 0, sizeof *maps);
     for (int k = 0; k < p.n; ++k) {
         const LevelView<float>& v = views[k];
         const unsigned RS = 2u * (unsigned)v.g.hx, rows = (unsigned)p.L[k].rows, nz = (unsigned)p.nz;
         const float* src[5] = {v.finv, v.gU, v.gE, v.gN, v.b};
-        std::memset(&maps[k], 0, sizeof maps[k]);
-        for (int a = 0; a < 4; ++a) maps[k].whole[a] = src[a];
+        for (int a = 0; a < 4; ++a) maps->whole[k][a] = src[a];
         if (k >= p.nd && k > 0) continue;  // (the first level's b is always a tensor copy)
         for (int a = 0; a < 5; ++a)
-            if (!encode_tail_map(&maps[k].m[a], src[a], v.g, RS, a == 3 ? rows + 1u : rows, nz)) return false;
+            if (!encode_tail_map(&maps->m[k][a], src[a], v.g, RS, a == 3 ? rows + 1u : rows, nz)) return false;
     }
     return true;
 }
@@ -668,7 +666,7 @@ bool tail_fits_device(const TailPlan& p) {
     return e == cudaSuccess && clusters > 0;
 }
 
-cudaError_t launch_tail(cudaStream_t st, const TailPlan& p, const TailMaps* maps, const int* table, Ctl* ctl,
+cudaError_t launch_tail(cudaStream_t st, const TailPlan& p, const TailMaps& maps, const int* table, Ctl* ctl,
                         Cond cond) {
     return with_tail_kernel(p.nz, [&](auto kern) {
         cudaLaunchConfig_t cfg;

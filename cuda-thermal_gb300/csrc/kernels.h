@@ -334,12 +334,15 @@ struct TailPlan {
     unsigned plane;        // its plane stride
     TailLevel L[kTailLevels];
 };
-// One level's arrays: 1/pivot, gU, gE, gN, b. A distributed level's as
-// tensor maps, whole rows (both colours) of all planes (gN with one row more);
-// the others' as they lie.
+// The levels' arrays: 1/pivot, gU, gE, gN, b. A distributed level's (and the first
+// level's b) as tensor maps, whole rows (both colours) of all planes (gN with one row
+// more); the others' as they lie. 5.6 KB of kernel parameters: maps in global memory
+// need a fence each (tma.cuh, acquire_map), and an iteration of 501 x 333 x 10 took
+// 150.9 us with them, 147.3 so; 800 x 800 x 10 344.8 and 341.5; 64 x 64 x 10 45.6
+// and 45.1.
 struct TailMaps {
-    CUtensorMap m[5];
-    const float* whole[16];  // (four, padded to the maps' alignment)
+    CUtensorMap m[kTailSpread][5];
+    const float* whole[kTailLevels][4];
 };
 // Lays out levels views[0 .. n) for a cluster of at most `ctas` CTAs, the bottom
 // levels on a CTA of their own (apart) or with the first rows; false if they do
@@ -349,7 +352,7 @@ void fill_tail_table(const TailPlan& p, int* table);  // p.table_bytes of it
 bool make_tail_maps(const TailPlan& p, const LevelView<float>* views, TailMaps* maps);
 bool encode_tail_map(CUtensorMap* out, const float* base, const Geo& g, unsigned row, unsigned rows, unsigned nz);
 bool tail_fits_device(const TailPlan& p);  // the device can hold such a cluster
-cudaError_t launch_tail(cudaStream_t st, const TailPlan& p, const TailMaps* maps, const int* table, Ctl* ctl,
+cudaError_t launch_tail(cudaStream_t st, const TailPlan& p, const TailMaps& maps, const int* table, Ctl* ctl,
                         Cond cond);
 template <class T>
 size_t small_smem_bytes(const TailLevels<T>& tl);

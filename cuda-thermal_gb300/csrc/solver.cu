@@ -137,7 +137,6 @@ ct_status Solver::create(const ct_model* m_in, ct_precond pc_, ct_precision prec
     const size_t o_part = ar.take((size_t)NSLOT * 4 * maxb * 8);
     const size_t o_ctl = ar.take(sizeof(Ctl));
     const bool want_tail = mt == MG_F32 && !skip_graphs;
-    const size_t o_tm = want_tail ? ar.take(kTailLevels * sizeof(TailMaps)) : 0;
     const size_t o_tt = want_tail ? ar.take(kTailTableMax) : 0;
     if (pc == CT_MULTIGRID) {
         Level L;
@@ -233,7 +232,6 @@ ct_status Solver::create(const ct_model* m_in, ct_precond pc_, ct_precision prec
     part = at<double>(o_part);
     ctl = at<Ctl>(o_ctl);
     if (want_tail) {
-        tail_maps = at<TailMaps>(o_tm);
         tail_table = at<int>(o_tt);
         const ct_status ts = choose_tail(tail_max);
         if (ts != CT_OK) return ts;
@@ -361,16 +359,16 @@ ct_status Solver::choose_tail(size_t smem_max) {
         best.n = 0;
         for (const bool apart : {false, true})  // the one with fewer rows a CTA; of two with the same, apart
             if (plan_tail(v, nl, kTailCtas, apart, smem_max, &p) && (best.n == 0 || p.rd <= best.rd)) best = p;
-        std::vector<TailMaps> m((size_t)nl);
+        TailMaps m;
         if (best.n == 0 || (size_t)best.table_bytes > kTailTableMax || !tail_fits_device(best) ||
-            !make_tail_maps(best, v, m.data()))
+            !make_tail_maps(best, v, &m))
             continue;
         std::vector<int> table((size_t)best.table_bytes / 4);
         fill_tail_table(best, table.data());
-        CT_CK(cudaMemcpyAsync(tail_maps, m.data(), m.size() * sizeof(TailMaps), cudaMemcpyHostToDevice, st));
         CT_CK(cudaMemcpyAsync(tail_table, table.data(), (size_t)best.table_bytes, cudaMemcpyHostToDevice, st));
         CT_CK(cudaStreamSynchronize(st));
         tail = best;
+        tail_maps = m;
         small_k0 = k0;
         return CT_OK;
     }

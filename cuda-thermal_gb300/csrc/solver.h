@@ -89,7 +89,7 @@ class Solver {
     bool have_cond = false;
     size_t small_k0 = 0;   // levels from small_k0 down run in one block from shared memory
     TailPlan tail{};       // FP32: those levels in one cluster launch (tail.n > 0)
-    TailMaps* tail_maps = nullptr;
+    TailMaps tail_maps{};
     int* tail_table = nullptr;
     bool fuse_sweep0 = true;  // a level's first (x = 0) sweep rides with the restriction into it
     bool sweep0_grid = true;  // x = 0 sweeps of the staged levels on the grid kernel

@@ -50,27 +50,22 @@ struct Stack {
 };
 
 int launch(const TailPlan& p, const Stack& s, const std::vector<int>& table) {
-    std::vector<TailMaps> m((size_t)p.n);
-    if (!make_tail_maps(p, s.v.data(), m.data())) return 1;
-    TailMaps* dm = nullptr;
+    TailMaps m;
+    if (!make_tail_maps(p, s.v.data(), &m)) return 1;
     int* dt = nullptr;
     Ctl *dc = nullptr, c;
     std::memset(&c, 0, sizeof c);
     const size_t n = (size_t)s.v[0].g.plane * s.v[0].g.nz;
     std::vector<float> before(n), after(n);
-    if (cudaMalloc(&dm, m.size() * sizeof(TailMaps)) != cudaSuccess || cudaMalloc(&dt, table.size() * 4) != cudaSuccess ||
-        cudaMalloc(&dc, sizeof c) != cudaSuccess)
-        return 1;
-    cudaMemcpy(dm, m.data(), m.size() * sizeof(TailMaps), cudaMemcpyHostToDevice);
+    if (cudaMalloc(&dt, table.size() * 4) != cudaSuccess || cudaMalloc(&dc, sizeof c) != cudaSuccess) return 1;
     cudaMemcpy(dt, table.data(), table.size() * 4, cudaMemcpyHostToDevice);
     cudaMemcpy(dc, &c, sizeof c, cudaMemcpyHostToDevice);
     cudaMemcpy(before.data(), s.v[0].x, n * 4, cudaMemcpyDeviceToHost);
-    if (launch_tail(nullptr, p, dm, dt, dc, Cond{0, 0}) != cudaSuccess) return 1;
+    if (launch_tail(nullptr, p, m, dt, dc, Cond{0, 0}) != cudaSuccess) return 1;
     if (cudaDeviceSynchronize() != cudaSuccess) return 1;
     cudaMemcpy(&c, dc, sizeof c, cudaMemcpyDeviceToHost);
     cudaMemcpy(after.data(), s.v[0].x, n * 4, cudaMemcpyDeviceToHost);
     std::printf("launch %d %d %d %d %d\n", p.ctas, c.err, c.breakdown, c.done, before == after ? 0 : 1);
-    cudaFree(dm);
     cudaFree(dt);
     cudaFree(dc);
     return 0;

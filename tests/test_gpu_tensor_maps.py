@@ -1,7 +1,7 @@
-"""Tensor maps that lie in device memory (the coarse end of the V-cycle, k_tail.cu;
-the batch's staged sweeps, k_sweep_tma.cu) where solvers are built, solved and freed
-one after another: stacks of two shapes with the same number of cells, so that a map
-lies where the other shape's lay. Every field is bit for bit the one that launches
+"""Tensor maps (the coarse end of the V-cycle, k_tail.cu; in device memory the batch's
+staged sweeps', k_sweep_tma.cu) where solvers are built, solved and freed one after
+another: stacks of several shapes with the same number of cells, so that arrays and
+maps lie where another shape's lay. Every field is bit for bit the one that launches
 without tensor maps give."""
 import numpy as np
 import pytest
