@@ -108,22 +108,25 @@ __device__ __forceinline__ bool publish_sums(const double (&v)[N], double* part,
     __shared__ int last;
     const double a = block_sums<N>(v);
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (w < N && lane == 0) {
-        part[(size_t)w * stride + slot] = a;
-        __threadfence();
-    }
+    if (w < N && lane == 0) part[(size_t)w * stride + slot] = a;
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == count - 1u ? 1 : 0;
+    if (threadIdx.x == 0) {
+        // the thread that takes the ticket fences on both sides of it: the barrier
+        // before puts the other warps' stores ahead of the first fence, the one
+        // after puts the second ahead of the loads of the last block's threads
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == count - 1u ? 1 : 0;
+        if (last) __threadfence();
+    }
     __syncthreads();
     return last != 0;
 }
-// In the last block: the totals of slots first .. first + count - 1, in thread 0.
-// Resets the ticket.
+// In the last block (after publish_sums): the totals of slots first .. first + count
+// - 1, in thread 0. Resets the ticket.
 template <int N>
 __device__ __forceinline__ void gather_sums(const double* part, int stride, unsigned first, unsigned count,
                                             unsigned* ticket, double (&total)[N]) {
     __shared__ double t[N];
-    __threadfence();
     double v[N];
 #pragma unroll
     for (int q = 0; q < N; ++q) v[q] = 0.0;
