@@ -70,8 +70,7 @@ constexpr unsigned kRowChunkDw = 64;
 // Candidate tiles of the autotuner (columns per block for the sweeps, coarse
 // cells per block for the restriction).
 constexpr unsigned kSweepTiles[] = {256, 512, 1024, 2048};
-// ... once more with a block per 32 of a tile's columns, a thread a column and plane
-// (the last candidate).
+// ... once more with a block per 32 of a tile's columns, a thread a column and plane.
 constexpr unsigned kSplitTile = 256;
 // ... and tiles per block of the staged sweeps (k_sweep_tma.cu).
 constexpr unsigned kTmaTiles[] = {1, 2, 4, 8};
@@ -476,6 +475,9 @@ ct_status Batch::build_bucket(Bucket& b) {
 // candidates on the bucket's own levels (the level arrays are scratch between
 // solves, so the timing runs leave nothing behind that a solve reads).
 ct_status Batch::tune_bucket(Bucket& b) {
+    // CT_BATCH_TILE fixes the grid sweeps' and restrictions' tile, CT_BATCH_SPLIT=1 the
+    // grid sweeps' form with a thread a column and plane (stacks of at most 32
+    // planes), CT_BATCH_TMA_TILES the staged sweeps' tiles a block.
     unsigned fixed = 0, fixed_tma = 0;
     if (const char* e = std::getenv("CT_BATCH_TILE")) fixed = (unsigned)std::atol(e);
     if (const char* e = std::getenv("CT_BATCH_TMA_TILES")) fixed_tma = (unsigned)std::atol(e);
@@ -483,8 +485,17 @@ ct_status Batch::tune_bucket(Bucket& b) {
     CT_BK(cudaEventCreate(&e0));
     CT_BK(cudaEventCreate(&e1));
     ct_status s = CT_OK;
-    std::vector<unsigned> grid_tiles(std::begin(kSweepTiles), std::end(kSweepTiles));
-    if (b.mz <= 32) grid_tiles.push_back(kSplitTile);
+    struct GridForm {
+        unsigned tile;
+        bool split;
+    };
+    std::vector<GridForm> grid_forms;
+    const char* force_split = std::getenv("CT_BATCH_SPLIT");
+    if (fixed)
+        grid_forms.push_back({fixed, false});
+    else if (!(force_split && force_split[0] == '1' && b.mz <= 32))
+        for (unsigned t : kSweepTiles) grid_forms.push_back({t, false});
+    if (!fixed && b.mz <= 32) grid_forms.push_back({kSplitTile, true});
     for (int d = 0; d < b.depth && s == CT_OK; ++d) {
         // staged instances (all of them in mode 1, the fitting ones in mode 2)
         // and grid-swept ones (all in mode 0, the rest in mode 2)
@@ -526,17 +537,18 @@ ct_status Batch::tune_bucket(Bucket& b) {
             const std::vector<int>& ins = tma ? ins_t : ins_g;
             const std::vector<unsigned>& items = tma ? items_t : items_g;
             if (ins.empty()) continue;
-            std::vector<unsigned> cands;
-            if (tma && fixed_tma) cands.push_back(fixed_tma);
-            else if (tma) cands.assign(std::begin(kTmaTiles), std::end(kTmaTiles));
-            else if (fixed) cands.push_back(fixed);
-            else cands = grid_tiles;
+            std::vector<GridForm> cands = grid_forms;
+            if (tma) {
+                cands.clear();
+                if (fixed_tma) cands.push_back({fixed_tma, false});
+                else
+                    for (unsigned t : kTmaTiles) cands.push_back({t, false});
+            }
             float best = 1e30f;
-            for (size_t c = 0; c < cands.size(); ++c) {
-                const unsigned tile = cands[c];
+            for (const auto [tile, split] : cands) {
                 Plan p;
                 if ((s = upload_plan(make_plan(ni, ins, items, tile), &p)) != CT_OK) break;
-                if (!tma && c >= std::size(kSweepTiles)) p.split = (int)(tile / 32u);
+                if (split) p.split = (int)(tile / 32u);
                 CT_BK(cudaStreamSynchronize(st));
                 const float t = cands.size() == 1 ? 0.0f : time_of([&] {
                     if (tma)
@@ -567,14 +579,10 @@ ct_status Batch::tune_bucket(Bucket& b) {
                 items.push_back((unsigned)g.ny * (unsigned)g.hx);
             }
             const float staged = part_best[0] + (ins_g.empty() ? 0.0f : part_best[1]);
-            std::vector<unsigned> cands;
-            if (fixed) cands.push_back(fixed);
-            else cands = grid_tiles;
-            for (size_t c = 0; c < cands.size(); ++c) {
-                const unsigned tile = cands[c];
+            for (const auto [tile, split] : grid_forms) {
                 Plan p;
                 if ((s = upload_plan(make_plan(ni, b.inst, items, tile), &p)) != CT_OK) break;
-                if (c >= std::size(kSweepTiles)) p.split = (int)(tile / 32u);
+                if (split) p.split = (int)(tile / 32u);
                 CT_BK(cudaStreamSynchronize(st));
                 const float t = time_of([&] {
                     launch_b_sweep(b.st, p, views[(size_t)d], views[(size_t)d], 1, false, false, b.mz, ctl);
@@ -607,14 +615,10 @@ ct_status Batch::tune_bucket(Bucket& b) {
                     launch_b_sweep(b.st, b.sweep_grid[(size_t)d], views[(size_t)d], views[(size_t)d], 0, true,
                                    false, b.mz, ctl);
             });
-            std::vector<unsigned> cands;
-            if (fixed) cands.push_back(fixed);
-            else cands = grid_tiles;
-            for (size_t c = 0; c < cands.size(); ++c) {
-                const unsigned tile = cands[c];
+            for (const auto [tile, split] : grid_forms) {
                 Plan p;
                 if ((s = upload_plan(make_plan(ni, b.inst, items, tile), &p)) != CT_OK) break;
-                if (c >= std::size(kSweepTiles)) p.split = (int)(tile / 32u);
+                if (split) p.split = (int)(tile / 32u);
                 CT_BK(cudaStreamSynchronize(st));
                 const float t = time_of([&] {
                     launch_b_sweep(b.st, p, views[(size_t)d], views[(size_t)d], 0, true, false, b.mz, ctl);

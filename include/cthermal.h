@@ -321,8 +321,10 @@ ct_status ct_batch_step_records(ct_batch* b, const double* dt, ct_step_record* o
  * sweeps of depth d are staged by bulk tensor copies, 2 where only the
  * instances whose level holds a full tile row are (the others run the grid
  * sweep), 0 where none is; sweep_tiles[d] the 32 x 8-column tiles per block
- * of the staged part, else the columns per block of the grid sweep;
- * restrict_tiles[d] the coarse cells per block of the restriction. */
+ * of the staged part, else the columns per task of the grid sweep (a block's;
+ * 256 also where eight blocks of 32 columns share a task, a thread a column
+ * and plane); restrict_tiles[d] the groups of four neighbouring coarse cells
+ * per block of the restriction. */
 ct_status ct_batch_num_buckets(const ct_batch* b, int* nbuckets);
 /* The batch's stream (a cudaStream_t): every ct_batch_* call is ordered on it,
  * and a solve's work on the buckets' own streams is joined back into it. */
