@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(NT)
     const LevelView<float> L = views[t.inst];
     const LevelView<float> C = PRO ? cviews[t.inst] : L;
     for (unsigned q = t.begin + threadIdx.x; q < t.end; q += NT)
-        sweep_column<float, MZ, ZERO, PRO, false>(L, C, color, q);
+        sweep_column<float, MZ, ZERO, PRO>(L, C, color, q);
 }
 
 // The same with one thread per column and plane (split_columns), 32 columns a block:

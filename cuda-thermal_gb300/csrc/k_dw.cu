@@ -276,38 +276,6 @@ __global__ void k_to_dw(unsigned n, const double* __restrict__ in, float2* __res
         out[k] = dw_of(in[k]);
 }
 
-// split double word -> natural double.
-__global__ void k_dw_to_natural(Geo g, const float2* __restrict__ in, double* __restrict__ out) {
-    const size_t nxy = (size_t)g.nx * g.ny;
-    const size_t n = nxy * (size_t)g.nz;
-    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n;
-         c += (size_t)gridDim.x * blockDim.x) {
-        const int l = (int)(c / nxy);
-        const size_t rem = c - (size_t)l * nxy;
-        const int j = (int)(rem / g.nx), i = (int)(rem - (size_t)j * g.nx);
-        out[c] = dw_d(in[(size_t)l * g.plane + scol(g, i, j)]);
-    }
-}
-
-// natural double -> split double word.
-__global__ void k_natural_to_dw(Geo g, const double* __restrict__ in, float2* __restrict__ out) {
-    const size_t nxy = (size_t)g.nx * g.ny;
-    const size_t n = nxy * (size_t)g.nz;
-    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n;
-         c += (size_t)gridDim.x * blockDim.x) {
-        const int l = (int)(c / nxy);
-        const size_t rem = c - (size_t)l * nxy;
-        const int j = (int)(rem / g.nx), i = (int)(rem - (size_t)j * g.nx);
-        out[(size_t)l * g.plane + scol(g, i, j)] = dw_of(in[c]);
-    }
-}
-
-// split double word -> split double (for the FP64 bookkeeping kernels).
-__global__ void k_dw_to_d(unsigned n, const float2* __restrict__ in, double* __restrict__ out) {
-    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-        out[k] = dw_d(in[k]);
-}
-
 unsigned blocks_of(size_t n) {
     size_t b = (n + NT - 1) / NT;
     if (b < 1) b = 1;
@@ -360,18 +328,6 @@ void launch_update_x_dw(cudaStream_t st, unsigned n, const float2* p, float2* x,
 
 void launch_to_dw(cudaStream_t st, unsigned n, const double* in, float2* out) {
     k_to_dw<<<blocks_of(n), NT, 0, st>>>(n, in, out);
-}
-
-void launch_dw_to_natural(cudaStream_t st, const Geo& g, const float2* split, double* nat) {
-    k_dw_to_natural<<<blocks_of((size_t)g.nx * g.ny * g.nz), NT, 0, st>>>(g, split, nat);
-}
-
-void launch_natural_to_dw(cudaStream_t st, const Geo& g, const double* nat, float2* split) {
-    k_natural_to_dw<<<blocks_of((size_t)g.nx * g.ny * g.nz), NT, 0, st>>>(g, nat, split);
-}
-
-void launch_dw_to_d(cudaStream_t st, unsigned n, const float2* in, double* out) {
-    k_dw_to_d<<<blocks_of(n), NT, 0, st>>>(n, in, out);
 }
 
 }  // namespace ct

@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(NT, (ZERO && sizeof(T) == 4 && MZ > 0 && MZ <=
     if (ZERO) pdl_trigger();
     const unsigned q = blockIdx.x * NT + threadIdx.x;
     if (q >= (unsigned)L.g.ny * (unsigned)L.g.hx) return;
-    sweep_column<T, MZ, ZERO, PRO, false>(L, C, color, q);
+    sweep_column<T, MZ, ZERO, PRO>(L, C, color, q);
 }
 
 // Sweep of a small level, a block per 32 columns (split_columns).
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(NT)
     pdl_enter();
     pdl_trigger();
     const int2 flags = loop_flags(ctl);  // tested after the sums' loads are issued
-    const T sum = on ? restrict_sum<T, false>(F, f, I, J, l) : T(0);
+    const T sum = on ? restrict_sum<T>(F, f, I, J, l) : T(0);
     if (loop_done(flags, cond) || !on) return;
     C.b[(unsigned)l * cg.plane + scol(cg, I, J)] = sum;
 }
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(32 * MZ)
     pdl_enter();
     pdl_trigger();
     const int2 flags = loop_flags(ctl);  // tested after the sums' loads are issued
-    if (on) sum = restrict_sum<T, false>(F, f, I, J, l);
+    if (on) sum = restrict_sum<T>(F, f, I, J, l);
     if (loop_done(flags, cond)) return;  // the same for every thread of the grid
     if (on) {
         C.b[id] = sum;

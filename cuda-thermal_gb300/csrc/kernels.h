@@ -196,9 +196,6 @@ void launch_step_dw(cudaStream_t st, unsigned n, const float* z, const float2* w
                     float2* r, float* b0, Ctl* ctl, const Red& red, Cond cond, bool write_x);
 void launch_update_x_dw(cudaStream_t st, unsigned n, const float2* p, float2* x, const Ctl* ctl, int blocks);
 void launch_to_dw(cudaStream_t st, unsigned n, const double* in, float2* out);
-void launch_dw_to_natural(cudaStream_t st, const Geo& g, const float2* split, double* nat);
-void launch_natural_to_dw(cudaStream_t st, const Geo& g, const double* nat, float2* split);
-void launch_dw_to_d(cudaStream_t st, unsigned n, const float2* in, double* out);
 
 // ---- multigrid, k_mg.cu ---------------------------------------------------
 // Coarse level from the fine one (mg_coarse_cell arithmetic, split layouts).

@@ -61,42 +61,33 @@ __device__ __forceinline__ double face<double>(float f) {
 __device__ __forceinline__ float fcp_of(float gu, float fi) { return __fmul_rn(-gu, fi); }
 __device__ __forceinline__ double fcp_of(float gu, double fi) { return __dmul_rn(-f64dev::widen(gu), fi); }
 
-// Loads of values that other blocks of the same kernel may have written
-// (x and b inside the cluster tail kernel) go to L2 (CG = true); everything
-// else may use the L1 path.
-template <bool CG, class T>
-__device__ __forceinline__ T ldm(const T* p) {
-    if (CG) return __ldcg(p);
-    return *p;
-}
-
 // Lateral neighbour sum of op_lat_sum (src/operator3d.h:62-78) at plane l:
 // west, east, south, north; with PRO each neighbour value carries its
 // parent's coarse correction.
-template <class T, bool PRO, bool CG>
+template <class T, bool PRO>
 __device__ __forceinline__ T lat_sum(const LevelView<T>& L, const LevelView<T>& C, const Nbr& n,
                                      int l) {
     const unsigned base = (unsigned)l * L.g.plane;
     const unsigned cbase = PRO ? (unsigned)l * C.g.plane : 0u;
     T s = 0;
     if (n.w) {
-        T xv = ldm<CG>(L.x + base + n.sw);
-        if (PRO) xv = xv + ldm<CG>(C.x + cbase + n.pw);
+        T xv = L.x[base + n.sw];
+        if (PRO) xv = xv + C.x[cbase + n.pw];
         s += face<T>(L.gE[base + n.sw]) * xv;
     }
     if (n.e) {
-        T xv = ldm<CG>(L.x + base + n.se);
-        if (PRO) xv = xv + ldm<CG>(C.x + cbase + n.pe);
+        T xv = L.x[base + n.se];
+        if (PRO) xv = xv + C.x[cbase + n.pe];
         s += face<T>(L.gE[base + n.s]) * xv;
     }
     if (n.so) {
-        T xv = ldm<CG>(L.x + base + n.ss);
-        if (PRO) xv = xv + ldm<CG>(C.x + cbase + n.ps);
+        T xv = L.x[base + n.ss];
+        if (PRO) xv = xv + C.x[cbase + n.ps];
         s += face<T>(L.gN[base + n.ss]) * xv;
     }
     if (n.no) {
-        T xv = ldm<CG>(L.x + base + n.sn);
-        if (PRO) xv = xv + ldm<CG>(C.x + cbase + n.pn);
+        T xv = L.x[base + n.sn];
+        if (PRO) xv = xv + C.x[cbase + n.pn];
         s += face<T>(L.gN[base + n.s]) * xv;
     }
     return s;
@@ -106,32 +97,29 @@ __device__ __forceinline__ T lat_sum(const LevelView<T>& L, const LevelView<T>& 
 // memory, where load latency bounds a sweep): b plus the lateral sum in op_lat_sum's order (west, east, south, north),
 // each neighbour value with its parent's coarse correction under PRO; an
 // absent neighbour reads the column itself with weight 0.
-template <class T, bool ZERO, bool PRO, bool CG>
+template <class T, bool PRO>
 __device__ __forceinline__ T bf_rhs(const LevelView<T>& L, const LevelView<T>& C, const Nbr& n, unsigned l) {
     const Geo& g = L.g;
     const unsigned base = l * g.plane, id = base + n.s;
-    T rhs = ldm<CG>(L.b + id);
-    if (!ZERO) {
-        const unsigned sw = n.w ? n.sw : n.s, se = n.e ? n.se : n.s;
-        const unsigned ss = n.so ? n.ss : n.s, sn = n.no ? n.sn : n.s;
-        T xw = ldm<CG>(L.x + base + sw), xe = ldm<CG>(L.x + base + se);
-        T xs = ldm<CG>(L.x + base + ss), xn = ldm<CG>(L.x + base + sn);
-        if (PRO) {
-            const T* cx = C.x + l * C.g.plane;
-            xw = xw + ldm<CG>(cx + n.pw);
-            xe = xe + ldm<CG>(cx + n.pe);
-            xs = xs + ldm<CG>(cx + n.ps);
-            xn = xn + ldm<CG>(cx + n.pn);
-        }
-        const float ew = L.gE[base + sw], ee = L.gE[id], ns = L.gN[base + ss], nn = L.gN[id];
-        T sum = 0;
-        sum += (n.w ? face<T>(ew) : T(0)) * xw;
-        sum += (n.e ? face<T>(ee) : T(0)) * xe;
-        sum += (n.so ? face<T>(ns) : T(0)) * xs;
-        sum += (n.no ? face<T>(nn) : T(0)) * xn;
-        rhs = rhs + sum;
+    const T rhs = L.b[id];
+    const unsigned sw = n.w ? n.sw : n.s, se = n.e ? n.se : n.s;
+    const unsigned ss = n.so ? n.ss : n.s, sn = n.no ? n.sn : n.s;
+    T xw = L.x[base + sw], xe = L.x[base + se];
+    T xs = L.x[base + ss], xn = L.x[base + sn];
+    if (PRO) {
+        const T* cx = C.x + l * C.g.plane;
+        xw = xw + cx[n.pw];
+        xe = xe + cx[n.pe];
+        xs = xs + cx[n.ps];
+        xn = xn + cx[n.pn];
     }
-    return rhs;
+    const float ew = L.gE[base + sw], ee = L.gE[id], ns = L.gN[base + ss], nn = L.gN[id];
+    T sum = 0;
+    sum += (n.w ? face<T>(ew) : T(0)) * xw;
+    sum += (n.e ? face<T>(ee) : T(0)) * xe;
+    sum += (n.so ? face<T>(ns) : T(0)) * xs;
+    sum += (n.no ? face<T>(nn) : T(0)) * xn;
+    return rhs + sum;
 }
 
 // The Thomas recurrence of sweep_column on the column at slot s whose
@@ -175,7 +163,7 @@ __device__ __forceinline__ void column_solve(const LevelView<T>& L, const T* src
 // all loads independent of one another, then the Thomas recurrence runs on
 // registers and x is written once. MZ = 0 is the general path for deep
 // columns, with forward values going through x as in the reference.
-template <class T, int MZ, bool ZERO, bool PRO, bool CG>
+template <class T, int MZ, bool ZERO, bool PRO>
 __device__ __forceinline__ void sweep_column(const LevelView<T>& L, const LevelView<T>& C,
                                              int color, unsigned q) {
     const Geo& g = L.g;
@@ -192,8 +180,8 @@ __device__ __forceinline__ void sweep_column(const LevelView<T>& L, const LevelV
         for (int l = 0; l < MZ; ++l) {
             if (l < g.nz) {
                 const unsigned id = (unsigned)l * g.plane + n.s;
-                T rhs = ldm<CG>(L.b + id);
-                if (!ZERO) rhs = rhs + lat_sum<T, PRO, CG>(L, C, n, l);
+                T rhs = L.b[id];
+                if (!ZERO) rhs = rhs + lat_sum<T, PRO>(L, C, n, l);
                 v[l] = rhs;
                 fi[l] = L.finv[id];
                 gu[l] = L.gU[id];
@@ -226,8 +214,8 @@ __device__ __forceinline__ void sweep_column(const LevelView<T>& L, const LevelV
         float gu_b = 0.0f;
         for (int l = 0; l < g.nz; ++l) {
             const unsigned id = (unsigned)l * g.plane + n.s;
-            T rhs = ldm<CG>(L.b + id);
-            if (!ZERO) rhs = rhs + lat_sum<T, PRO, CG>(L, C, n, l);
+            T rhs = L.b[id];
+            if (!ZERO) rhs = rhs + lat_sum<T, PRO>(L, C, n, l);
             const T lower = l > 0 ? -face<T>(gu_b) : T(0);
             prev = (rhs - lower * prev) * L.finv[id];
             L.x[id] = prev;
@@ -235,7 +223,7 @@ __device__ __forceinline__ void sweep_column(const LevelView<T>& L, const LevelV
         }
         for (int l = g.nz - 2; l >= 0; --l) {
             const unsigned id = (unsigned)l * g.plane + n.s;
-            prev = ldm<CG>(L.x + id) - L.fcp[id] * prev;
+            prev = L.x[id] - L.fcp[id] * prev;
             L.x[id] = prev;
         }
     }
@@ -426,11 +414,11 @@ __device__ __forceinline__ RedFaces red_faces(const LevelView<T>& F, int I, int 
 // The residual of all four children on all operands took 35.5 us at 800 x 800 x 10
 // (23.0 so) and, in FP64, 47 at 400 x 400 x 10 (13.1); an iteration 382 -> 359 and
 // 388 -> 318.
-template <class T, bool CG>
+template <class T>
 __device__ __forceinline__ T restrict_sum(const LevelView<T>& F, const RedFaces& f, int I, int J, int l) {
     const RedSlots r = red_slots(F.g, I, J, l);
-    const T x10 = ldm<CG>(F.x + r.c10), x01 = ldm<CG>(F.x + r.c01), xw = ldm<CG>(F.x + r.a_w), xs = ldm<CG>(F.x + r.a_s);
-    const T xe = ldm<CG>(F.x + r.a_e), xn = ldm<CG>(F.x + r.a_n);
+    const T x10 = F.x[r.c10], x01 = F.x[r.c01], xw = F.x[r.a_w], xs = F.x[r.a_s];
+    const T xe = F.x[r.a_e], xn = F.x[r.a_n];
     return red_residuals<T>(r.w, r.e, r.so, r.no, r.both, r.e2, r.n2, f.gw, f.ge, f.gs, f.gn, f.hw, f.he, f.hs, f.hn, xw,
                             x10, xs, x01, xe, xn);
 }
@@ -504,12 +492,12 @@ __device__ __forceinline__ void store_wide(const LevelView<T>& C, int I, int J, 
 }
 
 // Coarse cell q = J cnx + I, stored as coarse b.
-template <class T, bool CG>
+template <class T>
 __device__ __forceinline__ void restrict_cell(const LevelView<T>& F, const LevelView<T>& C, unsigned q,
                                               int l) {
     const Geo& cg = C.g;
     const int J = (int)(q / (unsigned)cg.nx), I = (int)(q - (unsigned)J * cg.nx);
-    C.b[(unsigned)l * cg.plane + scol(cg, I, J)] = restrict_sum<T, CG>(F, red_faces(F, I, J, l), I, J, l);
+    C.b[(unsigned)l * cg.plane + scol(cg, I, J)] = restrict_sum<T>(F, red_faces(F, I, J, l), I, J, l);
 }
 
 
@@ -528,7 +516,7 @@ __device__ __forceinline__ void gather_rhs(const LevelView<T>& L, const LevelVie
         const int i = 2 * t + ((j + color) & 1);
         if (i >= g.nx) continue;
         const Nbr n = neighbours<PRO>(g, C.g, i, j, t, color);
-        L.x[l * g.plane + n.s] = bf_rhs<T, false, PRO, false>(L, C, n, l);
+        L.x[l * g.plane + n.s] = bf_rhs<T, PRO>(L, C, n, l);
     }
 }
 
@@ -679,7 +667,7 @@ __device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, unsigned cha
             const unsigned work = ccols * (unsigned)C.g.nz;
             for (unsigned w = tid; w < work; w += nth) {
                 const int l = (int)(w / ccols);
-                restrict_cell<T, false>(L, C, w - (unsigned)l * ccols, l);
+                restrict_cell<T>(L, C, w - (unsigned)l * ccols, l);
             }
         } else if constexpr (MZ > 0) {
             // A sweep in two steps: one task per column and plane gathers
@@ -700,12 +688,12 @@ __device__ __forceinline__ int vsmall_body(const TailLevels<T>& tl, unsigned cha
                     column_solve<T, MZ>(L, src, (unsigned)(2 * j + color) * (unsigned)L.g.hx + (unsigned)t);
             }
         } else if (kind == 0) {  // deep columns (MZ = 0): x goes through memory
-            for (unsigned q = tid; q < ncol; q += nth) sweep_column<T, MZ, true, false, false>(L, L, 0, q);
+            for (unsigned q = tid; q < ncol; q += nth) sweep_column<T, MZ, true, false>(L, L, 0, q);
         } else if (kind == 1) {
-            for (unsigned q = tid; q < ncol; q += nth) sweep_column<T, MZ, false, false, false>(L, L, color, q);
+            for (unsigned q = tid; q < ncol; q += nth) sweep_column<T, MZ, false, false>(L, L, color, q);
         } else {
             const LevelView<T> C = small_view<T>(smem + soff[k + 1], sg[k + 1]);
-            for (unsigned q = tid; q < ncol; q += nth) sweep_column<T, MZ, false, true, false>(L, C, 1, q);
+            for (unsigned q = tid; q < ncol; q += nth) sweep_column<T, MZ, false, true>(L, C, 1, q);
         }
         __syncthreads();
     }

@@ -19,7 +19,6 @@ struct RN<float> {
     static __device__ float sub(float a, float b) { return __fsub_rn(a, b); }
     static __device__ float mul(float a, float b) { return __fmul_rn(a, b); }
     static __device__ float div(float a, float b) { return __fdiv_rn(a, b); }
-    static __device__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
     static __device__ float of(float f) { return f; }
 };
 template <>
@@ -28,7 +27,6 @@ struct RN<double> {
     static __device__ double sub(double a, double b) { return __dsub_rn(a, b); }
     static __device__ double mul(double a, double b) { return __dmul_rn(a, b); }
     static __device__ double div(double a, double b) { return __ddiv_rn(a, b); }
-    static __device__ double fma(double a, double b, double c) { return __fma_rn(a, b, c); }
     static __device__ double of(float f) { return f64dev::widen(f); }
 };
 
