@@ -101,8 +101,7 @@ __device__ __forceinline__ void issue_plane(const SweepMaps* m, float* sm, uint6
 // have arrived. No block-wide barrier inside the loop, so warps drift apart
 // and cover one another's waits. A wait that runs out raises `abort`, which
 // ends every other wait.
-// MAPS_GLOBAL: the maps lie in global memory (tma.cuh, acquire_map).
-template <int TT, int TJ, int NS, int MZ, bool ZERO, bool PRO, bool MAPS_GLOBAL>
+template <int TT, int TJ, int NS, int MZ, bool ZERO, bool PRO>
 __device__ __forceinline__ bool sweep_tiles_ws(const SweepMaps* m, const LevelView<float>& L,
                                                const LevelView<float>& C, int color,
                                                const TileList& tl, float* sm, uint64_t* full,
@@ -127,18 +126,6 @@ __device__ __forceinline__ bool sweep_tiles_ws(const SweepMaps* m, const LevelVi
     __syncthreads();
     if (warp == TJ) {  // producer
         if (lane == 0) {
-            if (MAPS_GLOBAL) {
-                acquire_map(&m->b);
-                acquire_map(&m->fi);
-                acquire_map(&m->gu);
-                if (!ZERO) {
-                    acquire_map(&m->ge);
-                    acquire_map(&m->gn);
-                    acquire_map(&m->ox);
-                    acquire_map(&m->oge);
-                    acquire_map(&m->ogn);
-                }
-            }
             for (int w = 0; w < nitems; ++w) {
                 const int s = w % NS;
                 if (w >= NS && !mbar_wait_or_abort(&empty[s], (unsigned)(w / NS - 1) & 1u, abort)) break;
@@ -273,7 +260,7 @@ __global__ void __launch_bounds__(TT * TJ + 32, MZ <= 16 ? kSweepWsBlocks : 2)
     const int ntiles = ((g.hx + TT - 1) / TT) * ((g.ny + TJ - 1) / TJ);
     const int count = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     const TileList tl{(int)blockIdx.x, (int)gridDim.x, count};
-    if (!sweep_tiles_ws<TT, TJ, NS, MZ, ZERO, PRO, false>(&m, L, C, color, tl, sm, full, empty, &flags[0],
+    if (!sweep_tiles_ws<TT, TJ, NS, MZ, ZERO, PRO>(&m, L, C, color, tl, sm, full, empty, &flags[0],
                                                      &flags[1]) &&
         threadIdx.x == 0)
         fail_wait(ctl, cond);
@@ -285,8 +272,13 @@ template <int TT, int TJ, int NS, int MZ, bool ZERO, bool PRO>
 __global__ void __launch_bounds__(TT * TJ + 32, MZ <= 16 ? kSweepWsBlocks : 2)
     kb_sweep_tma_ws(Plan p, const SweepMaps* __restrict__ maps, const LevelView<float>* __restrict__ views,
                     const LevelView<float>* __restrict__ cviews, int color, Ctl* ctl, BCtl* bc, Cond cond) {
-    pdl_enter();
     const Task t = p.tasks[blockIdx.x];
+    // The maps lie in global memory: the block fences them (a lane of the producer
+    // warp each) before its first copy, sweep_tiles_ws's first barrier in between,
+    // while it waits for the preceding kernel.
+    if ((int)threadIdx.x / 32 == TJ && (int)threadIdx.x % 32 < (ZERO ? kZeroMaps : kSweepMaps))
+        acquire_map(reinterpret_cast<const CUtensorMap*>(&maps[t.inst]) + threadIdx.x % 32);
+    pdl_enter();
     Ctl* c = &ctl[t.inst];
     if (*(volatile const int*)&c->done) return;
     extern __shared__ __align__(128) float sm[];
@@ -295,7 +287,7 @@ __global__ void __launch_bounds__(TT * TJ + 32, MZ <= 16 ? kSweepWsBlocks : 2)
     const LevelView<float> L = views[t.inst];
     const LevelView<float> C = PRO ? cviews[t.inst] : L;
     const TileList tl{(int)t.begin, 1, (int)(t.end - t.begin)};
-    if (!sweep_tiles_ws<TT, TJ, NS, MZ, ZERO, PRO, true>(&maps[t.inst], L, C, color, tl, sm, full, empty, &flags[0],
+    if (!sweep_tiles_ws<TT, TJ, NS, MZ, ZERO, PRO>(&maps[t.inst], L, C, color, tl, sm, full, empty, &flags[0],
                                                    &flags[1]) &&
         threadIdx.x == 0) {
         atomicExch(&c->err, 1);

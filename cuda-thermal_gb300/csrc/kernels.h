@@ -243,6 +243,8 @@ struct SweepMaps {
     CUtensorMap oge;                    // other colour's gE, box (kTileT + 8) x kTileJ
     CUtensorMap ogn;                    // other colour's gN, box kTileT x (kTileJ + 1)
 };
+constexpr int kSweepMaps = 8, kZeroMaps = 3;  // of them; those of the sweep from x = 0 (b, fi, gu)
+static_assert(sizeof(SweepMaps) == kSweepMaps * sizeof(CUtensorMap), "maps lie one after another");
 bool sweep_tma_fits(const Geo& g);  // nz <= 32 and at least one full tile row
 size_t sweep_tma_smem(bool zero_x);
 bool make_sweep_maps(const LevelView<float>& L, int color, SweepMaps* m, int tile_t = kTileT,

@@ -96,9 +96,10 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
         : "memory");
 }
 
-// Before a thread's first copy by a tensor map that lies in global memory (a map
-// among a kernel's parameters needs none): the copy engine may still hold what
-// another map, freed since, had at this address. System scope, as the host wrote it.
+// Before a block's first copy by a tensor map that lies in global memory (a map
+// among a kernel's parameters needs none), by one of its threads: the copy engine may
+// still hold what another map, freed since, had at this address. System scope, as the
+// host wrote it.
 __device__ __forceinline__ void acquire_map(const CUtensorMap* map) {
     asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(map))
                  : "memory");
