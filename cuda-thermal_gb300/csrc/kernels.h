@@ -53,7 +53,7 @@ inline int wave_blocks(K kernel, int cap) {
 // and pdl_trigger() only after it. The wait is what makes memory visible, so only
 // what no kernel of the loop writes (operator, factors, tables) may be loaded ahead
 // of it. The latency-bound kernels do that (the split sweeps and the restrictions),
-// and let their dependent start at once: 237 x 181 x 13 100 -> 95 us an iteration,
+// and the single solver's let their dependent start at once: 237 x 181 x 13 100 -> 95 us an iteration,
 // 400 x 400 x 10 in FP64 322 -> 300, 800 x 800 x 10 351 -> 342. b and x, which an
 // older kernel of the loop wrote, gain nothing by it (95.4 ahead of the wait and
 // 95.7 after, 305.6 and 300.0, 342.8 and 344.8): their loads are in flight together
