@@ -67,7 +67,8 @@ typedef enum ct_precision {
 } ct_precision;
 
 /* A finalized Model3D's arrays (src/stack3d.h:45-79): gE, gN, gU, cap have
- * nx*ny*nz entries, gB nx*ny, P nx*ny*nz. dx, dy (m) are the lateral cell
+ * nx*ny*nz entries, gB nx*ny, P nx*ny*nz; gE of the last column and gN of the
+ * last row are no faces and not used. dx, dy (m) are the lateral cell
  * sizes, which the multigrid coarsening needs (src/mg3d.h:139-166). */
 typedef struct ct_model {
     int nx, ny, nz;
