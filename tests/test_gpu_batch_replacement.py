@@ -1,6 +1,6 @@
 """The double-word batch's residual replacement where a block walks several tasks
 (more tasks of rows than one wave of blocks, k_batch.cu): instances whose first phases
-end in the same body, the last task of each shorter than a block's eight warps want,
+end in the same body, the last task of each shorter than the others,
 bit for bit as in batches of one task a block."""
 import numpy as np
 import pytest
